@@ -5,8 +5,8 @@
 // of one long vector, its operators and stage-0 products at their own offsets of
 // one operator buffer and one scratch buffer, so every batched matvec is one
 // launch per stage for all instances (mma.sync for FP64, tcgen05 for 3xTF32).
-// The Krylov recurrence runs segment-wise (one block per instance in every
-// vector kernel), and the host keeps one tridiagonal problem per instance; the
+// The Krylov recurrence runs segment-wise (krylov.cu: every segment cut into
+// ranges, a block each), and the host keeps one tridiagonal problem per instance; the
 // recurrence and its checks are those of lanczos1 (Lanczos::lanczos1,
 // src/dmrg_inst.cpp:1286-1348), applied per instance.
 #include <algorithm>
@@ -82,9 +82,30 @@ void HeffBatch<S>::finalize(Ctx& c) {
   P.finalize(c, kCxB<S>, /*mixed=*/true, &cb);
   M.scratch = std::make_shared<DevBuf>(sizeof(S) * std::max<long long>(P.scratch_elems, 1), c.stream);
   M.ntasks = (int)P.flat_terms.size();
-  d_seg = std::make_shared<DevBuf>(sizeof(long long) * seg.size(), c.stream);
-  SADMRG_CUDA(cudaMemcpyAsync(d_seg->get(), seg.data(), sizeof(long long) * seg.size(), cudaMemcpyHostToDevice,
-                              c.stream));
+  // ranges of the vector kernels: about 1024 of equal length over all segments (7 blocks
+  // of 256 threads per SM), whole multiples of a block's threads
+  long long per = (M.n + 1023) / 1024;
+  per = std::max<long long>(256, (per + 255) / 256 * 256);
+  std::vector<VecBlk> blk;
+  std::vector<int> blk0(np + 1, 0);
+  for (int i = 0; i < np; ++i) {
+    for (long long lo = seg[i]; lo < seg[i + 1]; lo += per)
+      blk.push_back(VecBlk{lo, (int)std::min(per, seg[i + 1] - lo), i});
+    blk0[i + 1] = (int)blk.size();
+  }
+  nblk = (int)blk.size();
+  const size_t bytes_blk = (sizeof(VecBlk) * blk.size() + 255) & ~size_t(255);
+  d_blk = std::make_shared<DevBuf>(bytes_blk + sizeof(int) * blk0.size(), c.stream);
+  if (nblk)
+    SADMRG_CUDA(cudaMemcpyAsync(d_blk->get(), blk.data(), sizeof(VecBlk) * blk.size(), cudaMemcpyHostToDevice, c.stream));
+  SADMRG_CUDA(cudaMemcpyAsync(d_blk->as<unsigned char>() + bytes_blk, blk0.data(), sizeof(int) * blk0.size(),
+                              cudaMemcpyHostToDevice, c.stream));
+  span = VecSpan{};
+  span.blk = d_blk->as<VecBlk>();
+  span.blk0 = reinterpret_cast<const int*>(d_blk->as<unsigned char>() + bytes_blk);
+  span.nblk = nblk;
+  span.nseg = np;
+  span.n = M.n;
   SADMRG_CUDA(cudaStreamSynchronize(c.stream));
   parts.clear();   // the merged buffers hold everything now
   ready = true;
@@ -97,37 +118,46 @@ template <class S>
 struct BatchKrylov {
   Ctx& c;
   long long N;
-  int ns, mlanc, bs;            // segments, Krylov size, beta row stride
-  DevBuf ff, vh, dots, coef, beta, cdev, mask, norm, active;
-  S* h_coef = nullptr;          // per step: coef (2 per segment) copied as it is made
-  double* h_beta = nullptr;     // beta rows (ns x bs)
+  int ns, mlanc;                // segments, Krylov size
+  VecSpan all;                  // every segment; the launches of a step and of a check mask it
+  DevBuf ff, vh, dots, coef, beta, cdev, mask, norm, active, partial, counter;
+  double* h_a = nullptr;        // a of step m, segment s: h_a[(m - 1) * ns + s]
+  double* h_beta = nullptr;     // b: h_beta[m * ns + s]
   S* h_dots = nullptr;          // 2 per segment
   double* h_cdev = nullptr;     // Ritz coefficients (ns x (mlanc + 1))
   int* h_mask = nullptr;
   int* h_active = nullptr;      // instances whose matvec work still runs (written only after a stream sync)
-  BatchKrylov(Ctx& cc, long long n, int nseg, int ml) : c(cc), N(n), ns(nseg), mlanc(ml), bs(ml + 2) {
+  BatchKrylov(Ctx& cc, const HeffBatch<S>& B, int ml) : c(cc), N(B.merged.n), ns(B.nseg()), mlanc(ml), all(B.span) {
     ff.alloc(sizeof(S) * N * (mlanc + 1), c.stream);
     vh.alloc(sizeof(S) * N * 2, c.stream);
     dots.alloc(sizeof(S) * (size_t)ns * (mlanc + 2), c.stream);
     coef.alloc(sizeof(S) * (size_t)ns * 2, c.stream);
-    beta.alloc(sizeof(double) * (size_t)ns * bs, c.stream);
+    beta.alloc(sizeof(double) * (size_t)ns * (mlanc + 2), c.stream);
     cdev.alloc(sizeof(double) * (size_t)ns * (mlanc + 1), c.stream);
     mask.alloc(sizeof(int) * ns, c.stream);
     norm.alloc(sizeof(double) * ns, c.stream);
     active.alloc(sizeof(int) * ns, c.stream);
-    SADMRG_CUDA(cudaMemsetAsync(beta.get(), 0, sizeof(double) * (size_t)ns * bs, c.stream));
-    SADMRG_CUDA(cudaMallocHost(&h_coef, sizeof(S) * (size_t)ns * 2 * (mlanc + 1)));
-    SADMRG_CUDA(cudaMallocHost(&h_beta, sizeof(double) * (size_t)ns * bs));
+    partial.alloc(sizeof(S) * (size_t)std::max(all.nblk, 1) * (mlanc + 1), c.stream);
+    counter.alloc(sizeof(unsigned) * ns, c.stream);
+    SADMRG_CUDA(cudaMemsetAsync(beta.get(), 0, beta.bytes(), c.stream));
+    SADMRG_CUDA(cudaMemsetAsync(counter.get(), 0, counter.bytes(), c.stream));
+    SADMRG_CUDA(cudaMemsetAsync(norm.get(), 0, norm.bytes(), c.stream));
+    SADMRG_CUDA(cudaMallocHost(&h_a, sizeof(double) * (size_t)ns * (mlanc + 1)));
+    SADMRG_CUDA(cudaMallocHost(&h_beta, sizeof(double) * (size_t)ns * (mlanc + 2)));
     SADMRG_CUDA(cudaMallocHost(&h_dots, sizeof(S) * (size_t)ns * 2));
     SADMRG_CUDA(cudaMallocHost(&h_cdev, sizeof(double) * (size_t)ns * (mlanc + 1)));
     SADMRG_CUDA(cudaMallocHost(&h_mask, sizeof(int) * ns));
     SADMRG_CUDA(cudaMallocHost(&h_active, sizeof(int) * ns));
+    // an instance without elements has no block to write its scalars: they read as zero
+    std::memset(h_a, 0, sizeof(double) * (size_t)ns * (mlanc + 1));
+    std::memset(h_beta, 0, sizeof(double) * (size_t)ns * (mlanc + 2));
+    std::memset(static_cast<void*>(h_dots), 0, sizeof(S) * (size_t)ns * 2);
     std::fill(h_active, h_active + ns, 1);
     SADMRG_CUDA(cudaMemcpyAsync(active.get(), h_active, sizeof(int) * ns, cudaMemcpyHostToDevice, c.stream));
   }
   ~BatchKrylov() {
     cudaStreamSynchronize(c.stream);
-    cudaFreeHost(h_coef);
+    cudaFreeHost(h_a);
     cudaFreeHost(h_beta);
     cudaFreeHost(h_dots);
     cudaFreeHost(h_cdev);
@@ -135,6 +165,17 @@ struct BatchKrylov {
     cudaFreeHost(h_active);
   }
   S* F(int i) { return ff.as<S>() + (size_t)i * N; }
+  VecSpan on(const DevBuf& m) const {   // the segments whose flag in m is set
+    VecSpan v = all;
+    v.active = m.as<int>();
+    return v;
+  }
+  void mdot(const VecSpan& v, const S* V, int nv, const S* x, const VecOut& o, const S* u0 = nullptr,
+            const S* u1 = nullptr) {
+    launch_vec_dots(kCxB<S>, v, V, N, nv, const_cast<S*>(x), u0, u1, coef.get(), partial.as<double>(), dots.get(),
+                    counter.as<unsigned>(), o, c.stream);
+    ++c.launches;
+  }
 };
 
 template <class S>
@@ -143,8 +184,7 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
   const HeffPlan<S>& H = B.merged;
   const int ns = B.nseg();
   const long long N = H.n;
-  const long long* seg = B.d_seg->template as<long long>();
-  BatchKrylov<S> K(c, N, ns, mlanc);
+  BatchKrylov<S> K(c, B, mlanc);
   const double tol = 1.e-6;
   BatchStats st;
   st.energy.assign(ns, 0.0);
@@ -166,40 +206,35 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
     for (int s = 0; s < ns; ++s)
       if (!done[s]) ++st.matvecs[s];
   };
-  // x /= |x| on the masked segments (all when mask is null); norms below 1e-12 are left alone
-  auto normalize = [&](S* x, bool masked) {
-    launch_seg_multi_dot(CX, x, N, 1, x, seg, ns, K.dots.get(), c.stream);
-    launch_seg_lanczos_scalar(CX, 1, K.dots.get(), nullptr, 0, K.norm.get(), 1, ns, c.stream);
-    SADMRG_CUDA(cudaMemcpyAsync(K.h_beta, K.norm.get(), sizeof(double) * ns, cudaMemcpyDeviceToHost, c.stream));
-    SADMRG_CUDA(cudaStreamSynchronize(c.stream));
-    for (int s = 0; s < ns; ++s) {
-      const double nr = K.h_beta[s];
-      K.h_cdev[s] = (nr > 1e-12 && (!masked || K.h_mask[s])) ? 1.0 / nr : 1.0;
-    }
-    SADMRG_CUDA(cudaMemcpyAsync(K.norm.get(), K.h_cdev, sizeof(double) * ns, cudaMemcpyHostToDevice, c.stream));
-    launch_seg_scale(CX, x, K.norm.template as<double>(), 1, 0, seg, ns, c.stream);
-    c.launches += 4;
-  };
-  // Ritz vectors of the masked segments into v: coefficients in h_cdev (row stride mlanc + 1)
+  VecOut to_norm;
+  to_norm.op = VO_NORM;
+  to_norm.scal = K.norm.get();
+  to_norm.sstride = 1;
+  // Ritz vectors of the masked segments into v (coefficients in h_cdev, row stride
+  // mlanc + 1) and their norms
   auto ritz = [&](int nv) {
     SADMRG_CUDA(cudaMemcpyAsync(K.cdev.get(), K.h_cdev, sizeof(double) * (size_t)ns * (mlanc + 1),
                                 cudaMemcpyHostToDevice, c.stream));
     SADMRG_CUDA(cudaMemcpyAsync(K.mask.get(), K.h_mask, sizeof(int) * ns, cudaMemcpyHostToDevice, c.stream));
-    launch_seg_lincomb(CX, v, K.F(0), N, nv, K.cdev.template as<double>(), mlanc + 1, K.mask.template as<int>(), seg,
-                       ns, c.stream);
+    launch_vec_lincomb(CX, K.on(K.mask), v, K.F(0), N, nv, K.cdev.template as<double>(), mlanc + 1,
+                       K.partial.template as<double>(), K.counter.template as<unsigned>(), to_norm, c.stream);
     ++c.launches;
   };
-  // Lanczos::check_eigenvector on the masked segments: normalise v, |<v|Hv>| / |Hv|
+  // Lanczos::check_eigenvector on the masked segments' Ritz vectors: normalise v (norms
+  // below 1e-12 are left alone), |<v|Hv>| / |Hv|
   std::vector<double> ov(ns, 0.0);
   auto check = [&]() {
-    normalize(v, true);
     S* vv = K.vh.template as<S>();
     S* hv = vv + N;
-    SADMRG_CUDA(cudaMemcpyAsync(vv, v, sizeof(S) * N, cudaMemcpyDeviceToDevice, c.stream));
-    matvec(vv, hv);
-    launch_seg_multi_dot(CX, vv, N, 2, hv, seg, ns, K.dots.get(), c.stream);
+    const VecSpan m = K.on(K.mask);
+    launch_vec_div(CX, m, v, v, vv, K.norm.template as<double>(), 1, 1e-12, c.stream);
     ++c.launches;
-    SADMRG_CUDA(cudaMemcpyAsync(K.h_dots, K.dots.get(), sizeof(S) * 2 * ns, cudaMemcpyDeviceToHost, c.stream));
+    matvec(vv, hv);
+    VecOut o;
+    o.op = VO_HOST;
+    o.host = K.h_dots;
+    o.hstride = 2;
+    K.mdot(m, vv, 2, hv, o);
     SADMRG_CUDA(cudaStreamSynchronize(c.stream));
     for (int s = 0; s < ns; ++s) {
       if (!K.h_mask[s]) continue;
@@ -215,42 +250,51 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
   };
 
   // F(0) = normalised v
-  SADMRG_CUDA(cudaMemcpyAsync(K.F(0), v, sizeof(S) * N, cudaMemcpyDeviceToDevice, c.stream));
-  std::fill(K.h_mask, K.h_mask + ns, 1);
-  normalize(K.F(0), false);
+  K.mdot(K.all, v, 1, v, to_norm);
+  launch_vec_div(CX, K.all, v, K.F(0), nullptr, K.norm.template as<double>(), 1, 1e-12, c.stream);
+  ++c.launches;
 
   int synced = 0;
   auto step = [&](int m) {
+    const VecSpan act = K.on(K.active);
+    double* bm = K.beta.template as<double>() + (size_t)m * ns;
     matvec(K.F(m - 1), K.F(m));
-    launch_seg_multi_dot(CX, K.F(m - 1), N, 1, K.F(m), seg, ns, K.dots.get(), c.stream);
-    launch_seg_lanczos_scalar(CX, 0, K.dots.get(), K.beta.template as<double>() + (m - 1), K.bs, K.coef.get(), 0, ns,
-                              c.stream);
-    if (m >= 2)
-      launch_seg_multi_axpy(CX, K.F(m), K.F(m - 2), N, 2, K.coef.get(), 2, seg, ns, c.stream);
-    else
-      launch_seg_multi_axpy(CX, K.F(m), K.F(m - 1), N, 1, K.coef.template as<S>() + 1, 2, seg, ns, c.stream);
+    VecOut o;
+    o.op = VO_COEF;
+    o.beta = bm - ns;
+    o.bstride = 1;
+    o.scal = K.coef.get();
+    o.host = K.h_a + (size_t)(m - 1) * ns;
+    o.hstride = 1;
+    K.mdot(act, K.F(m - 1), 1, K.F(m), o);
+    VecOut nb;
+    nb.op = VO_NORM;
+    nb.scal = bm;
+    nb.sstride = 1;
+    nb.host = K.h_beta + (size_t)m * ns;
+    nb.hstride = 1;
     if (m >= 2) {
-      launch_seg_multi_dot(CX, K.F(0), N, m, K.F(m), seg, ns, K.dots.get(), c.stream);
-      launch_seg_multi_axpy(CX, K.F(m), K.F(0), N, m, K.dots.get(), m, seg, ns, c.stream);
+      K.mdot(act, K.F(0), m, K.F(m), VecOut{}, K.F(m - 2), K.F(m - 1));
+      launch_vec_axpy(CX, act, K.F(m), K.F(0), N, m, K.dots.get(), m, K.partial.template as<double>(),
+                      K.counter.template as<unsigned>(), nb, c.stream);
+    } else {
+      launch_vec_axpy(CX, act, K.F(m), K.F(m - 1), N, 1, K.coef.template as<S>() + 1, 2,
+                      K.partial.template as<double>(), K.counter.template as<unsigned>(), nb, c.stream);
     }
-    launch_seg_multi_dot(CX, K.F(m), N, 1, K.F(m), seg, ns, K.dots.get(), c.stream);
-    launch_seg_lanczos_scalar(CX, 1, K.dots.get(), nullptr, 0, K.beta.template as<double>() + m, K.bs, ns, c.stream);
-    launch_seg_scale(CX, K.F(m), K.beta.template as<double>() + m, K.bs, 1, seg, ns, c.stream);
-    c.launches += 9;
-    SADMRG_CUDA(cudaMemcpyAsync(K.h_coef + (size_t)(m - 1) * 2 * ns, K.coef.get(), sizeof(S) * 2 * ns,
-                                cudaMemcpyDeviceToHost, c.stream));
+    launch_vec_div(CX, act, K.F(m), K.F(m), nullptr, bm, 1, -1.0, c.stream);
+    c.launches += 2;
   };
   auto sync_to = [&](int m, std::vector<int>& brk) {
-    SADMRG_CUDA(cudaMemcpyAsync(K.h_beta, K.beta.get(), sizeof(double) * (size_t)ns * K.bs, cudaMemcpyDeviceToHost,
-                                c.stream));
     SADMRG_CUDA(cudaStreamSynchronize(c.stream));
     brk.assign(ns, 0);
-    for (int s = 0; s < ns; ++s)
+    for (int s = 0; s < ns; ++s) {
+      if (done[s]) continue;
       for (int j = synced + 1; j <= m; ++j) {
-        aal[s][j - 1] = real_of(K.h_coef[(size_t)(j - 1) * 2 * ns + 2 * s + 1]);
-        nnl[s][j] = K.h_beta[(size_t)s * K.bs + j];
+        aal[s][j - 1] = K.h_a[(size_t)(j - 1) * ns + s];
+        nnl[s][j] = K.h_beta[(size_t)j * ns + s];
         if (!brk[s] && j >= 2 && nnl[s][j] < tol) brk[s] = j;
       }
+    }
     synced = m;
   };
 
@@ -300,9 +344,11 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
   // instances still open after mlanc - 1 steps: one more matvec, then the Ritz vector
   const int last = mlanc > 2 ? mlanc - 1 : 1;
   matvec(K.F(last), K.F(last + 1));
-  launch_seg_multi_dot(CX, K.F(last), N, 1, K.F(last + 1), seg, ns, K.dots.get(), c.stream);
-  ++c.launches;
-  SADMRG_CUDA(cudaMemcpyAsync(K.h_dots, K.dots.get(), sizeof(S) * ns, cudaMemcpyDeviceToHost, c.stream));
+  VecOut od;
+  od.op = VO_HOST;
+  od.host = K.h_dots;
+  od.hstride = 1;
+  K.mdot(K.on(K.active), K.F(last), 1, K.F(last + 1), od);
   SADMRG_CUDA(cudaStreamSynchronize(c.stream));
   std::fill(K.h_mask, K.h_mask + ns, 0);
   std::fill(K.h_cdev, K.h_cdev + (size_t)ns * (mlanc + 1), 0.0);

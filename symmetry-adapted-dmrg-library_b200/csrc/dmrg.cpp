@@ -306,10 +306,11 @@ void HeffPlan<S>::apply(Ctx& c, const S* psi, S* out, int prec) const {
 template <class S>
 void HeffPlan<S>::penalty(Ctx& c, const S* psi, S* out) const {
   if (npen <= 0) return;
-  launch_multi_dot(kCx<S>, pen_o->get(), n, npen, psi, n, c.d_partial, c.npart, pen_dot->get(), c.d_counter,
-                   c.stream);
-  launch_multi_axpy(kCx<S>, out, pen_wo->get(), n, npen, pen_dot->get(), n, c.stream);
-  c.launches += 3;
+  const VecSpan v = vec_span(n, c.npart);
+  launch_vec_dots(kCx<S>, v, pen_o->get(), n, npen, const_cast<S*>(psi), nullptr, nullptr, nullptr, c.d_partial,
+                  pen_dot->get(), c.d_counter, VecOut{}, c.stream);
+  launch_vec_axpy(kCx<S>, v, out, pen_wo->get(), n, npen, pen_dot->get(), 0, nullptr, nullptr, VecOut{}, c.stream);
+  c.launches += 2;
 }
 
 // ---------------------------------------------------------------------------
@@ -379,40 +380,70 @@ struct Krylov {
   Ctx& c;
   long long n;
   int mlanc;
-  DevBuf ff, vh, coef, dots, beta, cdev;
-  Krylov(Ctx& cc, long long nn, int ml) : c(cc), n(nn), mlanc(ml) {
+  VecSpan span;
+  DevBuf ff, vh, coef, dots, beta, cdev, partial;
+  // page-locked scalars of a solve: a_m at h_a[m - 1], b_m at h_b[m], Ritz coefficients, dots of a check
+  double *h_a, *h_b, *h_z;
+  S* h_dot;
+  Krylov(Ctx& cc, long long nn, int ml) : c(cc), n(nn), mlanc(ml), span(vec_span(nn, cc.npart)) {
     ff.alloc(sizeof(S) * n * (mlanc + 1), c.stream);
     vh.alloc(sizeof(S) * n * 2, c.stream);
     coef.alloc(sizeof(S) * (mlanc + 4), c.stream);
     dots.alloc(sizeof(S) * (mlanc + 4), c.stream);
     beta.alloc(sizeof(double) * (mlanc + 4), c.stream);
     cdev.alloc(sizeof(double) * (mlanc + 4), c.stream);
+    partial.alloc(sizeof(S) * (size_t)span.nblk * (mlanc + 1), c.stream);
     SADMRG_CUDA(cudaMemsetAsync(beta.get(), 0, sizeof(double) * (mlanc + 4), c.stream));
+    h_dot = reinterpret_cast<S*>(c.h_pinned);
+    h_a = c.h_pinned + 8;
+    h_b = h_a + mlanc + 2;
+    h_z = h_b + mlanc + 2;
   }
   S* F(int i) { return ff.as<S>() + (size_t)i * n; }
-  void mdot(const S* V, int nv, const S* x, void* out, int scalar_op = -1, const double* beta_prev = nullptr,
-            void* scalar_out = nullptr) {
-    launch_multi_dot(kCx<S>, V, n, nv, x, n, c.d_partial, c.npart, out, c.d_counter, c.stream, scalar_op, beta_prev,
-                     scalar_out);
+  double* norm() { return beta.as<double>() + mlanc + 2; }   // device word for norms outside the recurrence
+  // out[j] = <V_j|x> after x -= uc[0] u0 + uc[1] u1
+  void mdot(const S* V, int nv, S* x, void* out, const VecOut& o, const S* u0 = nullptr, const S* u1 = nullptr) {
+    launch_vec_dots(kCx<S>, span, V, n, nv, x, u0, u1, coef.get(), partial.as<double>(), out, c.d_counter, o,
+                    c.stream);
     ++c.launches;
   }
-  S dot_host(const S* a, const S* b) {  // <a|b>
-    mdot(a, 1, b, dots.get());
-    S r;
-    SADMRG_CUDA(cudaMemcpyAsync(&r, dots.get(), sizeof(S), cudaMemcpyDeviceToHost, c.stream));
-    SADMRG_CUDA(cudaStreamSynchronize(c.stream));
-    return r;
-  }
-  void scale_host(S* x, double s) {
-    launch_scale(kCx<S>, x, s, 0.0, n, c.stream);
+  // x -= sum c_j V_j and |x| to nrm (and host, when given)
+  void maxpy(S* x, const S* V, int nv, const S* cf, double* nrm, double* host) {
+    VecOut o;
+    o.op = VO_NORM;
+    o.scal = nrm;
+    o.host = host;
+    launch_vec_axpy(kCx<S>, span, x, V, n, nv, cf, 0, partial.as<double>(), c.d_counter, o, c.stream);
     ++c.launches;
   }
-  // vout = sum_j coef[j] F(j)
+  void div(const S* x, S* y, S* y2, const double* nrm, double floor) {
+    launch_vec_div(kCx<S>, span, x, y, y2, nrm, 0, floor, c.stream);
+    ++c.launches;
+  }
+  // |x| to norm()
+  void norm_of(const S* x) {
+    VecOut o;
+    o.op = VO_NORM;
+    o.scal = norm();
+    mdot(x, 1, const_cast<S*>(x), dots.get(), o);
+  }
+  // <V_j|x> to h_dot (after the next synchronisation)
+  void dots_to_host(const S* V, int nv, const S* x) {
+    VecOut o;
+    o.op = VO_HOST;
+    o.host = h_dot;
+    mdot(V, nv, const_cast<S*>(x), dots.get(), o);
+  }
+  // vout = sum_j z[j] F(j), its norm to norm()
   void ritz(S* vout, const std::vector<double>& z, int m) {
-    SADMRG_CUDA(cudaMemcpyAsync(cdev.get(), z.data(), sizeof(double) * m, cudaMemcpyHostToDevice, c.stream));
-    launch_lincomb(kCx<S>, vout, F(0), n, m, cdev.as<double>(), n, c.stream);
+    std::copy(z.begin(), z.begin() + m, h_z);
+    SADMRG_CUDA(cudaMemcpyAsync(cdev.get(), h_z, sizeof(double) * m, cudaMemcpyHostToDevice, c.stream));
+    VecOut o;
+    o.op = VO_NORM;
+    o.scal = norm();
+    launch_vec_lincomb(kCx<S>, span, vout, F(0), n, m, cdev.as<double>(), 0, partial.as<double>(), c.d_counter, o,
+                       c.stream);
     ++c.launches;
-    SADMRG_CUDA(cudaStreamSynchronize(c.stream));
   }
 };
 
@@ -437,63 +468,50 @@ LanczosStats lanczos1(Ctx& c, const HeffPlan<S>& H, S* v, int mlanc, int prec, b
     for (int i = 0; i + 1 < m; ++i) e[i] = nnl[i + 1];
     tridiag_eig(m, eig, e, z);
   };
-  auto ritz_vec = [&](int m) {
-    std::vector<double> col(z.begin(), z.begin() + m);  // eigenvector of the lowest Ritz value
-    K.ritz(v, col, m);
-  };
-  // Lanczos::check_eigenvector (src/dmrg_inst.cpp:1241-1254)
+  auto ritz_vec = [&](int m) { K.ritz(v, z, m); };  // eigenvector of the lowest Ritz value
+  // Lanczos::check_eigenvector (src/dmrg_inst.cpp:1241-1254) on the Ritz vector that
+  // ritz_vec just left in v (its norm beside it)
   auto check = [&](double& ee, double& ov) {
     S* vv = K.vh.template as<S>();
     S* hv = vv + n;
-    const double nor = std::sqrt(std::fabs(real_of(K.dot_host(v, v))));
-    K.scale_host(v, 1.0 / nor);
-    SADMRG_CUDA(cudaMemcpyAsync(vv, v, sizeof(S) * n, cudaMemcpyDeviceToDevice, c.stream));
+    K.div(v, v, vv, K.norm(), -1.0);
     matvec(vv, hv);
-    K.mdot(vv, 2, hv, K.dots.get());  // <v|h>, <h|h>
-    S r[2];
-    SADMRG_CUDA(cudaMemcpyAsync(r, K.dots.get(), sizeof(S) * 2, cudaMemcpyDeviceToHost, c.stream));
+    K.dots_to_host(vv, 2, hv);  // <v|h>, <h|h>
     SADMRG_CUDA(cudaStreamSynchronize(c.stream));
-    const double prod = std::sqrt(std::fabs(real_of(r[1])));
+    const double prod = std::sqrt(std::fabs(real_of(K.h_dot[1])));
     ee = prod;
-    ov = std::abs(r[0]) / prod;
+    ov = std::abs(K.h_dot[0]) / prod;
     st.overlap = ov;
   };
   // ff[0] = normalised v (Lanczos::initialize_lanczos, src/dmrg_inst.cpp:1201-1213)
-  SADMRG_CUDA(cudaMemcpyAsync(K.F(0), v, sizeof(S) * n, cudaMemcpyDeviceToDevice, c.stream));
-  {
-    const double nor = std::sqrt(std::fabs(real_of(K.dot_host(K.F(0), K.F(0)))));
-    if (nor > 1e-12) K.scale_host(K.F(0), 1.0 / nor);
-  }
+  K.norm_of(v);
+  K.div(v, K.F(0), nullptr, K.norm(), 1e-12);
   // one Lanczos step: F(m) = H F(m-1) - a F(m-1) - b F(m-2), reorthogonalised, normalised.
   // a and b go to page-locked host memory without a synchronisation; the host reads
   // them at the next check point (every 4 steps, as the reference checks), so the
   // steps in between queue back to back on the stream.
-  const int pin_stride = kCx<S> ? 2 : 1;
-  SADMRG_REQUIRE((mlanc + 2) * (pin_stride + 1) <= Ctx::kPinnedDoubles, SADMRG_ERR_LIMIT,
+  SADMRG_REQUIRE((mlanc + 2) * ((kCx<S> ? 2 : 1) + 1) <= Ctx::kLanczosScalars, SADMRG_ERR_LIMIT,
                  "lanczos: mlanc too large for the pinned scalar buffer");
-  double* pin_a = c.h_pinned;                             // Re(a_m) at pin_a[(m-1)*stride]
-  double* pin_b = c.h_pinned + (mlanc + 2) * pin_stride;  // b_m
   int synced = 0;                                          // steps whose a, b are on the host
   auto step = [&](int m, bool reorth) {
+    double* bm = K.beta.template as<double>() + m;
+    S* coef = K.coef.template as<S>();
     matvec(K.F(m - 1), K.F(m));
-    K.mdot(K.F(m - 1), 1, K.F(m), K.dots.get(), 0, K.beta.template as<double>() + (m - 1), K.coef.get());
-    if (m >= 2)
-      launch_multi_axpy(kCx<S>, K.F(m), K.F(m - 2), n, 2, K.coef.get(), n, c.stream);
-    else
-      launch_multi_axpy(kCx<S>, K.F(m), K.F(m - 1), n, 1, K.coef.template as<S>() + 1, n, c.stream);
-    ++c.launches;
+    VecOut o;
+    o.op = VO_COEF;
+    o.beta = bm - 1;
+    o.scal = coef;
+    o.host = K.h_a + (m - 1);
+    K.mdot(K.F(m - 1), 1, K.F(m), K.dots.get(), o);
     if (reorth) {
-      K.mdot(K.F(0), m, K.F(m), K.dots.get());
-      launch_multi_axpy(kCx<S>, K.F(m), K.F(0), n, m, K.dots.get(), n, c.stream);
-      ++c.launches;
+      K.mdot(K.F(0), m, K.F(m), K.dots.get(), VecOut{}, m >= 2 ? K.F(m - 2) : nullptr, K.F(m - 1));
+      K.maxpy(K.F(m), K.F(0), m, K.dots.template as<S>(), bm, K.h_b + m);
+    } else if (m >= 2) {
+      K.maxpy(K.F(m), K.F(m - 2), 2, coef, bm, K.h_b + m);
+    } else {
+      K.maxpy(K.F(m), K.F(m - 1), 1, coef + 1, bm, K.h_b + m);
     }
-    K.mdot(K.F(m), 1, K.F(m), K.dots.get(), 1, nullptr, K.beta.template as<double>() + m);
-    launch_scale_inv(kCx<S>, K.F(m), K.beta.template as<double>() + m, n, c.stream);
-    ++c.launches;
-    SADMRG_CUDA(cudaMemcpyAsync(pin_a + (m - 1) * pin_stride, K.coef.template as<S>() + 1, sizeof(S),
-                                cudaMemcpyDeviceToHost, c.stream));
-    SADMRG_CUDA(cudaMemcpyAsync(pin_b + m, K.beta.template as<double>() + m, sizeof(double), cudaMemcpyDeviceToHost,
-                                c.stream));
+    K.div(K.F(m), K.F(m), nullptr, bm, -1.0);
     st.iters = m;
   };
   // bring a, b of steps (synced, m] to the host; returns the first step in that
@@ -503,8 +521,8 @@ LanczosStats lanczos1(Ctx& c, const HeffPlan<S>& H, S* v, int mlanc, int prec, b
     SADMRG_CUDA(cudaStreamSynchronize(c.stream));
     int brk = 0;
     for (int j = synced + 1; j <= m; ++j) {
-      aal[j - 1] = pin_a[(j - 1) * pin_stride];
-      nnl[j] = pin_b[j];
+      aal[j - 1] = K.h_a[j - 1];
+      nnl[j] = K.h_b[j];
       if (!brk && j >= 2 && nnl[j] < tol) brk = j;
     }
     synced = m;
@@ -521,8 +539,9 @@ LanczosStats lanczos1(Ctx& c, const HeffPlan<S>& H, S* v, int mlanc, int prec, b
       return st;
     }
     matvec(K.F(1), K.F(2));
-    const S a1 = K.dot_host(K.F(1), K.F(2));
-    aal[1] = real_of(a1);
+    K.dots_to_host(K.F(1), 1, K.F(2));
+    SADMRG_CUDA(cudaStreamSynchronize(c.stream));
+    aal[1] = real_of(K.h_dot[0]);
     diatridiag(2);
     ritz_vec(2);
     st.energy = eig[0];
@@ -543,7 +562,7 @@ LanczosStats lanczos1(Ctx& c, const HeffPlan<S>& H, S* v, int mlanc, int prec, b
       st.iters = brk;
       diatridiag(brk - 1);
       ritz_vec(brk - 1);
-      K.scale_host(v, 1.0 / std::sqrt(std::fabs(real_of(K.dot_host(v, v)))));
+      K.div(v, v, nullptr, K.norm(), -1.0);
       st.energy = eig[0];
       return st;
     }
@@ -576,7 +595,9 @@ LanczosStats lanczos1(Ctx& c, const HeffPlan<S>& H, S* v, int mlanc, int prec, b
   }
   sync_to(mlanc - 1);
   matvec(K.F(mlanc - 1), K.F(mlanc));
-  aal[mlanc - 1] = real_of(K.dot_host(K.F(mlanc - 1), K.F(mlanc)));
+  K.dots_to_host(K.F(mlanc - 1), 1, K.F(mlanc));
+  SADMRG_CUDA(cudaStreamSynchronize(c.stream));
+  aal[mlanc - 1] = real_of(K.h_dot[0]);
   diatridiag(mlanc);
   ritz_vec(mlanc);
   if (!variant2) check(ee, ov);

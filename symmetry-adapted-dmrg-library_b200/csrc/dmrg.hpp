@@ -97,7 +97,9 @@ struct HeffBatch {
   std::vector<Part> parts;
   HeffPlan<S> merged;
   std::vector<long long> seg;        // nseg + 1 offsets
-  std::shared_ptr<DevBuf> d_seg;
+  std::shared_ptr<DevBuf> d_blk;     // ranges of the vector kernels over the segments
+  VecSpan span{};
+  int nblk = 0;
   bool ready = false;
   void add(Ctx& c, const HeffPlan<S>& H);
   void finalize(Ctx& c);

@@ -193,42 +193,51 @@ void launch_read(const void* x, long long bytes, unsigned* sink, cudaStream_t s)
 // fill with a constant
 void launch_fill(bool cplx, void* x, double vr, double vi, long long n, cudaStream_t s);
 
-// ---- Krylov vector operations ---------------------------------------------
-// out[j] = <V_j | x> (conjugated first argument), j < nv, deterministic, one launch
-// (counter: a device word, zero between launches).  scalar_op >= 0 also applies a
-// Krylov scalar step to out[0] in the same launch: 0 -> scalar_out[0] =
-// beta_prev[0], scalar_out[1] = Re out[0] (three-term recurrence coefficients);
-// 1 -> scalar_out[0] = sqrt(|Re out[0]|) (a norm).
-void launch_multi_dot(bool cplx, const void* V, long long ldv, int nv, const void* x, long long n,
-                      double* partial, int npart, void* out, unsigned* counter, cudaStream_t s, int scalar_op = -1,
-                      const double* beta_prev = nullptr, void* scalar_out = nullptr);
-// x -= sum_j c[j] V_j   (c read from device memory)
-void launch_multi_axpy(bool cplx, void* x, const void* V, long long ldv, int nv, const void* c, long long n,
-                       cudaStream_t s);
-// x *= 1 / scal[0].  scal is a device double.
-void launch_scale_inv(bool cplx, void* x, const double* scal, long long n, cudaStream_t s);
-// y = sum_j c[j] V_j (host coefficients, real)
-void launch_lincomb(bool cplx, void* y, const void* V, long long ldv, int nv, const double* c_dev, long long n,
-                    cudaStream_t s);
-
-// ---- segmented Krylov operations (independent instances back to back) -----
-// segment s covers [seg[s], seg[s + 1]) of every vector; one block per segment
-// out[s * nv + j] = <V_j | x> on segment s
-void launch_seg_multi_dot(bool cplx, const void* V, long long ldv, int nv, const void* x, const long long* seg,
-                          int nseg, void* out, cudaStream_t s);
-// x -= sum_j c[s * cstride + j] V_j on segment s
-void launch_seg_multi_axpy(bool cplx, void* x, const void* V, long long ldv, int nv, const void* c, int cstride,
-                           const long long* seg, int nseg, cudaStream_t s);
-// x *= scal[s * sstride] (inv = 0) or 1 / scal[s * sstride] (inv = 1) on segment s
-void launch_seg_scale(bool cplx, void* x, const double* scal, int sstride, int inv, const long long* seg, int nseg,
-                      cudaStream_t s);
-// y = sum_j c[s * cstride + j] V_j (real c) on the segments with mask[s] != 0
-void launch_seg_lincomb(bool cplx, void* y, const void* V, long long ldv, int nv, const double* c, int cstride,
-                        const int* mask, const long long* seg, int nseg, cudaStream_t s);
-// per segment: op 0: coef[2s] = beta_prev[s * bstride], coef[2s + 1] = Re(dot[s]); op 1: out[s * ostride] =
-// sqrt(|Re dot[s]|)
-void launch_seg_lanczos_scalar(bool cplx, int op, const void* dot, const double* beta_prev, int bstride, void* out,
-                               int ostride, int nseg, cudaStream_t s);
+// ---- Krylov vector operations (krylov.cu) ----------------------------------
+struct VecBlk {               // one thread block's range of a segment
+  long long lo;
+  int n, seg;
+};
+struct VecSpan {              // the vectors a launch works on: one segment of n elements in ranges of
+  const VecBlk* blk;          // `per` (blk null), or the ranges blk[0 .. nblk) of nseg segments, segment
+  const int* blk0;            // s owning blocks [blk0[s], blk0[s + 1])
+  const int* active;          // null, or per segment: 0 = leave the segment alone
+  long long n, per;
+  int nblk, nseg;
+};
+// one segment of n elements in at most max_blocks ranges
+VecSpan vec_span(long long n, int max_blocks);
+enum VecOp : int {
+  VO_NONE = -1,
+  VO_COEF = 0,                // scal[2 seg] = beta[seg * bstride], scal[2 seg + 1] = Re out[0] (elements of the
+                              // scalar type: the two-term recurrence's coefficients), host = Re out[0]
+  VO_NORM = 1,                // scal[seg * sstride] = host = sqrt(|Re out[0]|) (doubles)
+  VO_HOST = 2                 // host[seg * hstride + j] = out[j] (elements of the scalar type)
+};
+struct VecOut {               // what the last block of a segment does with its sums; host: page-locked
+  int op = VO_NONE;           // host memory (readable after a synchronisation), may be null for VO_NORM
+  const double* beta = nullptr;
+  int bstride = 0;
+  void* scal = nullptr;
+  int sstride = 0;
+  void* host = nullptr;
+  int hstride = 0;
+};
+// out[seg * nv + j] = <V_j | x> (conjugated first argument), after x -= uc[2 seg] u0 + uc[2 seg + 1] u1
+// when u1 is given (u0 may be null).  partial: nblk * nv elements of the scalar type; counter: a zeroed
+// word per segment (left zero).  Deterministic, one launch.
+void launch_vec_dots(bool cplx, const VecSpan& v, const void* V, long long ldv, int nv, void* x, const void* u0,
+                     const void* u1, const void* uc, double* partial, void* out, unsigned* counter, const VecOut& o,
+                     cudaStream_t s);
+// x -= sum_j c[seg * cstride + j] V_j; partial (nblk doubles) given: then |x| as VO_NORM
+void launch_vec_axpy(bool cplx, const VecSpan& v, void* x, const void* V, long long ldv, int nv, const void* c,
+                     int cstride, double* partial, unsigned* counter, const VecOut& o, cudaStream_t s);
+// y = sum_j c[seg * cstride + j] V_j (real c); partial given: then |y| as VO_NORM
+void launch_vec_lincomb(bool cplx, const VecSpan& v, void* y, const void* V, long long ldv, int nv, const double* c,
+                        int cstride, double* partial, unsigned* counter, const VecOut& o, cudaStream_t s);
+// y = x / scal[seg * sstride], copied to y2 when given; a value not above floor divides by 1
+void launch_vec_div(bool cplx, const VecSpan& v, const void* x, void* y, void* y2, const double* scal, int sstride,
+                    double floor, cudaStream_t s);
 
 // ---- one-sided Jacobi SVD of sector blocks --------------------------------
 struct SvdJob {

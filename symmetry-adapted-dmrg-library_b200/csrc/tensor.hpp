@@ -48,8 +48,9 @@ struct Ctx {
   double* d_partial = nullptr;
   unsigned* d_counter = nullptr; // last-block counter of the one-launch reductions (zero between launches)
   double* h_pinned = nullptr;    // page-locked host scratch (kPinnedDoubles) for async scalar reads
-  static constexpr int kPinnedDoubles = 4096;
-  int npart = 296;
+  static constexpr int kPinnedDoubles = 8192;
+  static constexpr int kLanczosScalars = 4096;   // limit of a solve: (mlanc + 2) x (1 + doubles per scalar)
+  int npart = 592;               // most blocks of a vector launch (d_partial: 512 dots of each)
   double lanczos_ov_tol = 1e-8;  // stop when |<v|Hv>|/|Hv| is this close to 1 (src/dmrg_inst.cpp:1338)
   // tcgen05 matvec as one cooperative launch instead of pack + one launch per
   // stage: 1 always, 0 never, -1 (default) for plans below kAutoFuseFlops
