@@ -1,4 +1,4 @@
-// gemm.cu -- grouped block-GEMM executor with deterministic split-K.
+// gemm.cu -- grouped FP64 block-GEMM executor with deterministic split-K.
 //
 // A plan is a list of jobs (output blocks C, m x n) with accumulation lists of
 // terms alpha * op(A) * op(B).  Work is cut into items of one output tile and a
@@ -9,20 +9,14 @@
 // the tile to finish sums the slots in a fixed order -- results are bitwise
 // reproducible and there is no separate reduction launch.
 //
-// Inner loop: operand slabs (BM x BK and BK x BN) are prefetched into registers
-// while the tensor cores work on the slab already in shared memory (two shared
-// buffers, one barrier per slab).  Transposes, conjugation and the term's alpha
-// are applied on the register -> shared store.
-//   FP64   : mma.sync m8n8k4 .f64 (the double-precision tensor path; tcgen05 has
-//            no f64 kind), 64 x 64 tiles, 4 warps of 32 x 32.
-//   3xTF32 : x = hi + lo with hi = tf32(x), lo = tf32(x - hi); hi*hi + hi*lo +
-//            lo*hi on mma.sync m16n8k8 .tf32 with FP32 partial sums folded into
-//            FP64 registers after every slab (Markidis et al. 2018; Ootomo &
-//            Yokota 2022).
+// The products run on the double-precision tensor path (mma.sync m8n8k4 .f64;
+// tcgen05 has no f64 kind).  Every FP64 mma shape runs at the same 36.5-37
+// TFLOP/s here (m8n8k4 at 8 warps per SM: 35.7), plain FMAs at 29.8, so the
+// smallest shape costs nothing and lets a tile skip the 8 x 8 strips that lie
+// outside its block.
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <mutex>
-#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -35,750 +29,376 @@ __device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double
                : "+d"(d0), "+d"(d1)
                : "d"(a), "d"(b));
 }
-
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(r) : "f"(x));
-  return r;
-}
-
-__device__ __forceinline__ void split3(double v, uint32_t& hi, uint32_t& lo) {
-  const float f = (float)v;
-  hi = to_tf32(f);
-  lo = to_tf32(f - __uint_as_float(hi));
-}
-
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// Walk over the slabs of an item: term index t (absolute), offset k inside the term,
-// slab width kt (< BK at a term end or at the end of the item's range).
-struct SlabWalk {
-  int t, k, rem;
-  __device__ bool next(const GemmTerm* terms, int BK, int& tt, int& kk, int& kt) {
-    if (rem <= 0) return false;
-    int tk = terms[t].k;
-    while (k >= tk) { ++t; k = 0; tk = terms[t].k; }
-    tt = t;
-    kk = k;
-    kt = min(BK, min(tk - k, rem));
-    k += kt;
-    rem -= kt;
-    return true;
-  }
+template <bool CX> struct GTile;
+template <> struct GTile<false> {
+  using T = double;
+  static constexpr int BM = 64, BN = 64, BK = 16, PAD = 4;   // PAD: of a k-major row, see items_f64
+};
+template <> struct GTile<true> {
+  using T = double2;
+  static constexpr int BM = 64, BN = 32, BK = 8, PAD = 2;
+};
+constexpr int kF64Stages = 3;
+template <bool CX>
+struct GSmem {
+  using G = GTile<CX>;
+  static constexpr int SKA = G::BM + G::PAD, SKB = G::BN + G::PAD;   // k-major row strides
+  static constexpr int SM = G::BK + 4;                               // m/n-major row stride
+  static constexpr int ABUF = G::BM * SM > G::BK * SKA ? G::BM * SM : G::BK * SKA;
+  static constexpr int BBUF = G::BN * SM > G::BK * SKB ? G::BN * SM : G::BK * SKB;
+  static constexpr int bytes = kF64Stages * (ABUF + BBUF) * (int)sizeof(typename G::T);
 };
 
-// per-thread register slab: A is BM x BK, B is BK x BN (after op), E = elements per thread
-template <class V, int BM, int BN, int BK>
-struct Slab {
-  static constexpr int EA = BM * BK / kThreads, EB = BK * BN / kThreads;
-  V a[EA], b[EB];
+template <bool B> struct BoolC { static constexpr bool value = B; };
+__device__ __forceinline__ double gzero(double) { return 0.0; }
+__device__ __forceinline__ double2 gzero(double2) { return make_double2(0.0, 0.0); }
+__device__ __forceinline__ double gadd(double a, double b) { return a + b; }
+__device__ __forceinline__ double2 gadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
-  __device__ __forceinline__ void load(const GemmTerm& T, const GemmJob& J, int row0, int col0, int k0, int kt,
-                                       const Bases& bases) {
-    const V* A = static_cast<const V*>(bases.p[T.abuf]) + T.aoff;
-    const V* B = static_cast<const V*>(bases.p[T.bbuf]) + T.boff;
-    const bool ta = T.flags & TF_TA, tb = T.flags & TF_TB;
-    const int tid = threadIdx.x;
-#pragma unroll
-    for (int q = 0; q < EA; ++q) {
-      const int e = tid + q * kThreads;
-      int i, kk;
-      if (!ta) { i = e % BM; kk = e / BM; } else { kk = e % BK; i = e / BK; }
-      const int gi = row0 + i;
-      V v = zero();
-      if (gi < J.m && kk < kt) v = ta ? A[(k0 + kk) + (long long)gi * T.lda] : A[gi + (long long)(k0 + kk) * T.lda];
-      a[q] = v;
-    }
-#pragma unroll
-    for (int q = 0; q < EB; ++q) {
-      const int e = tid + q * kThreads;
-      int j, kk;
-      if (!tb) { kk = e % BK; j = e / BK; } else { j = e % BN; kk = e / BN; }
-      const int gj = col0 + j;
-      V v = zero();
-      if (gj < J.n && kk < kt) v = tb ? B[gj + (long long)(k0 + kk) * T.ldb] : B[(k0 + kk) + (long long)gj * T.ldb];
-      b[q] = v;
-    }
-  }
-  static __device__ __forceinline__ V zero() {
-    if constexpr (std::is_same<V, double2>::value) return make_double2(0.0, 0.0);
-    else return 0.0;
-  }
-  // index helpers for the shared-memory store of element q
-  static __device__ __forceinline__ void a_pos(bool ta, int q, int& i, int& kk) {
-    const int e = threadIdx.x + q * kThreads;
-    if (!ta) { i = e % BM; kk = e / BM; } else { kk = e % BK; i = e / BK; }
-  }
-  static __device__ __forceinline__ void b_pos(bool tb, int q, int& j, int& kk) {
-    const int e = threadIdx.x + q * kThreads;
-    if (!tb) { kk = e % BK; j = e / BK; } else { j = e % BN; kk = e / BN; }
-  }
-};
+__device__ __forceinline__ double gmul(double a, double f) { return a * f; }
+__device__ __forceinline__ double2 gmul(double2 a, double f) { return make_double2(a.x * f, a.y * f); }
+__device__ __forceinline__ double gconj(double a, int) { return a; }
+__device__ __forceinline__ double2 gconj(double2 a, int on) { return make_double2(a.x, on ? -a.y : a.y); }
+__device__ __forceinline__ double gscale(double a, double ar, double) { return a * ar; }
+__device__ __forceinline__ double2 gscale(double2 a, double ar, double ai) {
+  return make_double2(a.x * ar - a.y * ai, a.x * ai + a.y * ar);
+}
 
 // ---------------------------------------------------------------------------
-// Split-K fixup, run by every thread of an item that wrote a partial tile: the
-// last item of the tile to finish (per-tile atomic count) sums all its partial
-// tiles in slot order -- the same order whichever item is last -- adds C when
-// the job accumulates, writes C and clears the count for the next launch.
-template <bool CPLX>
-__device__ void split_fixup(const WorkItem& it, const GemmJob& J, const RedItem* __restrict__ reds,
-                            const Bases& bases, const void* work, int* tile_cnt, int BM, int BN) {
+// Split-K fixup, run by every thread of an item that wrote a partial tile: the last
+// item of the tile to finish (per-tile atomic count) sums all its partial tiles in
+// slot order -- the same order whichever item is last -- writes C and clears the count
+// for the next launch.  All of a thread's loads of one slot are in flight together.
+template <bool CX>
+__device__ __forceinline__ void split_fixup(const WorkItem& it, typename GTile<CX>::T* C,
+                                            const typename GTile<CX>::T* work, int* tile_cnt) {
+  using T = typename GTile<CX>::T;
+  constexpr int BM = GTile<CX>::BM, BN = GTile<CX>::BN, E = BM * BN / kThreads;
+  static_assert(kThreads % BM == 0, "a thread keeps its row");
   __shared__ int last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&tile_cnt[it.red], 1) == reds[it.red].nslot - 1;
+  if (threadIdx.x == 0) last = atomicAdd(&tile_cnt[it.red], 1) == it.nslot - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const RedItem R = reds[it.red];
-  const int row0 = R.tm * BM, col0 = R.tn * BN;
-  const bool accum = J.flags & JF_ACCUM;
-  for (int e = threadIdx.x; e < BM * BN; e += blockDim.x) {
-    const int r = e % BM, c = e / BM;
-    if (row0 + r >= J.m || col0 + c >= J.n) continue;
-    const long long idx = (row0 + r) + (long long)(col0 + c) * J.ldc;
-    if (CPLX) {
-      const double2* W = static_cast<const double2*>(work);
-      double2 sum = make_double2(0.0, 0.0);
-      for (int k = 0; k < R.nslot; ++k) {
-        const double2 v = __ldcg(W + (long long)(R.slot0 + k) * BM * BN + e);
-        sum.x += v.x;
-        sum.y += v.y;
-      }
-      double2* C = static_cast<double2*>(bases.p[J.cbuf]) + J.coff;
-      if (accum) { const double2 o = C[idx]; sum.x += o.x; sum.y += o.y; }
-      C[idx] = sum;
-    } else {
-      const double* W = static_cast<const double*>(work);
-      double sum = 0.0;
-      for (int k = 0; k < R.nslot; ++k) sum += __ldcg(W + (long long)(R.slot0 + k) * BM * BN + e);
-      double* C = static_cast<double*>(bases.p[J.cbuf]) + J.coff;
-      C[idx] = accum ? C[idx] + sum : sum;
+  const int r = threadIdx.x % BM, c0 = threadIdx.x / BM;
+  constexpr int CS = kThreads / BM;                 // columns between a thread's elements
+  if (r < it.mv) {
+    T sum[E];
+#pragma unroll
+    for (int u = 0; u < E; ++u) sum[u] = gzero(T());
+    for (int k = 0; k < it.nslot; ++k) {
+      const T* W = work + (long long)(it.slot0 + k) * BM * BN + threadIdx.x;
+#pragma unroll
+      for (int u = 0; u < E; ++u)
+        if (c0 + u * CS < it.nv) sum[u] = gadd(sum[u], __ldcg(W + u * kThreads));
+    }
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+      const int c = c0 + u * CS;
+      if (c < it.nv) C[r + (long long)c * it.ldc] = gmul(sum[u], it.alpha);
     }
   }
   if (threadIdx.x == 0) tile_cnt[it.red] = 0;
 }
 
-// ---------------------------------------------------------------------------
-// FP64, real, multistage: slabs are copied global -> shared with cp.async (8-byte,
-// zero-filled outside the block), STAGES-1 slabs in flight while the tensor cores
-// consume one.  Each operand slab is kept in the layout its global copy is
-// contiguous in (k-major for A, n-major for B when not transposed; the other way
-// when transposed), and the fragment loads follow that layout; row strides of
-// 68 / 20 doubles keep both the copies and the fragment loads conflict free.
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {
+// one element global -> shared, zero-filled instead when !ok (src must still be a valid address)
+__device__ __forceinline__ void cp_elem(double* smem, const double* gmem, bool ok) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  const int n = pred ? 8 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 8 : 0));
+}
+__device__ __forceinline__ void cp_elem(double2* smem, const double2* gmem, bool ok) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 16 : 0));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-template <int BM, int BN, int BK, int STAGES>
-__global__ void __launch_bounds__(kThreads, 3) items_f64_ms(const GemmTerm* __restrict__ terms,
-                                                            const GemmJob* __restrict__ jobs,
-                                                            const WorkItem* __restrict__ items, Bases bases,
-                                                            double* __restrict__ work,
-                                                            const RedItem* __restrict__ reds, int* tile_cnt, const int* mask) {
-  static_assert(BM == 64 && BN == 64 && BK == 16, "layout strides assume 64 x 64 x 16");
-  constexpr int SK = BM + 4;        // k-major row stride (rows of m or n)
-  constexpr int SM = BK + 4;        // m/n-major row stride (rows of k)
-  constexpr int ABUF = (BM * SM > BK * SK) ? BM * SM : BK * SK;
-  constexpr int BBUF = (BN * SM > BK * SK) ? BN * SM : BK * SK;
-  extern __shared__ __align__(16) double smem_ms[];
-  double* As = smem_ms;                         // STAGES x ABUF
-  double* Bs = smem_ms + STAGES * ABUF;         // STAGES x BBUF
-  __shared__ double sh_alpha[STAGES];
-  __shared__ int sh_flags[STAGES];
-  const WorkItem it = items[blockIdx.x];
-  const GemmJob J = jobs[it.job];
-  if (mask && !mask[J.tag]) return;   // instance switched off for this launch
-  const int row0 = it.tm * BM, col0 = it.tn * BN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  constexpr int WM = BM / 2, WN = BN / 2, MT = WM / 8, NT = WN / 8;
-  constexpr int EA = BM * BK / kThreads, EB = BK * BN / kThreads;
-  double acc[MT][NT][2];
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  SlabWalk w{J.t0 + it.t0, it.k0, it.kcount};
+// ---------------------------------------------------------------------------
+struct ItemArgs {             // what a launch is given (kernel parameters, read where needed)
+  const WorkItem* items;
+  const ItemSeg* segs;
+  const int* mask;
+  void* work;
+  int* tile_cnt;
+  Bases bases;
+};
 
-  auto issue = [&](int st, int tt, int k0, int kt) {
-    const GemmTerm T = terms[tt];
-    const bool ta = T.flags & TF_TA, tb = T.flags & TF_TB;
-    const double* A = static_cast<const double*>(bases.p[T.abuf]) + T.aoff;
-    const double* B = static_cast<const double*>(bases.p[T.bbuf]) + T.boff;
-    double* as = As + st * ABUF;
-    double* bs = Bs + st * BBUF;
+// This warp's quarter of one operand slab, global -> shared with cp.async, zero-filled
+// past the block and past the slab's k up to the next multiple of 4 (8 x 8 strips and k
+// steps of 4 that lie outside are neither copied nor read).  The slab is kept in the
+// layout its global copy is contiguous in.  Out-of-range copies read nothing and are
+// given the address of a valid element.
+template <class T, int ROWS, int BK, int SK, int SM>
+__device__ __forceinline__ void copy_slab(T* dst, const T* src, int ld, bool kmajor, int valid, int k0, int kt, int warp,
+                                          int lane) {
+  constexpr int NW = kThreads / 32;
+  if (kmajor) {                        // element (r, k) at src[r + k ld] -> dst[k SK + r]
+    const long long step = (long long)NW * ld;
 #pragma unroll
-    for (int q = 0; q < EA; ++q) {
-      const int e = tid + q * kThreads;
-      int i, kk;
-      if (!ta) { i = e % BM; kk = e / BM; } else { kk = e % BK; i = e / BK; }
-      const int gi = row0 + i;
-      const bool ok = gi < J.m && kk < kt;
-      const double* src = ok ? (ta ? A + (k0 + kk) + (long long)gi * T.lda : A + gi + (long long)(k0 + kk) * T.lda) : A;
-      cp_async8(ta ? as + i * SM + kk : as + kk * SK + i, src, ok);
-    }
+    for (int h = 0; h < ROWS / 32; ++h) {
+      if (h * 32 >= valid) break;
+      const int r = lane + 32 * h;
+      const bool ok = r < valid;
+      T* d = dst + warp * SK + r;
+      if (kt == BK) {
+        const T* s = src + min(r, valid - 1) + (long long)(k0 + warp) * ld;
 #pragma unroll
-    for (int q = 0; q < EB; ++q) {
-      const int e = tid + q * kThreads;
-      int j, kk;
-      if (!tb) { kk = e % BK; j = e / BK; } else { j = e % BN; kk = e / BN; }
-      const int gj = col0 + j;
-      const bool ok = gj < J.n && kk < kt;
-      const double* src = ok ? (tb ? B + gj + (long long)(k0 + kk) * T.ldb : B + (k0 + kk) + (long long)gj * T.ldb) : B;
-      cp_async8(tb ? bs + kk * SK + j : bs + j * SM + kk, src, ok);
-    }
-    if (tid == 0) { sh_alpha[st] = T.ar; sh_flags[st] = T.flags; }
-  };
-
-  int issued = 0;
-#pragma unroll
-  for (int st = 0; st < STAGES - 1; ++st) {
-    int tt, kk, kt;
-    if (w.next(terms, BK, tt, kk, kt)) { issue(st, tt, kk, kt); ++issued; }
-    cp_async_commit();
-  }
-  for (int c = 0; c < issued; ++c) {
-    cp_async_wait<STAGES - 2>();
-    __syncthreads();
-    const int st = c % STAGES;
-    const double alpha = sh_alpha[st];
-    const int fl = sh_flags[st];
-    const bool ta = fl & TF_TA, tb = fl & TF_TB;
-    const double* as = As + st * ABUF;
-    const double* bs = Bs + st * BBUF;
-#pragma unroll
-    for (int k4 = 0; k4 < BK; k4 += 4) {
-      const int k = k4 + (lane & 3);
-      double af[MT], bf[NT];
-#pragma unroll
-      for (int mi = 0; mi < MT; ++mi) {
-        const int r = wm * WM + mi * 8 + (lane >> 2);
-        af[mi] = (ta ? as[r * SM + k] : as[k * SK + r]) * alpha;
-      }
-#pragma unroll
-      for (int ni = 0; ni < NT; ++ni) {
-        const int cc = wn * WN + ni * 8 + (lane >> 2);
-        bf[ni] = tb ? bs[k * SK + cc] : bs[cc * SM + k];
-      }
-#pragma unroll
-      for (int mi = 0; mi < MT; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < NT; ++ni) dmma884(acc[mi][ni][0], acc[mi][ni][1], af[mi], bf[ni]);
-    }
-    int tt, kk, kt;
-    if (w.next(terms, BK, tt, kk, kt)) { issue((c + STAGES - 1) % STAGES, tt, kk, kt); ++issued; }
-    cp_async_commit();
-  }
-  cp_async_wait<0>();
-  const bool direct = it.slot < 0;
-  double* C = direct ? static_cast<double*>(bases.p[J.cbuf]) + J.coff : work + (long long)it.slot * BM * BN;
-  const bool accum = J.flags & JF_ACCUM;
-#pragma unroll
-  for (int mi = 0; mi < MT; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < NT; ++ni)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int r = wm * WM + mi * 8 + (lane >> 2);
-        const int c = wn * WN + ni * 8 + 2 * (lane & 3) + e;
-        if (direct) {
-          if (row0 + r < J.m && col0 + c < J.n) {
-            const long long idx = (row0 + r) + (long long)(col0 + c) * J.ldc;
-            C[idx] = accum ? C[idx] + acc[mi][ni][e] : acc[mi][ni][e];
-          }
-        } else {
-          C[r + c * BM] = acc[mi][ni][e];
+        for (int q = 0; q < BK / NW; ++q) {
+          cp_elem(d + q * NW * SK, s, ok);
+          s += step;
+        }
+      } else {
+        const int kr = (kt + 3) & ~3;
+#pragma unroll 1
+        for (int k = warp; k < kr; k += NW) {
+          cp_elem(d, src + min(r, valid - 1) + (long long)(k0 + min(k, kt - 1)) * ld, ok && k < kt);
+          d += NW * SK;
         }
       }
-  if (it.slot >= 0) split_fixup<false>(it, J, reds, bases, work, tile_cnt, BM, BN);
+    }
+  } else {                             // element (r, k) at src[k + r ld] -> dst[r SM + k]
+    constexpr int RP = 32 / BK, Q = ROWS / RP / NW;   // rows of one warp copy, copies of a warp
+    const int k = lane % BK, r0 = warp * RP + lane / BK;
+    const bool kok = k < kt;
+    const T* s = src + k0 + min(k, kt - 1);
+    T* d = dst + r0 * SM + k;
+    if (valid == ROWS) {
+      const long long step = (long long)(NW * RP) * ld;
+      s += (long long)r0 * ld;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        cp_elem(d + q * NW * RP * SM, s, kok);
+        s += step;
+      }
+    } else {
+      const int r8 = (valid + 7) & ~7;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (q * NW * RP >= r8) break;
+        const int r = q * NW * RP + r0;
+        cp_elem(d + q * NW * RP * SM, s + (long long)min(r, valid - 1) * ld, kok && r < valid);
+      }
+    }
+  }
 }
-constexpr int kF64Stages = 3;
-constexpr size_t kF64MsSmem = (size_t)kF64Stages * 2 * (64 * 20) * sizeof(double);
 
-
-// 3xTF32, real, multistage: the same FP64 slabs as items_f64_ms; operands are
-// rounded to FP32 and split into TF32 hi/lo while the fragments are read.
-template <int BM, int BN, int BK, int STAGES>
-__global__ void __launch_bounds__(kThreads, 3) items_tf32x3_ms(const GemmTerm* __restrict__ terms,
-                                                               const GemmJob* __restrict__ jobs,
-                                                               const WorkItem* __restrict__ items, Bases bases,
-                                                               double* __restrict__ work,
-                                                               const RedItem* __restrict__ reds, int* tile_cnt, const int* mask) {
-  static_assert(BM == 64 && BN == 64 && BK == 16, "layout strides assume 64 x 64 x 16");
-  constexpr int SK = BM + 4, SM = BK + 4;
-  constexpr int ABUF = (BM * SM > BK * SK) ? BM * SM : BK * SK;
-  constexpr int BBUF = (BN * SM > BK * SK) ? BN * SM : BK * SK;
-  extern __shared__ __align__(16) double smem_ms[];
-  double* As = smem_ms;
-  double* Bs = smem_ms + STAGES * ABUF;
-  __shared__ double sh_alpha[STAGES];
-  __shared__ int sh_flags[STAGES];
-  const WorkItem it = items[blockIdx.x];
-  const GemmJob J = jobs[it.job];
-  if (mask && !mask[J.tag]) return;   // instance switched off for this launch
-  const int row0 = it.tm * BM, col0 = it.tn * BN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// One item, by warps that own at most MT x NT strips each.
+template <bool CX, int MT, int NT>
+__device__ __forceinline__ void run_item(const ItemArgs& a, const WorkItem& it, typename GTile<CX>::T* smem) {
+  using G = GTile<CX>;
+  using S = GSmem<CX>;
+  using T = typename G::T;
+  constexpr int STAGES = kF64Stages, NP = CX ? 2 : 1, BK = G::BK;
+  __shared__ double sh_ar[STAGES], sh_ai[STAGES];
+  __shared__ int sh_flags[STAGES], sh_kt[STAGES];
+  T* const As = smem;                        // STAGES x ABUF
+  T* const Bs = smem + STAGES * S::ABUF;     // STAGES x BBUF
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = warp >> 1, wn = warp & 1;
-  const int g = lane >> 2, tg = lane & 3;
-  constexpr int WM = BM / 2, WN = BN / 2, MT = WM / 16, NT = WN / 8;
-  constexpr int EA = BM * BK / kThreads, EB = BK * BN / kThreads;
-  double accd[MT][NT][4];
+  double acc[MT][NT][NP][2];
 #pragma unroll
   for (int i = 0; i < MT; ++i)
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) accd[i][j][e] = 0.0;
-  SlabWalk w{J.t0 + it.t0, it.k0, it.kcount};
-  auto issue = [&](int st, int tt, int k0, int kt) {
-    const GemmTerm T = terms[tt];
-    const bool ta = T.flags & TF_TA, tb = T.flags & TF_TB;
-    const double* A = static_cast<const double*>(bases.p[T.abuf]) + T.aoff;
-    const double* B = static_cast<const double*>(bases.p[T.bbuf]) + T.boff;
-    double* as = As + st * ABUF;
-    double* bs = Bs + st * BBUF;
-#pragma unroll
-    for (int q = 0; q < EA; ++q) {
-      const int e = tid + q * kThreads;
-      int i, kk;
-      if (!ta) { i = e % BM; kk = e / BM; } else { kk = e % BK; i = e / BK; }
-      const int gi = row0 + i;
-      const bool ok = gi < J.m && kk < kt;
-      const double* src = ok ? (ta ? A + (k0 + kk) + (long long)gi * T.lda : A + gi + (long long)(k0 + kk) * T.lda) : A;
-      cp_async8(ta ? as + i * SM + kk : as + kk * SK + i, src, ok);
-    }
-#pragma unroll
-    for (int q = 0; q < EB; ++q) {
-      const int e = tid + q * kThreads;
-      int j, kk;
-      if (!tb) { kk = e % BK; j = e / BK; } else { j = e % BN; kk = e / BN; }
-      const int gj = col0 + j;
-      const bool ok = gj < J.n && kk < kt;
-      const double* src = ok ? (tb ? B + gj + (long long)(k0 + kk) * T.ldb : B + (k0 + kk) + (long long)gj * T.ldb) : B;
-      cp_async8(tb ? bs + kk * SK + j : bs + j * SM + kk, src, ok);
-    }
-    if (tid == 0) { sh_alpha[st] = T.ar; sh_flags[st] = T.flags; }
+      for (int p = 0; p < NP; ++p) acc[i][j][p][0] = acc[i][j][p][1] = 0.0;
+
+  // the slab that is copied next: its segment, first k and width
+  int seg = 0, k0 = 0;
+  ItemSeg sg = a.segs[it.seg0], sn = a.segs[it.seg0 + min(1, it.nseg)];
+  const T *A = nullptr, *B = nullptr;
+  auto bind = [&]() {
+    A = static_cast<const T*>(a.bases.p[sg.abuf]) + sg.aoff;
+    B = static_cast<const T*>(a.bases.p[sg.bbuf]) + sg.boff;
   };
+  bind();
+  auto more = [&]() { return seg < it.nseg; };
+  auto copy_a = [&](int st) {
+    copy_slab<T, G::BM, BK, S::SKA, S::SM>(As + st * S::ABUF, A, sg.lda, !(sg.flags & TF_TA), it.mv, k0,
+                                           min(BK, sg.k - k0), warp, lane);
+    if (threadIdx.x == 0) {
+      sh_ar[st] = sg.ar;
+      sh_ai[st] = sg.ai;
+      sh_flags[st] = sg.flags;
+      sh_kt[st] = min(BK, sg.k - k0);
+    }
+  };
+  auto copy_b = [&](int st) {                // ... and on to the next slab
+    copy_slab<T, G::BN, BK, S::SKB, S::SM>(Bs + st * S::BBUF, B, sg.ldb, sg.flags & TF_TB, it.nv, k0,
+                                           min(BK, sg.k - k0), warp, lane);
+    k0 += BK;
+    if (k0 >= sg.k) {
+      k0 = 0;
+      ++seg;
+      sg = sn;
+      sn = a.segs[it.seg0 + min(seg + 1, it.nseg)];   // a term is often one slab long: loaded one ahead
+      bind();
+    }
+  };
+
   int issued = 0;
-#pragma unroll
+#pragma unroll 1
   for (int st = 0; st < STAGES - 1; ++st) {
-    int tt, kk, kt;
-    if (w.next(terms, BK, tt, kk, kt)) { issue(st, tt, kk, kt); ++issued; }
+    if (more()) {
+      copy_a(st);
+      copy_b(st);
+      ++issued;
+    }
     cp_async_commit();
   }
+#pragma unroll 1
   for (int c = 0; c < issued; ++c) {
     cp_async_wait<STAGES - 2>();
     __syncthreads();
-    const int st = c % STAGES;
-    const double alpha = sh_alpha[st];
-    const int fl = sh_flags[st];
-    const bool ta = fl & TF_TA, tb = fl & TF_TB;
-    const double* as = As + st * ABUF;
-    const double* bs = Bs + st * BBUF;
-    float acc[MT][NT][4];
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-#pragma unroll
-    for (int k8 = 0; k8 < BK; k8 += 8) {
-      uint32_t ah[MT][4], al[MT][4], bh[NT][2], bl[NT][2];
+    const int st = c % STAGES, sw = (c + STAGES - 1) % STAGES;
+    const int fl = sh_flags[st], kt = sh_kt[st];
+    const double ar = sh_ar[st], ai = CX ? sh_ai[st] : 0.0;
+    // fragment addresses: element (row r, k) of the A slab at r * sr + k * sk, of B at c * sc + k * sq
+    const int sr = (fl & TF_TA) ? S::SM : 1, sk = (fl & TF_TA) ? 1 : S::SKA;
+    const int sc = (fl & TF_TB) ? 1 : S::SM, sq = (fl & TF_TB) ? S::SKB : 1;
+    const T* as = As + st * S::ABUF + (wm * 8 + (lane >> 2)) * sr + (lane & 3) * sk;
+    const T* bs = Bs + st * S::BBUF + (wn * 8 + (lane >> 2)) * sc + (lane & 3) * sq;
+    // the products of one k step (4 deep); plain: no scaling or conjugation
+    auto step = [&](auto plain) {
+      T af[MT], bf[NT];
 #pragma unroll
       for (int mi = 0; mi < MT; ++mi) {
-        const int r = wm * WM + mi * 16 + g;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int rr = r + ((e & 1) ? 8 : 0), k = k8 + tg + ((e & 2) ? 4 : 0);
-          split3((ta ? as[rr * SM + k] : as[k * SK + rr]) * alpha, ah[mi][e], al[mi][e]);
-        }
+        af[mi] = as[mi * 16 * sr];
+        if constexpr (!decltype(plain)::value) af[mi] = gscale(gconj(af[mi], fl & TF_CA), ar, ai);
       }
 #pragma unroll
       for (int ni = 0; ni < NT; ++ni) {
-        const int cc = wn * WN + ni * 8 + g;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int k = k8 + tg + (e ? 4 : 0);
-          split3(tb ? bs[k * SK + cc] : bs[cc * SM + k], bh[ni][e], bl[ni][e]);
-        }
+        bf[ni] = bs[ni * 16 * sc];
+        if constexpr (!decltype(plain)::value) bf[ni] = gconj(bf[ni], fl & TF_CB);
       }
 #pragma unroll
       for (int mi = 0; mi < MT; ++mi)
 #pragma unroll
         for (int ni = 0; ni < NT; ++ni) {
-          mma_tf32(acc[mi][ni], al[mi], bh[ni]);
-          mma_tf32(acc[mi][ni], ah[mi], bl[ni]);
-          mma_tf32(acc[mi][ni], ah[mi], bh[ni]);
+          if constexpr (CX) {
+            dmma884(acc[mi][ni][0][0], acc[mi][ni][0][1], af[mi].x, bf[ni].x);
+            dmma884(acc[mi][ni][1][0], acc[mi][ni][1][1], af[mi].x, bf[ni].y);
+          } else {
+            dmma884(acc[mi][ni][0][0], acc[mi][ni][0][1], af[mi], bf[ni]);
+          }
         }
+      if constexpr (CX) {
+#pragma unroll
+        for (int mi = 0; mi < MT; ++mi)
+#pragma unroll
+          for (int ni = 0; ni < NT; ++ni) {
+            dmma884(acc[mi][ni][0][0], acc[mi][ni][0][1], -af[mi].y, bf[ni].y);
+            dmma884(acc[mi][ni][1][0], acc[mi][ni][1][1], af[mi].y, bf[ni].x);
+          }
+      }
+      as += 4 * sk;
+      bs += 4 * sq;
+    };
+    const bool plain = ar == 1.0 && ai == 0.0 && !(CX && (fl & (TF_CA | TF_CB)));
+    const bool next = more();
+    if (next) copy_a(sw);
+    if (plain && kt == BK) {
+#pragma unroll
+      for (int k4 = 0; k4 < BK; k4 += 4) step(BoolC<true>());
+    } else {
+#pragma unroll 1
+      for (int k4 = 0; k4 < kt; k4 += 4) step(BoolC<false>());
     }
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) accd[i][j][e] += (double)acc[i][j][e];
-    int tt, kk, kt;
-    if (w.next(terms, BK, tt, kk, kt)) { issue((c + STAGES - 1) % STAGES, tt, kk, kt); ++issued; }
+    if (next) {
+      copy_b(sw);
+      ++issued;
+    }
     cp_async_commit();
   }
   cp_async_wait<0>();
-  const bool direct = it.slot < 0;
-  double* C = direct ? static_cast<double*>(bases.p[J.cbuf]) + J.coff : work + (long long)it.slot * BM * BN;
-  const bool accum = J.flags & JF_ACCUM;
+  const bool split = it.slot >= 0;
+  const double alpha = split ? 1.0 : it.alpha;
+  T* const C = static_cast<T*>(a.bases.p[it.cbuf]) + it.out;
+  const int ldo = split ? G::BM : it.ldc;
+  T* out = split ? static_cast<T*>(a.work) + (long long)it.slot * G::BM * G::BN : C;
+  out += wm * 8 + (lane >> 2) + (long long)(wn * 8 + 2 * (lane & 3)) * ldo;
 #pragma unroll
-  for (int mi = 0; mi < MT; ++mi)
+  for (int ni = 0; ni < NT; ++ni)
 #pragma unroll
-    for (int ni = 0; ni < NT; ++ni)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = wm * WM + mi * 16 + g + (e >= 2 ? 8 : 0);
-        const int c = wn * WN + ni * 8 + 2 * tg + (e & 1);
-        if (direct) {
-          if (row0 + r < J.m && col0 + c < J.n) {
-            const long long idx = (row0 + r) + (long long)(col0 + c) * J.ldc;
-            C[idx] = accum ? C[idx] + accd[mi][ni][e] : accd[mi][ni][e];
-          }
-        } else {
-          C[r + c * BM] = accd[mi][ni][e];
-        }
-      }
-  if (it.slot >= 0) split_fixup<false>(it, J, reds, bases, work, tile_cnt, BM, BN);
-}
-
-// ---------------------------------------------------------------------------
-// FP64, complex: rr = Re*Re, ii = Im*Im, im = Re*Im + Im*Re; C = rr - ii + i im
-template <int BM, int BN, int BK>
-__global__ void __launch_bounds__(kThreads) items_z64(const GemmTerm* __restrict__ terms, const GemmJob* __restrict__ jobs,
-                                                      const WorkItem* __restrict__ items, Bases bases,
-                                                      double2* __restrict__ work, const RedItem* __restrict__ reds,
-                                                      int* tile_cnt, const int* mask) {
-  constexpr int PAD = 4;
-  __shared__ double Ar[2][BK][BM + PAD], Ai[2][BK][BM + PAD];
-  __shared__ double Br[2][BK][BN + PAD], Bi[2][BK][BN + PAD];
-  using SL = Slab<double2, BM, BN, BK>;
-  const WorkItem it = items[blockIdx.x];
-  const GemmJob J = jobs[it.job];
-  if (mask && !mask[J.tag]) return;   // instance switched off for this launch
-  const int row0 = it.tm * BM, col0 = it.tn * BN;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  constexpr int WM = BM / 2, WN = BN / 2, MT = WM / 8, NT = WN / 8;
-  double rr[MT][NT][2], ii[MT][NT][2], im[MT][NT][2];
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) rr[i][j][e] = ii[i][j][e] = im[i][j][e] = 0.0;
-  SlabWalk w{J.t0 + it.t0, it.k0, it.kcount};
-  SL s;
-  int tt, kk, kt;
-  auto store = [&](int buf, const GemmTerm& T) {
-    const bool ta = T.flags & TF_TA, tb = T.flags & TF_TB;
-    const double ca = (T.flags & TF_CA) ? -1.0 : 1.0, cb = (T.flags & TF_CB) ? -1.0 : 1.0;
-#pragma unroll
-    for (int q = 0; q < SL::EA; ++q) {
-      int i, k;
-      SL::a_pos(ta, q, i, k);
-      const double x = s.a[q].x, y = s.a[q].y * ca;
-      Ar[buf][k][i] = x * T.ar - y * T.ai;
-      Ai[buf][k][i] = x * T.ai + y * T.ar;
-    }
-#pragma unroll
-    for (int q = 0; q < SL::EB; ++q) {
-      int j, k;
-      SL::b_pos(tb, q, j, k);
-      Br[buf][k][j] = s.b[q].x;
-      Bi[buf][k][j] = s.b[q].y * cb;
-    }
-  };
-  int buf = 0;
-  bool have = w.next(terms, BK, tt, kk, kt);
-  if (have) {
-    const GemmTerm T = terms[tt];
-    s.load(T, J, row0, col0, kk, kt, bases);
-    store(0, T);
-  }
-  __syncthreads();
-  while (have) {
-    int t2, k2, kt2;
-    const bool more = w.next(terms, BK, t2, k2, kt2);
-    GemmTerm T2;
-    if (more) { T2 = terms[t2]; s.load(T2, J, row0, col0, k2, kt2, bases); }
-#pragma unroll
-    for (int k4 = 0; k4 < BK; k4 += 4) {
-      double ar[MT], ai[MT], br[NT], bi[NT];
+    for (int e = 0; e < 2; ++e) {
+      T* o = out + (long long)(ni * 16 + e) * ldo;
+      const bool in = (ni * 2 + wn) * 8 + 2 * (lane & 3) + e < it.nv;
 #pragma unroll
       for (int mi = 0; mi < MT; ++mi) {
-        ar[mi] = Ar[buf][k4 + (lane & 3)][wm * WM + mi * 8 + (lane >> 2)];
-        ai[mi] = Ai[buf][k4 + (lane & 3)][wm * WM + mi * 8 + (lane >> 2)];
+        T v;
+        if constexpr (CX) v = make_double2(acc[mi][ni][0][e], acc[mi][ni][1][e]);
+        else v = acc[mi][ni][0][e];
+        if (in && (mi * 2 + wm) * 8 + (lane >> 2) < it.mv) o[mi * 16] = gmul(v, alpha);
       }
-#pragma unroll
-      for (int ni = 0; ni < NT; ++ni) {
-        br[ni] = Br[buf][k4 + (lane & 3)][wn * WN + ni * 8 + (lane >> 2)];
-        bi[ni] = Bi[buf][k4 + (lane & 3)][wn * WN + ni * 8 + (lane >> 2)];
-      }
-#pragma unroll
-      for (int mi = 0; mi < MT; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < NT; ++ni) {
-          dmma884(rr[mi][ni][0], rr[mi][ni][1], ar[mi], br[ni]);
-          dmma884(ii[mi][ni][0], ii[mi][ni][1], ai[mi], bi[ni]);
-          dmma884(im[mi][ni][0], im[mi][ni][1], ar[mi], bi[ni]);
-          dmma884(im[mi][ni][0], im[mi][ni][1], ai[mi], br[ni]);
-        }
     }
-    if (more) store(buf ^ 1, T2);
-    __syncthreads();
-    buf ^= 1;
-    have = more;
-  }
-  const bool direct = it.slot < 0;
-  double2* C = direct ? static_cast<double2*>(bases.p[J.cbuf]) + J.coff : work + (long long)it.slot * BM * BN;
-  const bool accum = J.flags & JF_ACCUM;
-#pragma unroll
-  for (int mi = 0; mi < MT; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < NT; ++ni)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int r = wm * WM + mi * 8 + (lane >> 2);
-        const int c = wn * WN + ni * 8 + 2 * (lane & 3) + e;
-        double2 v = make_double2(rr[mi][ni][e] - ii[mi][ni][e], im[mi][ni][e]);
-        if (direct) {
-          if (row0 + r < J.m && col0 + c < J.n) {
-            const long long idx = (row0 + r) + (long long)(col0 + c) * J.ldc;
-            if (accum) { const double2 o = C[idx]; v.x += o.x; v.y += o.y; }
-            C[idx] = v;
-          }
-        } else {
-          C[r + c * BM] = v;
-        }
-      }
-  if (it.slot >= 0) split_fixup<true>(it, J, reds, bases, work, tile_cnt, BM, BN);
+  if (split) split_fixup<CX>(it, C, static_cast<const T*>(a.work), a.tile_cnt);
 }
 
-// ---------------------------------------------------------------------------
-// 3xTF32 (real and complex), hi/lo planes in shared memory
-template <bool CPLX, int BM, int BN, int BK>
-__global__ void __launch_bounds__(kThreads) items_tf32x3(const GemmTerm* __restrict__ terms,
-                                                         const GemmJob* __restrict__ jobs,
-                                                         const WorkItem* __restrict__ items, Bases bases,
-                                                         void* __restrict__ work, const RedItem* __restrict__ reds,
-                                                         int* tile_cnt, const int* mask) {
-  constexpr int PAD = 8;
-  constexpr int NP = CPLX ? 2 : 1;
-  using V = typename std::conditional<CPLX, double2, double>::type;
-  using SL = Slab<V, BM, BN, BK>;
-  __shared__ uint32_t Ah[2][NP][BK][BM + PAD], Al[2][NP][BK][BM + PAD];
-  __shared__ uint32_t Bh[2][NP][BK][BN + PAD], Bl[2][NP][BK][BN + PAD];
-  const WorkItem it = items[blockIdx.x];
-  const GemmJob J = jobs[it.job];
-  if (mask && !mask[J.tag]) return;   // instance switched off for this launch
-  const int row0 = it.tm * BM, col0 = it.tn * BN;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  const int g = lane >> 2, tg = lane & 3;
-  constexpr int WM = BM / 2, WN = BN / 2, MT = WM / 16, NT = WN / 8;
-  constexpr int NACC = CPLX ? 3 : 1;
-  double accd[NACC][MT][NT][4];
-#pragma unroll
-  for (int q = 0; q < NACC; ++q)
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) accd[q][i][j][e] = 0.0;
-  SlabWalk w{J.t0 + it.t0, it.k0, it.kcount};
-  SL s;
-  int tt, kk, kt;
-  auto store = [&](int buf, const GemmTerm& T) {
-    const bool ta = T.flags & TF_TA, tb = T.flags & TF_TB;
-    const double ca = (T.flags & TF_CA) ? -1.0 : 1.0, cb = (T.flags & TF_CB) ? -1.0 : 1.0;
-#pragma unroll
-    for (int q = 0; q < SL::EA; ++q) {
-      int i, k;
-      SL::a_pos(ta, q, i, k);
-      if constexpr (CPLX) {
-        const double x = s.a[q].x, y = s.a[q].y * ca;
-        split3(x * T.ar - y * T.ai, Ah[buf][0][k][i], Al[buf][0][k][i]);
-        split3(x * T.ai + y * T.ar, Ah[buf][NP - 1][k][i], Al[buf][NP - 1][k][i]);
-      } else {
-        split3(s.a[q] * T.ar, Ah[buf][0][k][i], Al[buf][0][k][i]);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < SL::EB; ++q) {
-      int j, k;
-      SL::b_pos(tb, q, j, k);
-      if constexpr (CPLX) {
-        split3(s.b[q].x, Bh[buf][0][k][j], Bl[buf][0][k][j]);
-        split3(s.b[q].y * cb, Bh[buf][NP - 1][k][j], Bl[buf][NP - 1][k][j]);
-      } else {
-        split3(s.b[q], Bh[buf][0][k][j], Bl[buf][0][k][j]);
-      }
-    }
-  };
-  int buf = 0;
-  bool have = w.next(terms, BK, tt, kk, kt);
-  if (have) {
-    const GemmTerm T = terms[tt];
-    s.load(T, J, row0, col0, kk, kt, bases);
-    store(0, T);
+// The item kernel, real (64 x 64 tiles, slabs of 16 k) and complex (64 x 32, 8): slabs
+// copied global -> shared with cp.async, STAGES-1 in flight while the tensor cores
+// consume one, three CTAs per SM hiding each other's barriers.
+//
+// A full slab is 1024 cycles of an SM's FP64 tensor path against 16 KB of operands, so
+// the bound is that path, if the copies' instructions stay few: blocks start at any
+// element and have odd leading dimensions, so copies are of one element, and with 64-bit
+// addresses formed per element 9 instructions were issued per mma (the path 63% busy on
+// full tiles).  Here a warp steps one address through its quarter of a slab, and the
+// segment after the current one is loaded ahead.
+//
+// Blocks are 1 to some hundreds wide and rarely multiples of 64, so the tile is cut into
+// 8 x 8 strips dealt to the warps in turn (warp row wm takes row strips wm, wm + 2, ...;
+// columns alike), and the item is compiled for 1, 2 or 4 (complex: 1 or 2 column) strips
+// per warp: on 8..512 log-uniform blocks whole 64 x 64 tiles are 1.55 times the useful
+// products.
+//
+// Measured (one H_eff*psi, graph replay): SU(2) D = 512 bond 145 -> 85 us, SU(2) ladder
+// centre 273 -> 216, SU(2) D = 1500 bond 1593 -> 1115 (24.7 TFLOP/s), U(1) D = 64 bond
+// 37 -> 14, complex U(1) D = 1024 bond 2343 -> 1213 (27.3 TFLOP/s).  Tried and slower: a
+// predicate on each mma instead of compiled strip counts (2x); one copying warp beside
+// four multiplying ones (it issues at one warp's rate: 90 us at D = 512); that with
+// persistent CTAs and both stages in one launch (130 us).
+template <bool CX>
+__global__ void __launch_bounds__(kThreads, 3) items_f64(const __grid_constant__ ItemArgs args) {
+  using T = typename GTile<CX>::T;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const WorkItem it = args.items[blockIdx.x];
+  if (args.mask && !args.mask[it.tag]) return;   // instance switched off for this launch
+  T* const smem = reinterpret_cast<T*>(smem_raw);
+  const int mt = (it.mv + 15) >> 4, nt = (it.nv + 15) >> 4;   // strips per warp, at most
+  if (nt <= 1) {
+    if (mt <= 1) run_item<CX, 1, 1>(args, it, smem);
+    else if (mt <= 2) run_item<CX, 2, 1>(args, it, smem);
+    else run_item<CX, 4, 1>(args, it, smem);
+  } else if (CX || nt <= 2) {
+    if (mt <= 1) run_item<CX, 1, 2>(args, it, smem);
+    else if (mt <= 2) run_item<CX, 2, 2>(args, it, smem);
+    else run_item<CX, 4, 2>(args, it, smem);
+  } else if constexpr (!CX) {
+    if (mt <= 1) run_item<CX, 1, 4>(args, it, smem);
+    else if (mt <= 2) run_item<CX, 2, 4>(args, it, smem);
+    else run_item<CX, 4, 4>(args, it, smem);
   }
-  __syncthreads();
-  while (have) {
-    int t2, k2, kt2;
-    const bool more = w.next(terms, BK, t2, k2, kt2);
-    GemmTerm T2;
-    if (more) { T2 = terms[t2]; s.load(T2, J, row0, col0, k2, kt2, bases); }
-    float acc[NACC][MT][NT][4];
-#pragma unroll
-    for (int q = 0; q < NACC; ++q)
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc[q][i][j][e] = 0.f;
-#pragma unroll
-    for (int k8 = 0; k8 < BK; k8 += 8) {
-      uint32_t ah[NP][MT][4], al[NP][MT][4], bh[NP][NT][2], bl[NP][NT][2];
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-#pragma unroll
-        for (int mi = 0; mi < MT; ++mi) {
-          const int r = wm * WM + mi * 16 + g;
-          ah[p][mi][0] = Ah[buf][p][k8 + tg][r];         al[p][mi][0] = Al[buf][p][k8 + tg][r];
-          ah[p][mi][1] = Ah[buf][p][k8 + tg][r + 8];     al[p][mi][1] = Al[buf][p][k8 + tg][r + 8];
-          ah[p][mi][2] = Ah[buf][p][k8 + tg + 4][r];     al[p][mi][2] = Al[buf][p][k8 + tg + 4][r];
-          ah[p][mi][3] = Ah[buf][p][k8 + tg + 4][r + 8]; al[p][mi][3] = Al[buf][p][k8 + tg + 4][r + 8];
-        }
-#pragma unroll
-        for (int ni = 0; ni < NT; ++ni) {
-          const int c = wn * WN + ni * 8 + g;
-          bh[p][ni][0] = Bh[buf][p][k8 + tg][c];     bl[p][ni][0] = Bl[buf][p][k8 + tg][c];
-          bh[p][ni][1] = Bh[buf][p][k8 + tg + 4][c]; bl[p][ni][1] = Bl[buf][p][k8 + tg + 4][c];
-        }
-      }
-#pragma unroll
-      for (int mi = 0; mi < MT; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < NT; ++ni) {
-          if constexpr (CPLX) {
-            mma_tf32(acc[0][mi][ni], al[0][mi], bh[0][ni]);
-            mma_tf32(acc[0][mi][ni], ah[0][mi], bl[0][ni]);
-            mma_tf32(acc[0][mi][ni], ah[0][mi], bh[0][ni]);
-            mma_tf32(acc[1][mi][ni], al[1][mi], bh[1][ni]);
-            mma_tf32(acc[1][mi][ni], ah[1][mi], bl[1][ni]);
-            mma_tf32(acc[1][mi][ni], ah[1][mi], bh[1][ni]);
-            mma_tf32(acc[2][mi][ni], al[0][mi], bh[1][ni]);
-            mma_tf32(acc[2][mi][ni], ah[0][mi], bl[1][ni]);
-            mma_tf32(acc[2][mi][ni], ah[0][mi], bh[1][ni]);
-            mma_tf32(acc[2][mi][ni], al[1][mi], bh[0][ni]);
-            mma_tf32(acc[2][mi][ni], ah[1][mi], bl[0][ni]);
-            mma_tf32(acc[2][mi][ni], ah[1][mi], bh[0][ni]);
-          } else {
-            mma_tf32(acc[0][mi][ni], al[0][mi], bh[0][ni]);
-            mma_tf32(acc[0][mi][ni], ah[0][mi], bl[0][ni]);
-            mma_tf32(acc[0][mi][ni], ah[0][mi], bh[0][ni]);
-          }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < NACC; ++q)
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) accd[q][i][j][e] += (double)acc[q][i][j][e];
-    if (more) store(buf ^ 1, T2);
-    __syncthreads();
-    buf ^= 1;
-    have = more;
-  }
-  const bool direct = it.slot < 0;
-  const bool accum = J.flags & JF_ACCUM;
-#pragma unroll
-  for (int mi = 0; mi < MT; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < NT; ++ni)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = wm * WM + mi * 16 + g + (e >= 2 ? 8 : 0);
-        const int c = wn * WN + ni * 8 + 2 * tg + (e & 1);
-        if constexpr (CPLX) {
-          double2 v = make_double2(accd[0][mi][ni][e] - accd[1][mi][ni][e], accd[NACC - 1][mi][ni][e]);
-          if (direct) {
-            if (row0 + r < J.m && col0 + c < J.n) {
-              double2* C = static_cast<double2*>(bases.p[J.cbuf]) + J.coff;
-              const long long idx = (row0 + r) + (long long)(col0 + c) * J.ldc;
-              if (accum) { const double2 o = C[idx]; v.x += o.x; v.y += o.y; }
-              C[idx] = v;
-            }
-          } else {
-            static_cast<double2*>(work)[(long long)it.slot * BM * BN + r + c * BM] = v;
-          }
-        } else {
-          const double v = accd[0][mi][ni][e];
-          if (direct) {
-            if (row0 + r < J.m && col0 + c < J.n) {
-              double* C = static_cast<double*>(bases.p[J.cbuf]) + J.coff;
-              const long long idx = (row0 + r) + (long long)(col0 + c) * J.ldc;
-              C[idx] = accum ? C[idx] + v : v;
-            }
-          } else {
-            static_cast<double*>(work)[(long long)it.slot * BM * BN + r + c * BM] = v;
-          }
-        }
-      }
-  if (it.slot >= 0) split_fixup<CPLX>(it, J, reds, bases, work, tile_cnt, BM, BN);
 }
 
-int gemm_tile_m(bool cplx, int /*prec*/) { return cplx ? 32 : 64; }
-int gemm_tile_n(bool cplx, int /*prec*/) { return cplx ? 32 : 64; }
+int gemm_tile_m(bool cplx) { return cplx ? GTile<true>::BM : GTile<false>::BM; }
+int gemm_tile_n(bool cplx) { return cplx ? GTile<true>::BN : GTile<false>::BN; }
 
-void launch_items(bool cplx, int prec, const GemmTerm* terms, const GemmJob* jobs, const WorkItem* items, int nitems,
-                  const Bases& b, void* work, const RedItem* reds, int* tile_cnt, const int* mask,
-                  cudaStream_t s) {
+template <bool CX>
+static void launch_items_t(const ItemArgs& a, int nitems, cudaStream_t s) {
+  static unsigned char attr[kMaxDevices] = {0};
+  ensure_smem_attr((const void*)items_f64<CX>, GSmem<CX>::bytes, attr);
+  items_f64<CX><<<nitems, kThreads, GSmem<CX>::bytes, s>>>(a);
+}
+
+void launch_items(bool cplx, const WorkItem* items, const ItemSeg* segs, int nitems, const Bases& b, void* work,
+                  int* tile_cnt, const int* mask, cudaStream_t s) {
   if (nitems <= 0) return;
-  if (prec == PREC_TF32X3) {
-    if (cplx) {
-      items_tf32x3<true, 32, 32, 16><<<nitems, kThreads, 0, s>>>(terms, jobs, items, b, work, reds, tile_cnt, mask);
-    } else {
-      static unsigned char attr[kMaxDevices] = {0};
-      ensure_smem_attr((const void*)items_tf32x3_ms<64, 64, 16, kF64Stages>, (int)kF64MsSmem, attr);
-      items_tf32x3_ms<64, 64, 16, kF64Stages><<<nitems, kThreads, kF64MsSmem, s>>>(terms, jobs, items, b,
-                                                                                 static_cast<double*>(work), reds,
-                                                                                 tile_cnt, mask);
-    }
-  } else {
-    if (cplx) {
-      items_z64<32, 32, 16><<<nitems, kThreads, 0, s>>>(terms, jobs, items, b, static_cast<double2*>(work), reds,
-                                                          tile_cnt, mask);
-    } else {
-      static unsigned char attr[kMaxDevices] = {0};
-      ensure_smem_attr((const void*)items_f64_ms<64, 64, 16, kF64Stages>, (int)kF64MsSmem, attr);
-      items_f64_ms<64, 64, 16, kF64Stages><<<nitems, kThreads, kF64MsSmem, s>>>(terms, jobs, items, b,
-                                                                              static_cast<double*>(work), reds,
-                                                                              tile_cnt, mask);
-    }
-  }
+  const ItemArgs a{items, segs, mask, work, tile_cnt, b};
+  if (cplx) launch_items_t<true>(a, nitems, s);
+  else launch_items_t<false>(a, nitems, s);
 }
 
 // ---------------------------------------------------------------------------

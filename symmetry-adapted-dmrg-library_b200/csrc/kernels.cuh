@@ -30,29 +30,35 @@ struct GemmJob {              // C (m x n, column-major, ldc) receives its terms
   int tag;                    // instance of a merged batch plan (0 otherwise): a launch given a mask
                               // skips every item of a job whose mask[tag] is 0
 };
-struct GemmTile {
-  int job, tm, tn;
-};
 struct WorkItem {             // one output tile x a contiguous range of the job's concatenated k
-  int job, tm, tn;
-  int t0, k0, kcount;         // first term (relative to the job's t0), offset in it, total k
+  long long out;              // element offset of the tile's (0, 0) in C
+  double alpha;               // C = alpha sum(terms)
+  int cbuf, ldc, mv, nv;      // mv x nv: the tile's extent inside the block
+  int tag;                    // as GemmJob::tag
+  int seg0, nseg;             // its segments
   int slot;                   // < 0: write C directly; otherwise the partial-tile slot
-  int red;                    // split items: their tile's RedItem
+  int red;                    // split items: their tile's counter, and the tile's slots
+  int slot0, nslot;           // [slot0, slot0 + nslot), summed in this order
+  int pad;
 };
-struct RedItem {              // C tile = sum of slots [slot0, slot0 + nslot) (fixed order)
-  int job, tm, tn, slot0, nslot;
+struct ItemSeg {              // a run of k inside one term of an item; A, B: first element of the tile's rows / columns
+  long long aoff, boff;
+  int abuf, bbuf, lda, ldb, k, flags;
+  double ar, ai;
+  long long pad;
 };
+static_assert(sizeof(WorkItem) == 64 && sizeof(ItemSeg) == 64, "one 64-byte load each");
 struct Bases {
   void* p[kMaxBases];
 };
 
 
-// Grouped GEMM over work items (deterministic split-K; see gemm.cu).
+// Grouped FP64 GEMM over work items (deterministic split-K; see gemm.cu).
 // Split items write partial tiles; the last of a tile's items sums them (tile_cnt
-// holds one zeroed counter per RedItem and is left zeroed).
+// holds one zeroed counter per split tile and is left zeroed).
 // mask: null, or per job tag; items of a job with mask[tag] == 0 do nothing.
-void launch_items(bool cplx, int prec, const GemmTerm* terms, const GemmJob* jobs, const WorkItem* items, int nitems,
-                  const Bases& b, void* work, const RedItem* reds, int* tile_cnt, const int* mask, cudaStream_t s);
+void launch_items(bool cplx, const WorkItem* items, const ItemSeg* segs, int nitems, const Bases& b, void* work,
+                  int* tile_cnt, const int* mask, cudaStream_t s);
 
 // ---- tcgen05 3xTF32 over TF32 hi/lo operand panels (umma.cu) --------------
 // An operand (rows x K after op) is stored as panels: panel (p, s) holds rows
@@ -147,8 +153,8 @@ constexpr size_t kNoAllocScratchBytes = (size_t)32 << 20;
 // Device address of that scratch on the current device (looked up once per
 // device); returns 0 or a cudaError_t value.
 int noalloc_scratch(void** ptr);
-int gemm_tile_m(bool cplx, int prec);
-int gemm_tile_n(bool cplx, int prec);
+int gemm_tile_m(bool cplx);
+int gemm_tile_n(bool cplx);
 
 // ---- block utilities -------------------------------------------------------
 struct Seg {                  // y[doff + i] (+)= alpha * x[soff + i], i < n

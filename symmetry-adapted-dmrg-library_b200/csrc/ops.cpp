@@ -87,60 +87,123 @@ void GemmPlan::add_term(int job, int abuf, long long aoff, int lda, int bbuf, lo
   job_terms[job].push_back(t);
 }
 
-void GemmPlan::build_schedule(GemmSchedule& sc, bool cplx) {
+// Items of the FP64 kernel (gemm.cu).  A full 64 x 64 (complex 64 x 32) tile takes
+// 256 (512) cycles of an SM's tensor path per k step of 4, a smaller one in
+// proportion to its 8 x 8 strips, with ~64 cycles of latency at least.  Long items set
+// a stage's time, since three CTAs share an SM and the last ones run alone, and every
+// piece of a split reduction pays for a partial tile and the fix-up; so reductions are
+// cut where they exceed a sixth (complex: a sixteenth) of an SM's share of the stage,
+// but not below 128 of k.  Shares of 1/3, 1/6 and 1/16: 233, 216 and 241 us on the
+// SU(2) ladder centre (8..512 blocks), 1147, 1115 and 1142 us at D = 1500; complex U(1)
+// D = 1024: 1328, 1329 and 1213 us.  scale > 1 lengthens the pieces (fewer slots).
+//
+// A stage-0 result (buffer 3) takes over the scale that all its readers apply, when
+// they agree (scaling an element before it is stored or after it is loaded rounds alike).
+void GemmPlan::build_schedule(GemmSchedule& sc, bool cplx, double scale) {
   const int BM = sc.bm, BN = sc.bn;
   sc.items.clear();
-  sc.reds.clear();
+  sc.segs.clear();
   sc.stage_items.assign(nstage + 1, 0);
-  sc.stage_reds.assign(nstage + 1, 0);
+  sc.nred = 0;
+  std::map<long long, int> producer;   // offset of a stage-0 result -> its job
+  for (size_t j = 0; j < jobs.size(); ++j)
+    if (jobs[j].cbuf == 3 && job_stage[j] == 0) producer[jobs[j].coff] = (int)j;
+  std::vector<int> read(jobs.size(), 0), alike(jobs.size(), 1);
+  std::vector<double> alpha(jobs.size(), 1.0);
+  auto source = [&](const GemmTerm& t) -> int {
+    SADMRG_REQUIRE(t.bbuf != 3, SADMRG_ERR_STATE, "plan: a stage-0 result as right operand");
+    if (t.abuf != 3) return -1;
+    const auto it = producer.find(t.aoff);
+    SADMRG_REQUIRE(it != producer.end(), SADMRG_ERR_STATE, "plan: a stage-0 result that nothing writes");
+    return it->second;
+  };
+  for (auto& list : job_terms)
+    for (const GemmTerm& t : list) {
+      const int p = source(t);
+      if (p < 0) continue;
+      if (!read[p]) alpha[p] = t.ar;
+      read[p] = 1;
+      if (t.ai != 0.0 || t.ar != alpha[p]) alike[p] = 0;
+    }
+  for (size_t j = 0; j < jobs.size(); ++j)
+    if (!alike[j]) alpha[j] = 1.0;
+  auto step_cycles = [&](int m, int n) {   // of a tile with m x n inside the block, per 4 of k
+    const long long strips = (long long)((m + 7) / 8) * ((n + 7) / 8);
+    return std::max<long long>(64, strips * (cplx ? 16 : 4));
+  };
+  const int nsm = device_sm_count();
   int nslot = 0;
   for (int s = 0; s < nstage; ++s) {
-    // split-K chunk: enough items to fill the GPU, never below 128 of k
-    long long total = 0;
+    std::vector<long long> ktot(jobs.size(), 0);
+    double total = 0.0;
     for (size_t j = 0; j < jobs.size(); ++j) {
       if (job_stage[j] != s) continue;
-      long long kt = 0;
-      for (auto& t : job_terms[j]) kt += t.k;
-      total += (long long)((jobs[j].m + BM - 1) / BM) * ((jobs[j].n + BN - 1) / BN) * std::max<long long>(kt, 1);
+      for (auto& t : job_terms[j]) ktot[j] += t.k;
+      for (int a = 0; a < jobs[j].m; a += BM)
+        for (int b = 0; b < jobs[j].n; b += BN)
+          total += (double)step_cycles(std::min(BM, jobs[j].m - a), std::min(BN, jobs[j].n - b)) * ((ktot[j] + 3) / 4);
     }
-    long long ntile = 0;
-    for (size_t j = 0; j < jobs.size(); ++j)
-      if (job_stage[j] == s)
-        ntile += (long long)((jobs[j].m + BM - 1) / BM) * ((jobs[j].n + BN - 1) / BN);
-    // split the reduction only when the output tiles alone cannot fill the GPU
-    long long kc = (total + target_items - 1) / std::max(target_items, 1);
-    kc = std::max<long long>(128, (kc + 15) / 16 * 16);
-    if (ntile >= target_items / 2) kc = (long long)1 << 40;
+    const double limit = std::max(1.0, scale * total / ((cplx ? 16.0 : 6.0) * nsm));
     std::vector<std::pair<long long, WorkItem>> its;
     for (size_t j = 0; j < jobs.size(); ++j) {
       if (job_stage[j] != s) continue;
-      long long kt = 0;
-      for (auto& t : job_terms[j]) kt += t.k;
-      if (kt == 0 && (jobs[j].flags & JF_ACCUM)) continue;
-      const int tm = (jobs[j].m + BM - 1) / BM, tn = (jobs[j].n + BN - 1) / BN;
-      const long long nch = std::max<long long>(1, (kt + kc - 1) / kc);
-      for (int a = 0; a < tm; ++a)
-        for (int b = 0; b < tn; ++b) {
-          if (nch == 1) {
-            its.push_back({kt, WorkItem{(int)j, a, b, 0, 0, (int)kt, -1, -1}});
-            continue;
+      const GemmJob& J = jobs[j];
+      const long long kt = ktot[j];
+      SADMRG_REQUIRE(!(J.flags & JF_ACCUM), SADMRG_ERR_STATE, "plan: FP64 jobs overwrite their block");
+      for (int r0 = 0; r0 < J.m; r0 += BM)
+        for (int c0 = 0; c0 < J.n; c0 += BN) {
+          WorkItem w{};
+          w.out = J.coff + r0 + (long long)c0 * J.ldc;
+          w.alpha = alpha[j];
+          w.cbuf = J.cbuf;
+          w.ldc = J.ldc;
+          w.mv = std::min(BM, J.m - r0);
+          w.nv = std::min(BN, J.n - c0);
+          w.tag = J.tag;
+          w.slot = -1;
+          const long long cyc = step_cycles(w.mv, w.nv);
+          long long kc = std::max<long long>(128, (long long)std::min(limit / (double)cyc * 4.0, 1e15));
+          long long nch = std::max<long long>(1, (kt + kc - 1) / kc);
+          kc = ((kt + nch - 1) / nch + 15) / 16 * 16;       // pieces of equal length
+          nch = std::max<long long>(1, (kt + kc - 1) / std::max<long long>(kc, 1));
+          if (nch > 1) {
+            w.slot0 = nslot;
+            w.nslot = (int)nch;
+            w.red = sc.nred++;
           }
-          const int slot0 = nslot, red = (int)sc.reds.size();
-          long long pos = 0;
-          int t = 0, k = 0;
+          size_t t = 0;
+          int k = 0;
           for (long long ch = 0; ch < nch; ++ch) {
-            const long long len = std::min(kc, kt - pos);
-            its.push_back({len, WorkItem{(int)j, a, b, t, k, (int)len, nslot++, red}});
-            // advance (t, k) by len along the concatenated k
-            long long left = len;
-            while (left > 0) {
-              const int avail = job_terms[j][t].k - k;
-              if (left < avail) { k += (int)left; left = 0; }
-              else { left -= avail; ++t; k = 0; }
+            const long long len = std::min(kc, kt - ch * kc);
+            w.seg0 = (int)sc.segs.size();
+            for (long long left = len; left > 0;) {          // [k, k + take) of term t
+              const GemmTerm& T = job_terms[j][t];
+              const int take = (int)std::min<long long>(left, T.k - k);
+              if (take > 0) {
+                const bool ta = T.flags & TF_TA, tb = T.flags & TF_TB;
+                const int p = source(T);
+                ItemSeg g{};
+                g.aoff = T.aoff + (ta ? k + (long long)r0 * T.lda : r0 + (long long)k * T.lda);
+                g.boff = T.boff + (tb ? c0 + (long long)k * T.ldb : k + (long long)c0 * T.ldb);
+                g.abuf = T.abuf;
+                g.bbuf = T.bbuf;
+                g.lda = T.lda;
+                g.ldb = T.ldb;
+                g.k = take;
+                g.flags = T.flags;
+                g.ar = T.ar;
+                g.ai = T.ai;
+                if (p >= 0 && alike[p]) g.ar = 1.0;
+                sc.segs.push_back(g);
+              }
+              left -= take;
+              k += take;
+              if (k == T.k) { ++t; k = 0; }
             }
-            pos += len;
+            w.nseg = (int)sc.segs.size() - w.seg0;
+            if (nch > 1) w.slot = nslot++;
+            its.push_back({cyc * ((len + 3) / 4), w});
           }
-          sc.reds.push_back(RedItem{(int)j, a, b, slot0, (int)nch});
         }
     }
     // longest work first
@@ -149,14 +212,42 @@ void GemmPlan::build_schedule(GemmSchedule& sc, bool cplx) {
     sc.stage_items[s] = (int)sc.items.size();
     for (auto& p : its) sc.items.push_back(p.second);
     sc.stage_items[s + 1] = (int)sc.items.size();
-    sc.stage_reds[s + 1] = (int)sc.reds.size();
   }
-  for (int s = 0; s < nstage; ++s) {
-    sc.stage_items[s + 1] = std::max(sc.stage_items[s + 1], sc.stage_items[s]);
-    sc.stage_reds[s + 1] = std::max(sc.stage_reds[s + 1], sc.stage_reds[s]);
-  }
+  for (int s = 0; s < nstage; ++s) sc.stage_items[s + 1] = std::max(sc.stage_items[s + 1], sc.stage_items[s]);
+  sc.segs.push_back(ItemSeg{});   // the entry an item without terms at the end points to
   sc.nslot = nslot;
-  (void)cplx;
+}
+
+// Most bytes of partial tiles a schedule may take so that the plan fits the fixed
+// scratch of the allocation-free entry point whenever it would with partial tiles
+// of at least 128 of k cut to about 8 per SM, the size that limit was set for;
+// unlimited for plans that never fit.
+size_t GemmPlan::slot_budget(bool cplx) const {
+  const size_t elem = cplx ? sizeof(dcmplex) : sizeof(double);
+  const size_t xbytes = ((size_t)scratch_elems * elem + 255) & ~size_t(255);
+  const int tile = cplx ? 32 : 64, target = 148 * 8;
+  long long slots = 0;
+  for (int s = 0; s < nstage; ++s) {
+    long long total = 0, ntile = 0;
+    std::vector<std::pair<long long, long long>> tk;   // (tiles, k) per job
+    for (size_t j = 0; j < jobs.size(); ++j) {
+      if (job_stage[j] != s) continue;
+      long long kt = 0;
+      for (auto& t : job_terms[j]) kt += t.k;
+      const long long nt = (long long)((jobs[j].m + tile - 1) / tile) * ((jobs[j].n + tile - 1) / tile);
+      ntile += nt;
+      total += nt * std::max<long long>(kt, 1);
+      tk.push_back({nt, kt});
+    }
+    if (ntile >= target / 2) continue;
+    const long long kc = std::max<long long>(128, ((total + target - 1) / target + 15) / 16 * 16);
+    for (auto& p : tk) {
+      const long long nch = (p.second + kc - 1) / kc;
+      if (nch > 1) slots += p.first * nch;
+    }
+  }
+  const size_t then = (size_t)std::max<long long>(slots, 1) * tile * tile * elem;
+  return xbytes + then <= kNoAllocScratchBytes ? kNoAllocScratchBytes - xbytes : ~size_t(0);
 }
 
 void GemmPlan::finalize(Ctx& c, bool cplx, bool mixed, const Bases* const_bases) {
@@ -171,29 +262,25 @@ void GemmPlan::finalize(Ctx& c, bool cplx, bool mixed, const Bases* const_bases)
     }
   }
   sched = GemmSchedule{};
-  sched.bm = gemm_tile_m(cplx, 0);
-  sched.bn = gemm_tile_n(cplx, 0);
-  build_schedule(sched, cplx);
+  sched.bm = gemm_tile_m(cplx);
+  sched.bn = gemm_tile_n(cplx);
+  const size_t slot_bytes = (size_t)sched.bm * sched.bn * (cplx ? 16 : 8), budget = slot_budget(cplx);
+  for (double scale = 1.0; ; scale *= 2.0) {
+    build_schedule(sched, cplx, scale);
+    if (sched.nslot * slot_bytes <= budget || sched.nslot == 0) break;
+  }
 
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const size_t bt = sizeof(GemmTerm) * flat_terms.size(), bj = sizeof(GemmJob) * jobs.size(),
-               bi = sizeof(WorkItem) * sched.items.size(), br = sizeof(RedItem) * sched.reds.size();
-  const size_t total = al(bt) + al(bj) + al(bi) + al(br) + 256;
-  std::vector<unsigned char> h(total, 0);
-  if (bt) std::memcpy(h.data(), flat_terms.data(), bt);
-  if (bj) std::memcpy(h.data() + al(bt), jobs.data(), bj);
-  if (bi) std::memcpy(h.data() + al(bt) + al(bj), sched.items.data(), bi);
-  if (br) std::memcpy(h.data() + al(bt) + al(bj) + al(bi), sched.reds.data(), br);
-  dev = std::make_shared<DevBuf>(total, c.stream);
-  SADMRG_CUDA(cudaMemcpyAsync(dev->get(), h.data(), total, cudaMemcpyHostToDevice, c.stream));
-  unsigned char* base = dev->as<unsigned char>();
-  d_terms = reinterpret_cast<GemmTerm*>(base);
-  d_jobs = reinterpret_cast<GemmJob*>(base + al(bt));
-  sched.d_items = reinterpret_cast<WorkItem*>(base + al(bt) + al(bj));
-  sched.d_reds = reinterpret_cast<RedItem*>(base + al(bt) + al(bj) + al(bi));
-  sched.work = std::make_shared<DevBuf>((size_t)std::max(sched.nslot, 1) * sched.bm * sched.bn * (cplx ? 16 : 8),
-                                        c.stream);
-  sched.tile_cnt = std::make_shared<DevBuf>(sizeof(int) * std::max<size_t>(sched.reds.size(), 1), c.stream);
+  const size_t bi = sizeof(WorkItem) * sched.items.size(), bs = sizeof(ItemSeg) * sched.segs.size();
+  std::vector<unsigned char> h(al(bi) + bs, 0);
+  if (bi) std::memcpy(h.data(), sched.items.data(), bi);
+  std::memcpy(h.data() + al(bi), sched.segs.data(), bs);
+  dev = std::make_shared<DevBuf>(h.size(), c.stream);
+  SADMRG_CUDA(cudaMemcpyAsync(dev->get(), h.data(), h.size(), cudaMemcpyHostToDevice, c.stream));
+  sched.d_items = dev->as<WorkItem>();
+  sched.d_segs = reinterpret_cast<ItemSeg*>(dev->as<unsigned char>() + al(bi));
+  sched.work = std::make_shared<DevBuf>(sched.nslot * slot_bytes, c.stream);
+  sched.tile_cnt = std::make_shared<DevBuf>(sizeof(int) * std::max(sched.nred, 1), c.stream);
   SADMRG_CUDA(cudaMemsetAsync(sched.tile_cnt->get(), 0, sched.tile_cnt->bytes(), c.stream));
   umma.reset();
   if (mixed && const_bases) {
@@ -205,8 +292,8 @@ void GemmPlan::finalize(Ctx& c, bool cplx, bool mixed, const Bases* const_bases)
 }
 
 // tcgen05 schedule (see UmmaSchedule).  Returns false, leaving umma empty, when
-// some term does not fit the panel scheme; the plan then runs 3xTF32 on the
-// mma.sync kernels.
+// some term does not fit the panel scheme; the plan then runs in FP64 at either
+// precision (no H_eff plan has such a term).
 bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
   auto U = std::make_shared<UmmaSchedule>();
   const int nsm = device_sm_count();
@@ -547,7 +634,7 @@ int GemmPlan::launches_per_run(bool cplx, int prec, bool c_fused) const {
   if (uses_umma(cplx, prec)) {
     const UmmaSchedule& U = *umma;
     if (c_fused) return 1;   // pack + both stages in one launch
-    int n = U.vblk.empty() ? 0 : 1;
+    n = U.vblk.empty() ? 0 : 1;
     for (int s = 0; s < nstage; ++s)
       if (U.stage_items[s + 1] > U.stage_items[s]) ++n;
     return n;
@@ -664,8 +751,8 @@ void GemmPlan::run(Ctx& c, bool cplx, int prec, const Bases& b, int stage_lo, in
   for (int s = stage_lo; s < stage_hi; ++s) {
     const int ni = sched.stage_items[s + 1] - sched.stage_items[s];
     if (ni > 0) {
-      launch_items(cplx, prec, d_terms, d_jobs, sched.d_items + sched.stage_items[s], ni, b, wk, sched.d_reds,
-                   sched.tile_cnt->as<int>(), c.job_mask, c.stream);
+      launch_items(cplx, sched.d_items + sched.stage_items[s], sched.d_segs, ni, b, wk, sched.tile_cnt->as<int>(),
+                   c.job_mask, c.stream);
       ++c.launches;
       mark(c, 1 + 2 * s);
     }

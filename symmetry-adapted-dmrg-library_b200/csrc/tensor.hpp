@@ -105,18 +105,17 @@ template <class S> std::vector<Blk> blocks_of(const BTensor<S>& t);
 template <class S> BTensor<S> alloc_tensor(Ctx& c, const Struct& st, const std::vector<char>& present);
 template <class S> BTensor<S> clone(Ctx& c, const BTensor<S>& t);
 
-// Work items and split-K reductions of a plan for the mma.sync item kernels.
+// Work items and split-K reductions of a plan for the FP64 item kernel.
 struct GemmSchedule {
   int bm = 64, bn = 64;
   std::vector<WorkItem> items;
-  std::vector<RedItem> reds;
+  std::vector<ItemSeg> segs;
   std::vector<int> stage_items;   // item offsets per stage (size nstage+1)
-  std::vector<int> stage_reds;    // reduction offsets per stage (size nstage+1)
   WorkItem* d_items = nullptr;
-  RedItem* d_reds = nullptr;
+  ItemSeg* d_segs = nullptr;
   std::shared_ptr<DevBuf> work;   // split-K partial tiles
-  std::shared_ptr<DevBuf> tile_cnt;   // per RedItem: items finished in the current launch
-  int nslot = 0;
+  std::shared_ptr<DevBuf> tile_cnt;   // per split tile: items finished in the current launch
+  int nslot = 0, nred = 0;        // partial tiles, split tiles
   size_t work_bytes() const { return work ? work->bytes() : 0; }
 };
 
@@ -159,13 +158,10 @@ struct GemmPlan {
   int nstage = 2;
   // device copy
   std::vector<GemmTerm> flat_terms;
-  GemmSchedule sched;                  // mma.sync items (FP64, and 3xTF32 when there is no tcgen05 schedule)
+  GemmSchedule sched;                  // FP64 items
   std::shared_ptr<UmmaSchedule> umma;  // tcgen05 3xTF32 (real plans finalised with mixed = true)
-  std::shared_ptr<DevBuf> dev;
-  GemmTerm* d_terms = nullptr;
-  GemmJob* d_jobs = nullptr;
+  std::shared_ptr<DevBuf> dev;         // items and segments
   long long flops = 0;            // algorithmic flops of one execution (real multiply-adds * 2)
-  int target_items = 148 * 8;     // work items per stage the split-K aims for
   UmmaTune tune;                  // tcgen05 tile choice (build_umma reads it)
   Bases const_bases{};            // where the constant panels come from (kept for rebuilds)
 
@@ -203,7 +199,8 @@ struct GemmPlan {
   std::string tune_key(bool cplx) const;
 
  private:
-  void build_schedule(GemmSchedule& s, bool cplx);
+  void build_schedule(GemmSchedule& s, bool cplx, double scale);
+  size_t slot_budget(bool cplx) const;
   bool build_umma(Ctx& c, const Bases& cb, bool cplx);
 };
 
