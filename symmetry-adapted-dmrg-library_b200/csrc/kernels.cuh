@@ -253,10 +253,9 @@ struct SvdJob {
   long long soff;             // singular values (double), min(m,n)
   int m, n, trans;            // trans = 1 when m < n (work on A^H)
 };
-// Host driver: one launch per round of block pairs, one sync per sweep to test
-// convergence.  Returns the sweeps taken, or -1 if max_sweeps was reached.
-// kernel_ms (optional): device time of the sweep kernel when it ran as one launch
-// (with the QR preconditioning: plus the QR and the Q application).
+// Host driver: all sweeps in one cooperative launch.  Returns the sweeps taken, or -1 if
+// max_sweeps was reached.  kernel_ms (optional): device time of that launch (with the
+// QR preconditioning: plus the QR and the Q application).
 // precondition: Jacobi on R1^H after Householder QRs of the norm-ordered columns
 // and of R^H (fewer sweeps): 0 never, 1 when the widest block has at least 32
 // columns, 2 always; the outputs have the same meaning either way.

@@ -8,8 +8,7 @@
 // are ordered by decreasing norm at the start of every sweep and split into
 // column blocks of b = 8 or 16 (chosen per call).  Every round of a sweep
 // pairs the blocks by the circle method; one CTA forms the 2b x 2b Gram matrix
-// of its pair on the FP64
-// tensor cores (DMMA, W streamed in row chunks), runs a cyclic sweep of the
+// of its pair on the FP64 tensor cores (DMMA), runs a cyclic sweep of the
 // one-sided rotations on it, and applies the accumulated 2b x 2b rotation to
 // the pair's columns of W and V (DMMA again).  Sweeps repeat until a full sweep
 // performs no rotation, so the result keeps the columnwise relative accuracy of
@@ -18,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "common.hpp"
@@ -29,8 +29,10 @@ constexpr int kSvdThreads = 512;
 constexpr int kSvdWarps = kSvdThreads / 32;
 // columns per block (a visit takes two blocks): 8 or 16, chosen per call by run_jacobi_svd
 
-struct SvdPair {
-  int job, bi, bj, b;   // column blocks bi, bj (bj < 0: bi alone); b = block width
+// What one CTA of the Jacobi kernel does: sectors order[j0 .. j0 + nj - 1] one after
+// another, as CTA `rank` of the `size` that share each of them and barrier `group`.
+struct SvdCta {
+  int group, rank, size, j0, nj;
 };
 
 template <bool CPLX> struct SvdT;
@@ -58,6 +60,8 @@ __device__ __forceinline__ double cconj(double a) { return a; }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double cre(double a) { return a; }
 __device__ __forceinline__ double cre(double2 a) { return a.x; }
+__device__ __forceinline__ double cim(double) { return 0.0; }
+__device__ __forceinline__ double cim(double2 a) { return a.y; }
 template <class T> __device__ __forceinline__ T czero();
 template <> __device__ __forceinline__ double czero<double>() { return 0.0; }
 template <> __device__ __forceinline__ double2 czero<double2>() { return make_double2(0.0, 0.0); }
@@ -81,237 +85,354 @@ __device__ __forceinline__ double pow2_scale_of(double m) {
 // r = sqrt(d^2 + 4 g^2).  With u = |d| + r and q = 1 / sqrt(2 r u) (since
 // 1 + t^2 = 2 r / u): c = cos(theta) = u q, s = sin(theta) = 2 g q sgn(d) and
 // t = 4 g r q^2 sgn(d) -- two inverse square roots and no division on the chain
-// that sets the time of an inner round.  d and g are first scaled by a power of two
-// (the larger of |d| and 2 g into [1, 2)), so that the squares neither overflow nor
-// underflow; c, s and t do not depend on the scale.  Returns c, s and t g.
-__device__ __forceinline__ void jacobi_rotation(double a, double b, double g, double& c, double& s, double& tg) {
-  const double d = b - a;
-  const double sc = pow2_scale_of(fmax(fabs(d), 2.0 * g));
-  const double dn = d * sc, gn = g * sc;
-  const double x = fma(dn, dn, 4.0 * gn * gn);
-  const double r = x * rsqrt(x);
-  const double u = fabs(dn) + r;
-  const double q = rsqrt(2.0 * r * u);
-  const double sg = d >= 0.0 ? 1.0 : -1.0;
+// that sets the time of an inner round.  d and g are first scaled by a power of two,
+// so that the squares neither overflow nor underflow; c, s and t do not depend on the
+// scale.  The scale takes the larger of a and b, which bounds |d| and (up to rounding) g,
+// into [1, 2): known before g is.  Returns c, s sgn (sgn = 1 or -1) and t g.
+__device__ __forceinline__ void jacobi_rotation(double a, double b, double g, double sgn, double& c, double& s,
+                                                double& tg) {
+  const double d = b - a, sc = pow2_scale_of(fmax(a, b)), sd = d >= 0.0 ? 1.0 : -1.0;
+  const double dn = fabs(d) * sc, h = g * (2.0 * sc);
+  const double x = fma(dn, dn, __dmul_rn(h, h));
+  const double r = __dmul_rn(x, rsqrt(x));
+  const double u = __dadd_rn(dn, r);
+  const double q = rsqrt(__dmul_rn(2.0 * r, u));
   c = u * q;
-  s = sg * (2.0 * gn * q);
-  tg = sg * (4.0 * gn * r * q * q) * g;
+  s = (sd * sgn * h) * q;
+  tg = (2.0 * h * r * q * q) * (sd * g);
 }
 
-// One element (8 or 16 bytes) copied global -> shared without passing through
-// registers (cp.async, Ampere and later); zero-filled instead when !ok (src must
-// still be a valid address).
-template <class T>
-__device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool ok) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(T) == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(src), "r"(ok ? 16 : 0) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(src), "r"(ok ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// all but the most recently committed group of this thread's copies have landed
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+constexpr int kChunk = 128;            // rows per streamed chunk of W
 
-constexpr int kChunk = 128;            // rows per streamed chunk of W or V
-constexpr int kInnerMax = 1;           // inner sweeps of one visit (more cut outer sweeps by less than they cost)
-
-template <int B>                       // B: columns per block
+template <bool CPLX, int B>            // B: columns per block
 struct SvdGeom {
   static constexpr int Nc = 2 * B;                          // columns of one visit
   static constexpr int TD = Nc / 8;                         // 8 x 8 DMMA tiles along one side of G
-  static constexpr int Ld = Nc + 1;                         // row stride of G, Q and the row chunk
-  static constexpr int ChunkPer = kChunk * Nc / kSvdThreads;   // chunk elements per thread
+  // strides in shared memory, in elements, are 32 bytes past a multiple of 128: the four
+  // rows and four columns that half a warp reads of a DMMA fragment then lie in different
+  // banks (at Nc + 1 the Gram of a 128-row chunk took 5,200 cycles, four times its mma)
+  static constexpr int Pad = CPLX ? 2 : 4;
+  static constexpr int Ld = Nc + Pad;                       // rows of G, columns of Q
+  static constexpr int LdC = kChunk + Pad;                  // columns of a row chunk of W
+  // columns of all rows of W or V (a resident visit)
+  __host__ __device__ static constexpr int ldr(int rows) { return ((rows + 15) & ~15) + Pad; }
+  static constexpr int Split = B == 8 ? 4 : 1;              // row parts of a resident visit's Gram
+  static constexpr int TU = TD * (TD + 1) / 2;              // tiles on and above the diagonal
+  static constexpr int Units = B == 8 ? 1 : 4;              // of a streamed one: GramUnit
+  // threads of the inner sweep: a deciding warp, one thread per 2 x 2 block of G, and
+  // those that rotate Q
+  static constexpr int GT = B * B, QT = B == 8 ? 64 : 128;
+  static constexpr int IT = 32 + GT + QT;
+  static_assert(IT <= kSvdThreads && GT % 32 == 0 && QT % Nc == 0, "threads of a visit");
 };
 
 template <bool CPLX, int B>
-constexpr size_t svd_smem_bytes() {   // G, Q and two row-chunk buffers
-  return (size_t)(2 * SvdGeom<B>::Nc + 2 * kChunk) * SvdGeom<B>::Ld * (CPLX ? 16 : 8);
+constexpr size_t svd_smem_bytes() {   // G twice, Q and two row-chunk buffers
+  using Gm = SvdGeom<CPLX, B>;
+  return (size_t)(3 * Gm::Ld + 2 * Gm::LdC) * Gm::Nc * (CPLX ? 16 : 8);
 }
-// shared memory of a resident visit (all rows of the pair's W and V columns) of a
-// block with R + C rows in total; launches whose largest pair needs more stream
-// row chunks instead
+// shared memory of a resident visit (all rows of the pair's W and V columns) of an
+// R x C block; launches whose largest pair needs more stream row chunks instead
 template <bool CPLX, int B>
-constexpr size_t svd_res_smem_bytes(long long rows) {
-  return (size_t)(2 * SvdGeom<B>::Nc + rows) * SvdGeom<B>::Ld * (CPLX ? 16 : 8) + (size_t)kSvdWarps * 32 * 4 * 8;
+constexpr size_t svd_res_smem_bytes(int R, int C) {
+  using Gm = SvdGeom<CPLX, B>;
+  return (size_t)(3 * Gm::Ld + Gm::ldr(R) + Gm::ldr(C)) * Gm::Nc * (CPLX ? 16 : 8) + (size_t)kSvdWarps * 32 * 4 * 8;
 }
-constexpr size_t kSvdResMax = 160 * 1024;
+constexpr size_t kSvdResMax = 188 * 1024;
+
+// Tiles of G on and above the diagonal that one warp forms, from the fragments of nl
+// column groups of 8: tile t is between the groups l[x[t]] and l[y[t]] (l, x and y are
+// lists of digits, the first lowest).  Of 4 groups
+// (B = 16) by four warps, of 2 (B = 8) by one as the last two of 4: 10 fragments for 10
+// mma instead of 20, which took as long as the mma.
+template <int U> struct GramUnit;
+__device__ constexpr int digit(int list, int i) { return list >> 4 * i & 15; }
+template <> struct GramUnit<0> { static constexpr int nl = 2, nt = 2, l = 0x10, x = 0x00, y = 0x10; };
+template <> struct GramUnit<1> { static constexpr int nl = 3, nt = 2, l = 0x320, x = 0x00, y = 0x21; };
+template <> struct GramUnit<2> { static constexpr int nl = 3, nt = 3, l = 0x321, x = 0x000, y = 0x210; };
+template <> struct GramUnit<3> { static constexpr int nl = 2, nt = 3, l = 0x32, x = 0x100, y = 0x110; };
+
+__device__ __forceinline__ void gram_mma(double* g, double x, double y) { dmma(g[0], g[1], x, y); }
+__device__ __forceinline__ void gram_mma(double* g, double2 x, double2 y) {   // conj(x) y
+  dmma(g[0], g[1], x.x, y.x);
+  dmma(g[0], g[1], x.y, y.y);
+  dmma(g[2], g[3], x.x, y.y);
+  dmma(g[2], g[3], -x.y, y.x);
+}
+// g[t] += tiles of unit U over the k steps k0, k0 + STEP, ... < k1 of four rows each, of
+// columns at D (column-major, stride ldd; D points to this lane's row and column)
+template <int U, int TD, int STEP, class T, int NG>
+__device__ __forceinline__ void gram_unit(const T* D, int ldd, int k0, int k1, double (&g)[3][NG]) {
+  using Un = GramUnit<U>;
+#pragma unroll 4
+  for (int k = k0; k < k1; k += STEP) {
+    T f[Un::nl];
+#pragma unroll
+    for (int i = 0; i < Un::nl; ++i) f[i] = D[(digit(Un::l, i) - 4 + TD) * 8 * ldd + k];
+#pragma unroll
+    for (int t = 0; t < Un::nt; ++t) gram_mma(g[t], f[digit(Un::x, t)], f[digit(Un::y, t)]);
+  }
+}
+template <int TD, int STEP, class T, int NG>
+__device__ __forceinline__ void gram_any(int unit, const T* D, int ldd, int k0, int k1, double (&g)[3][NG]) {
+  if constexpr (TD == 2) {
+    gram_unit<3, TD, STEP>(D, ldd, k0, k1, g);
+  } else {
+    if (unit == 0) gram_unit<0, TD, STEP>(D, ldd, k0, k1, g);
+    else if (unit == 1) gram_unit<1, TD, STEP>(D, ldd, k0, k1, g);
+    else if (unit == 2) gram_unit<2, TD, STEP>(D, ldd, k0, k1, g);
+    else gram_unit<3, TD, STEP>(D, ldd, k0, k1, g);
+  }
+}
+
+template <int U, int TD, class F, int NG>
+__device__ __forceinline__ void gram_unit_tiles(F f, const double (&g)[3][NG]) {
+  using Un = GramUnit<U>;
+#pragma unroll
+  for (int t = 0; t < Un::nt; ++t)
+    f(digit(Un::l, digit(Un::x, t)) - 4 + TD, digit(Un::l, digit(Un::y, t)) - 4 + TD, g[t]);
+}
+// f(row tile, column tile, sums) for the tiles of a unit
+template <int TD, class F, int NG>
+__device__ __forceinline__ void gram_tiles(int unit, F f, const double (&g)[3][NG]) {
+  if (TD == 2 || unit == 3) gram_unit_tiles<3, TD>(f, g);
+  else if (unit == 0) gram_unit_tiles<0, TD>(f, g);
+  else if (unit == 1) gram_unit_tiles<1, TD>(f, g);
+  else gram_unit_tiles<2, TD>(f, g);
+}
+
+// A pair's rotation, c and s e^{i phi} (on = 0: none).
+struct SvdRot {
+  double c, sr, si;
+  int on;
+};
+// Columns x, y <- c x - conj(s) y, s x + c y.  The real form names its roundings: the
+// signs of singular vectors of blocks of about 1,400 columns depend on each.
+__device__ __forceinline__ void rot_cols(double& x, double& y, const SvdRot& t) {
+  const double u = x, v = y;
+  x = __fma_rn(t.c, u, -__dmul_rn(t.sr, v));
+  y = __fma_rn(t.sr, u, __dmul_rn(t.c, v));
+}
+__device__ __forceinline__ void rot_cols(double2& x, double2& y, const SvdRot& t) {
+  const double2 u = x, v = y, ep = make_double2(t.sr, t.si), em = make_double2(-t.sr, t.si);
+  x = cadd(make_double2(t.c * u.x, t.c * u.y), cmul(v, em));
+  y = cadd(cmul(u, ep), make_double2(t.c * v.x, t.c * v.y));
+}
+// rows x, y <- c x - s y, conj(s) x + c y
+__device__ __forceinline__ void rot_rows(double& x, double& y, const SvdRot& t) { rot_cols(x, y, t); }
+__device__ __forceinline__ void rot_rows(double2& x, double2& y, const SvdRot& t) {
+  const double2 u = x, v = y, mp = make_double2(-t.sr, -t.si), pm = make_double2(t.sr, -t.si);
+  x = cadd(make_double2(t.c * u.x, t.c * u.y), cmul(mp, v));
+  y = cadd(cmul(pm, u), make_double2(t.c * v.x, t.c * v.y));
+}
+// the first or second of the two that rot_cols (row = 0) or rot_rows (row = 1) returns
+__device__ __forceinline__ double rot_one(double u, double v, const SvdRot& t, bool second, int) {
+  const double a = second ? t.sr : t.c, b = second ? t.c : -t.sr;
+  const double w = __fma_rn(a, u, __dmul_rn(b, v));
+  return t.on ? w : second ? v : u;
+}
+__device__ __forceinline__ double2 rot_one(double2 u, double2 v, const SvdRot& t, bool second, int row) {
+  double2 x = u, y = v;
+  if (row) rot_rows(x, y, t);
+  else rot_cols(x, y, t);
+  return second ? (t.on ? y : v) : (t.on ? x : u);
+}
+
+// A pair of a round: its columns p < q (p + 256 q) and the 2 x 2 block of the round
+// before that its G_pq comes from: rows of pair i, columns of pair j (j + 256 i), p and q
+// being the second of them (+ 32768, + 128), and the offsets of its entries in G.
+struct alignas(16) SvdLook {
+  unsigned short o00, o01, o10, o11, pq, ij;
+};
+
+template <class P>
+__device__ __forceinline__ void swap_ptr(P*& a, P*& b) { P* const t = a; a = b; b = t; }
+
+// pair k of round rnd of the circle method over N (even) columns, p < q
+__device__ __forceinline__ void circle_pair(int N, int rnd, int k, int& p, int& q) {
+  int u = rnd + k, v = k == 0 ? N - 1 : rnd - k;
+  if (u >= N - 1) u -= N - 1;
+  if (v < 0) v += N - 1;
+  p = min(u, v);
+  q = max(u, v);
+}
 
 // One visit of a column-block pair (Hestenes one-sided Jacobi in Gram form):
-//   1. G = Wp^H Wp for the pair's nc <= 2B columns Wp, streamed from W in row chunks;
+//   1. G = Wp^H Wp for the pair's nc <= 2B columns Wp;
 //   2. cyclic one-sided Jacobi on G: rotation (p, q) from a = G_pp, b = G_qq,
 //      g = G_pq exactly as on the columns themselves, G <- J^H G J, Q <- Q J,
-//      with the rotated diagonal set to a - t|g|, b + t|g| and G_pq to 0; up to
-//      kInnerMax sweeps, stopping after a sweep that rotates nothing;
-//   3. Wp <- Wp Q and Vp <- Vp Q, streamed in row chunks.
-// Only G, Q and one row chunk live in shared memory, so the visit width does not
-// depend on the height of the block -- or, when the launch's largest pair fits
-// (res), all rows of the pair's columns of W and V: one load, the Gram tiles with
-// their rows split over all warps (partials summed in a fixed order), and Q applied
-// in place by warps that own whole 8-row tiles.  The rotations rotate the Gram entries of
-// the columns exactly as the column updates would (a rotation that mixes a small
-// column with a large one has |s| <= sqrt(a_small / a_large)), so the entries
-// keep the columnwise relative accuracy of the direct method; W itself changes
-// only by the orthogonal Q.  Adds the number of rotations to *rotations.  Every
-// thread of the block calls it; 16 warps, warp k owns pair k of each round.
-template <bool CPLX, int B>
-__device__ void jacobi_pair_visit(const SvdJob& J, const SvdPair& P, void* work, void* vmat, const int* perm,
-                                  double tol, unsigned char* smem_raw, int* rotations, bool res) {
+//      with the rotated diagonal set to a - t|g|, b + t|g| and G_pq to 0 (one sweep:
+//      more cut the outer sweeps by less than they cost);
+//   3. Wp <- Wp Q and Vp <- Vp Q.
+// The rotations rotate the Gram entries of the columns exactly as the column updates
+// would (a rotation that mixes a small column with a large one has |s| <=
+// sqrt(a_small / a_large)), so the entries keep the columnwise relative accuracy of the
+// direct method; W itself changes only by the orthogonal Q.  Adds the number of
+// rotations to *rotations.  Every thread of the block calls it.
+//
+// The Gram and the application of Q run on the FP64 tensor cores.  When the launch's
+// largest pair fits in shared memory (RES) the pair's W columns are read there first and
+// its V columns by idle warps during part 2; otherwise half of the warps read W in row
+// chunks while the others form the Gram, and the application reads its fragments straight
+// from L2.  Only the Gram tiles on and above the diagonal are formed, and new columns go
+// from registers to memory.
+//
+// Part 2 is a chain of Nc - 1 rounds and the longest part of a resident visit: a load of
+// the deciding entries, two inverse square roots and a barrier.  One warp computes the
+// rotations and runs a round ahead: the entry G_pq that decides a pair of the next round
+// comes from one 2 x 2 block of G and two rotations of this round, so it computes that
+// entry itself (SvdLook) while others, one thread per 2 x 2 block, write the rotated G to
+// a second copy and others again rotate Q.  The deciding warp passes alone over rounds in
+// which no pair rotates.  950 cycles a round (b = 8) and 1,130 (b = 16), after 1,300 with
+// the test, the rotations and the rotation of G one after another.
+//
+// Cycles of a visit, real: b = 8, 344 x 344 (D = 512): load 1,340, Gram 2,350, part 2
+// 14,000, part 3 5,200, between visits 5,000: 4.6 ms of Jacobi after 7.8; b = 16,
+// 1,319 x 1,319 (D = 2,048): Gram 32,600, part 2 35,000, part 3 63,600 (44,000 of mma),
+// between visits 11,500: 46.9 ms after 115.
+//
+// The sums run in a fixed order: of a resident visit's Gram in kSplit row parts of one
+// chain each, of a streamed one over even and odd k steps apart.  With blocks of about
+// 1,400 columns the signs of singular vectors depend on every rounding, so the orders
+// are part of the result.
+template <bool CPLX, int B, bool RES>
+__device__ __forceinline__ void jacobi_pair_visit(typename SvdT<CPLX>::T* W, int R, typename SvdT<CPLX>::T* V, int C, const int* cols,
+                                  int nc, double tol, unsigned char* smem_raw, SvdLook (*looks)[B], int& looks_n, int* rotations) {
   using T = typename SvdT<CPLX>::T;
-  constexpr int kNc = SvdGeom<B>::Nc, kTD = SvdGeom<B>::TD, kLdG = SvdGeom<B>::Ld;
-  constexpr int kChunkPer = SvdGeom<B>::ChunkPer;
-  static_assert(kSvdWarps * 2 >= kNc, "one warp per column pair of a round");
-  const int R = J.trans ? J.n : J.m;
-  const int C = J.trans ? J.m : J.n;
-  __shared__ int cols[kNc];
-  T* G = reinterpret_cast<T*>(smem_raw);   // kNc x kLdG, row-major
-  T* Q = G + kNc * kLdG;
-  T* Ck = Q + kNc * kLdG;                  // kChunk x kLdG: rows of W or V, row-major
+  using Gm = SvdGeom<CPLX, B>;
+  constexpr int kNc = Gm::Nc, kTD = Gm::TD, kLdG = Gm::Ld, kTU = Gm::TU, kSplit = Gm::Split, kUnits = Gm::Units;
+  constexpr int kE = CPLX ? 4 : 2;
+  __shared__ double dg[kNc];             // the diagonal of G
+  // by pair of the round: its rotation, its columns p < q as p + 256 q + 65536 on
+  __shared__ double par_c[2][B], par_sr[2][B], par_si[2][CPLX ? B : 1];
+  __shared__ int par_pq[2][B];
+  __shared__ int msg[2];                 // 1: par holds rotations (2: the last), 0: it holds none, -1: end
+  __shared__ int nrot_sh;
+  T* G = reinterpret_cast<T*>(smem_raw); // kNc x kLdG, row-major
+  T* G2 = G + kNc * kLdG;                // the other copy of G
+  T* Q = G2 + kNc * kLdG;                // kNc x kLdG, column-major
+  T* Ck = Q + kNc * kLdG;                // two row chunks of W, column-major
   // resident visit: all R rows of the pair's W columns, then all C rows of its V columns
+  const int ldw = Gm::ldr(R), ldv = Gm::ldr(C);
   T* Ws = Ck;
-  T* Vs = Ws + R * kLdG;
-  double* Gp = reinterpret_cast<double*>(Vs + C * kLdG);   // Gram partials, 4 per lane per warp
-  T* W = static_cast<T*>(work) + J.woff;
-  T* V = static_cast<T*>(vmat) + J.voff;
+  T* Vs = Ws + kNc * ldw;
+  double* Gp = reinterpret_cast<double*>(Vs + kNc * ldv);   // Gram partials, 4 per lane per warp
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int nc = 0;
-  {
-    const int n0 = min(P.b, C - P.bi * P.b);
-    const int n1 = P.bj >= 0 ? min(P.b, C - P.bj * P.b) : 0;
-    nc = n0 + n1;
-    // block position -> column through the job's current order (columns by decreasing norm)
-    const int* pj = perm + J.soff;
-    if (tid < n0) cols[tid] = pj[P.bi * P.b + tid];
-    else if (tid < nc) cols[tid] = pj[P.bj * P.b + (tid - n0)];
-  }
-  __syncthreads();
-
-  // 1. Gram matrix on the FP64 tensor cores: warp w < kTD^2 owns the 8 x 8 tile
-  //    (w / kTD, w % kTD) of G = Wp^H Wp; k runs over the rows of the chunk
-  //    (zero-filled past the block)
-  static_assert(kNc % 8 == 0 && kTD * kTD <= kSvdWarps, "one warp per Gram tile");
-  constexpr int kTiles = kTD * kTD, kSplit = kSvdWarps / kTiles;
-  const bool gram_warp = warp < kTiles;
-  const int fr = lane >> 2, fk = lane & 3;
-  double g0 = 0.0, g1 = 0.0, h0 = 0.0, h1 = 0.0;   // Re (and Im) of D(fr, 2 fk + i)
-  // Streamed visits: row chunks of a column set (W or V) copied asynchronously
-  // into two shared buffers, the next chunk in flight while one is multiplied
-  // (rows past the block and columns past nc zero-filled); one group per chunk.
-  T* const Cb0 = Ck;
-  T* const Cb1 = Ck + kChunk * kLdG;
-  auto issue = [&](const T* M, int ld, int r0, int rows, T* dst) {
+  // Rows r0, r0 + 32, ... of column c of M (zeros past the column or past nc): read
+  // together, so that a thread's loads are in flight at once (cp.async of 8 bytes
+  // passed at 12 bytes a cycle: 7,500 cycles for 350 rows of W and V)
+  auto load = [&](const T* M, int ld, int c, int r0, auto& v) {
+    const T* src = M + (long long)cols[min(c, nc - 1)] * ld;
 #pragma unroll
-    for (int u = 0; u < kChunkPer; ++u) {
-      const int e = tid + u * kSvdThreads, r = e % kChunk, c = e / kChunk;
-      const bool ok = r < rows && c < nc;
-      cp_async_elem(dst + r * kLdG + c, ok ? M + (r0 + r) + (long long)cols[c] * ld : M, ok);
-    }
-    cp_async_commit();
+    for (int u = 0; u < (int)(sizeof(v) / sizeof(T)); ++u)
+      v[u] = c < nc && r0 + u * 32 < ld ? __ldcg(src + r0 + u * 32) : czero<T>();
   };
-  if (res) {
-    // one load of everything the visit touches (columns past nc zero-filled), then
-    // the Gram tiles with their rows split over all warps: warp w computes tile
-    // w % kTiles over the w / kTiles-th part of the rows; the parts are summed in
-    // part order
-    // one thread per row of W then V, its columns read into registers together so
-    // that all of a thread's loads are in flight at once (coalesced along rows)
-    constexpr int kU = CPLX ? 8 : 16;
-    for (int r0 = 0; r0 < R + C; r0 += kSvdThreads) {
-      const int rr = r0 + tid;
-      if (rr < R + C) {
-        const bool isw = rr < R;
-        const int r = isw ? rr : rr - R, ld = isw ? R : C;
-        const T* M = isw ? W : V;
-        T* D = (isw ? Ws : Vs) + r * kLdG;
+  // all rows of the columns of M, and zeros to a multiple of four, by nw warps
+  auto load_all = [&](const T* M, int ld, T* dst, int ldd, int w, int nw) {
+    T v[CPLX ? 6 : 12];
+    const int ldz = (ld + 3) & ~3;
+    constexpr int kU = sizeof(v) / sizeof(T);
+    for (int c = w; c < kNc; c += nw)
+      for (int r0 = lane; r0 < ldz; r0 += 32 * kU) {
+        load(M, ld, c, r0, v);
 #pragma unroll
-        for (int c0 = 0; c0 < kNc; c0 += kU) {
-          T v[kU];
-#pragma unroll
-          for (int u = 0; u < kU; ++u) v[u] = c0 + u < nc ? M[r + (long long)cols[c0 + u] * ld] : czero<T>();
-#pragma unroll
-          for (int u = 0; u < kU; ++u) D[c0 + u] = v[u];
-        }
+        for (int u = 0; u < kU; ++u)
+          if (r0 + u * 32 < ldz) dst[c * ldd + r0 + u * 32] = v[u];
       }
-    }
+  };
+
+  // 1. Gram matrix
+  const int fr = lane >> 2, fk = lane & 3;
+  // tiles of this warp, a resident visit: one in one part of the rows; streamed: GramUnit
+  double g[RES ? 1 : 3][kE] = {};   // Re (and Im) of D(fr, 2 fk + i)
+  int pt = 0, qt = 0, unit = warp % kUnits;
+  bool gram_warp = warp < (RES ? kTU : kUnits);   // of which the tiles are stored
+  if constexpr (RES) {
+    load_all(W, R, Ws, ldw, warp, kSvdWarps);
+    qt = warp % kTU;
+    while (qt >= kTD - pt) { qt -= kTD - pt; ++pt; }
+    qt += pt;
+    const int part = warp / kTU;
     __syncthreads();
-    const int tile = warp % kTiles, part = warp / kTiles;
-    const int pt = tile / kTD, qt = tile % kTD;
-    const int rs = (((R + kSplit - 1) / kSplit) + 3) & ~3;
-    const int k0s = part * rs, k1s = min(R, k0s + rs);
-    for (int k0 = k0s; k0 < k1s; k0 += 4) {
-      const int k = k0 + fk;
-      const T x = k < k1s ? Ws[k * kLdG + pt * 8 + fr] : czero<T>();   // A(p, r) = conj(W(r, p))
-      const T y = k < k1s ? Ws[k * kLdG + qt * 8 + fr] : czero<T>();   // B(r, q) = W(r, q)
-      if constexpr (CPLX) {
-        dmma(g0, g1, x.x, y.x);
-        dmma(g0, g1, x.y, y.y);
-        dmma(h0, h1, x.x, y.y);
-        dmma(h0, h1, -x.y, y.x);
-      } else {
-        dmma(g0, g1, x, y);
-      }
+    if (part < kSplit) {
+      const int rs = (((R + kSplit - 1) / kSplit) + 3) & ~3;
+      const int k0s = part * rs, k1s = min(R, k0s + rs);
+      const T* xa = Ws + (pt * 8 + fr) * ldw + fk;   // A(p, r) = conj(W(r, p))
+      const T* yb = Ws + (qt * 8 + fr) * ldw + fk;   // B(r, q) = W(r, q)
+#pragma unroll 4
+      for (int k0 = k0s; k0 < k1s; k0 += 4) gram_mma(g[0], xa[k0], yb[k0]);
     }
     if constexpr (kSplit > 1) {
-      if (part > 0) {
-        double* o = Gp + (warp * 32 + lane) * 4;
-        o[0] = g0; o[1] = g1; o[2] = h0; o[3] = h1;
-      }
+      if (part > 0 && part < kSplit)
+#pragma unroll
+        for (int e = 0; e < kE; ++e) Gp[(warp * kE + e) * 32 + lane] = g[0][e];
       __syncthreads();
       if (part == 0)
-        for (int pp = 1; pp < kSplit; ++pp) {
-          const double* o = Gp + ((tile + pp * kTiles) * 32 + lane) * 4;
-          g0 += o[0]; g1 += o[1]; h0 += o[2]; h1 += o[3];
-        }
+        for (int pp = 1; pp < kSplit; ++pp)
+#pragma unroll
+          for (int e = 0; e < kE; ++e) g[0][e] += Gp[((warp + pp * kTU) * kE + e) * 32 + lane];
     }
   } else {
-    const int pt = warp / kTD, qt = warp % kTD;
+    // Row chunks of W in two shared buffers: half of the warps read the next chunk while
+    // the first 2 kUnits multiply one, even and odd k steps apart (units so that each
+    // quarter of the SM gets as many mma)
+    const bool loads = warp >= kSvdWarps / 2;
+    const int odd = warp / kUnits;
+    if (odd == 1) unit = (warp + 2) % kUnits;
     const int nch = (R + kChunk - 1) / kChunk;
-    issue(W, R, 0, min(kChunk, R), Cb0);
-    if (nch > 1) issue(W, R, kChunk, min(kChunk, R - kChunk), Cb1);
-    else cp_async_commit();
-    double e0 = 0.0, e1 = 0.0, f0 = 0.0, f1 = 0.0;   // a second chain over the odd k steps
-    for (int ch = 0; ch < nch; ++ch) {
-      cp_async_wait1();
-      __syncthreads();
-      const T* Cc = (ch & 1) ? Cb1 : Cb0;
-      if (gram_warp) {
-#pragma unroll 4
-        for (int k0 = 0; k0 < kChunk; k0 += 8) {
-          const T x = Cc[(k0 + fk) * kLdG + pt * 8 + fr];       // A(p, r) = conj(W(r, p))
-          const T y = Cc[(k0 + fk) * kLdG + qt * 8 + fr];       // B(r, q) = W(r, q)
-          const T x2 = Cc[(k0 + 4 + fk) * kLdG + pt * 8 + fr];
-          const T y2 = Cc[(k0 + 4 + fk) * kLdG + qt * 8 + fr];
-          if constexpr (CPLX) {
-            dmma(g0, g1, x.x, y.x);
-            dmma(g0, g1, x.y, y.y);
-            dmma(h0, h1, x.x, y.y);
-            dmma(h0, h1, -x.y, y.x);
-            dmma(e0, e1, x2.x, y2.x);
-            dmma(e0, e1, x2.y, y2.y);
-            dmma(f0, f1, x2.x, y2.y);
-            dmma(f0, f1, -x2.y, y2.x);
-          } else {
-            dmma(g0, g1, x, y);
-            dmma(e0, e1, x2, y2);
-          }
+    for (int ch = -1; ch < nch; ++ch) {
+      if (loads && ch + 1 < nch) {
+        constexpr int kCols = kNc / (kSvdWarps / 2), kAt = CPLX ? 1 : kCols;
+        T* Cn = Ck + ((ch + 1) & 1) * kNc * Gm::LdC + lane;
+        for (int i0 = 0; i0 < kCols; i0 += kAt) {
+          T v[kAt][kChunk / 32];
+#pragma unroll
+          for (int i = 0; i < kAt; ++i) load(W, R, warp - kSvdWarps / 2 + (i0 + i) * (kSvdWarps / 2), (ch + 1) * kChunk + lane, v[i]);
+#pragma unroll
+          for (int i = 0; i < kAt; ++i)
+#pragma unroll
+            for (int u = 0; u < kChunk / 32; ++u)
+              Cn[(warp - kSvdWarps / 2 + (i0 + i) * (kSvdWarps / 2)) * Gm::LdC + u * 32] = v[i][u];
         }
+      } else if (odd < 2 && ch >= 0) {
+        const int kend = min(kChunk, (R - ch * kChunk + 7) & ~7);   // zero rows beyond add nothing
+        gram_any<kTD, 8>(unit, Ck + (ch & 1) * kNc * Gm::LdC + fr * Gm::LdC + fk, Gm::LdC, odd * 4, kend, g);
       }
       __syncthreads();
-      if (ch + 2 < nch) issue(W, R, (ch + 2) * kChunk, min(kChunk, R - (ch + 2) * kChunk), (ch & 1) ? Cb1 : Cb0);
-      else cp_async_commit();
     }
-    g0 += e0; g1 += e1; h0 += f0; h1 += f1;
+    double* sums = reinterpret_cast<double*>(Ck);   // of the odd steps
+    if (odd == 1)
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int e = 0; e < kE; ++e) sums[((unit * 3 + t) * kE + e) * 32 + lane] = g[t][e];
+    __syncthreads();
+    if (gram_warp)
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int e = 0; e < kE; ++e) g[t][e] += sums[((unit * 3 + t) * kE + e) * 32 + lane];
   }
   // stored from the tiles on and above the diagonal, mirrored, so that G is exactly Hermitian
-  const int pt = warp / kTD, qt = warp % kTD;
-  for (int i = 0; i < 2 && gram_warp; ++i) {
-    const int p = pt * 8 + fr, q = qt * 8 + 2 * fk + i;
-    if (p > q) continue;
-    T v;
-    if constexpr (CPLX) v = make_double2(i ? g1 : g0, i ? h1 : h0);
-    else v = i ? g1 : g0;
-    G[p * kLdG + q] = v;
-    G[q * kLdG + p] = cconj(v);
+  auto store = [&](int pt, int qt, const double* d) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int p = pt * 8 + fr, q = qt * 8 + 2 * fk + i;
+      if (p > q) continue;
+      T v;
+      if constexpr (CPLX) v = make_double2(d[i], d[2 + i]);
+      else v = d[i];
+      if (p == q) {
+        dg[p] = cre(v);
+      } else {
+        G[p * kLdG + q] = v;
+        G[q * kLdG + p] = cconj(v);
+      }
+    }
+  };
+  if (gram_warp) {
+    if constexpr (RES) store(pt, qt, g[0]);
+    else gram_tiles<kTD>(unit, store, g);
   }
   for (int e = tid; e < kNc * kNc; e += kSvdThreads) {
     const int r = e / kNc, c = e % kNc;
@@ -320,267 +441,289 @@ __device__ void jacobi_pair_visit(const SvdJob& J, const SvdPair& P, void* work,
   }
   __syncthreads();
 
+  // the rounds over N columns, made when N changes (the last block of a sector is narrower)
+  const int N = nc + (nc & 1), np = N / 2;
+  if (N != looks_n)
+    for (int e = tid; e < (N - 1) * np; e += kSvdThreads) {
+      const int rnd = e / np, k = e % np;
+      // columns rnd + k and rnd - k were in pairs k + 1 and k - 1 of the round before
+      const int pu = min(k + 1, np - 1), pv = max(k - 1, 0);
+      int p, q, p0, p1, q0, q1;
+      circle_pair(N, rnd, k, p, q);
+      const bool uv = p == (rnd + k >= N - 1 ? rnd + k - (N - 1) : rnd + k);
+      const int i = uv ? pu : pv, j = uv ? pv : pu;
+      circle_pair(N, max(rnd - 1, 0), i, p0, p1);
+      circle_pair(N, max(rnd - 1, 0), j, q0, q1);
+      SvdLook L;
+      L.pq = (unsigned short)(p + 256 * q);
+      L.ij = (unsigned short)(j + 256 * i + (p == p1 ? 32768 : 0) + (q == q1 ? 128 : 0));
+      L.o00 = (unsigned short)(p0 * kLdG + q0);
+      L.o01 = (unsigned short)(p0 * kLdG + q1);
+      L.o10 = (unsigned short)(p1 * kLdG + q0);
+      L.o11 = (unsigned short)(p1 * kLdG + q1);
+      looks[rnd][k] = L;
+    }
   // a pair that needs no rotation on the fresh G keeps the inner sweep from
   // rotating at all: skip the visit when no pair of it does
   {
     int need = 0;
-    for (int e = tid; e < nc * nc; e += kSvdThreads) {
-      const int p = e / nc, q = e % nc;
-      if (p >= q) continue;
-      const double ab = cre(G[p * kLdG + p]) * cre(G[q * kLdG + q]);
+    for (int e = tid; e < kNc * kNc; e += kSvdThreads) {
+      const int p = e / kNc, q = e % kNc;
+      if (p >= q || q >= nc) continue;
+      const double ab = dg[p] * dg[q];
       const T gpq = G[p * kLdG + q];
       double g2;
       if constexpr (CPLX) g2 = gpq.x * gpq.x + gpq.y * gpq.y; else g2 = gpq * gpq;
       if (ab > 0.0 && g2 > tol * tol * ab) need = 1;
     }
-    if (!__syncthreads_or(need)) return;
+    const int any = __syncthreads_or(need);
+    if (tid == 0) looks_n = N;
+    if (!any) return;
   }
 
-  // 2. inner sweeps on G
-  const int N = nc + (nc & 1);
-  int nrot = 0;
-  for (int isw = 0; isw < kInnerMax && N > 1; ++isw) {
-    int sr = 0;   // rotations of this inner sweep (the same count in every thread)
+  // 2. the inner sweep on G
+  constexpr int GT = Gm::GT;
+  auto sync = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(Gm::IT) : "memory"); };
+  auto rot_of = [&](int buf, int pair) {
+    SvdRot t;
+    t.c = par_c[buf][pair];
+    t.sr = par_sr[buf][pair];
+    t.si = CPLX ? par_si[buf][pair] : 0.0;
+    t.on = par_pq[buf][pair] >> 16;
+    return t;
+  };
+  if (warp == 0) {
+    // lane k decides pair k of a round.  ahead: the others are still applying the
+    // rotations par[buf] of the round before to Gc, else Gc is as it should be.
+    T* Gc = G;
+    T* Gn = G2;
+    int nrot = 0, buf = 0;
+    bool ahead = false;
+    const int k = min(lane, np - 1);
+    SvdLook L = looks[0][k];
+    int pp = 0, pq = 0;             // the last rotation's columns and their new diagonal,
+    double pa = 0.0, pb = 0.0;      // stored while the next G_pq is on its way
+    bool pend = false;
     for (int rnd = 0; rnd < N - 1; ++rnd) {
-      bool act = false;
-      int p = 0, q = 0;
-      double c = 1.0, s = 0.0, er = 1.0, ei = 0.0, tg = 0.0, a = 0.0, b = 0.0;
-      if (warp < N / 2) {
-        if (warp == 0) { p = N - 1; q = rnd; }
-        else {
-          p = rnd + warp;
-          if (p >= N - 1) p -= N - 1;
-          q = rnd - warp;
-          if (q < 0) q += N - 1;
-        }
-        if (p > q) { const int t = p; p = q; q = t; }
-        if (q < nc) {
-          a = cre(G[p * kLdG + p]);
-          b = cre(G[q * kLdG + q]);
-          const T gpq = G[p * kLdG + q];
-          double gr, gi = 0.0;
-          if constexpr (CPLX) { gr = gpq.x; gi = gpq.y; } else { gr = gpq; }
-          const double g2 = gr * gr + gi * gi;
-          // rotate when |g| > tol sqrt(ab), compared squared; the parameters keep the
-          // dependent chain of square roots and divisions short (it sets the round time)
-          if (a * b > 0.0 && g2 > tol * tol * (a * b)) {
-            double g;
-            if constexpr (CPLX) {
-              g = sqrt(g2);
-              const double ig = 1.0 / g;
-              er = gr * ig;
-              ei = gi * ig;
-            } else {
-              g = fabs(gr);
-              er = gr >= 0.0 ? 1.0 : -1.0;
-            }
-            jacobi_rotation(a, b, g, c, s, tg);
-            act = true;
-          }
-        }
+      T b00, b01, b10, b11;
+      SvdRot ri, rj;
+      const int p = L.pq & 255, q = L.pq >> 8 & 255;
+      const bool p_second = L.ij & 32768, q_second = L.ij & 128;
+      if (ahead) {
+        b00 = Gc[L.o00];
+        b01 = Gc[L.o01];
+        b10 = Gc[L.o10];
+        b11 = Gc[L.o11];
+        ri = rot_of(buf, L.ij >> 8 & 127);
+        rj = rot_of(buf, L.ij & 127);
+      } else {
+        b00 = Gc[p * kLdG + q];
+      }
+      L = looks[min(rnd + 1, N - 2)][k];
+      if (pend) {
+        dg[pp] = pa;
+        dg[pq] = pb;
       }
       __syncwarp();
-      // columns p, q of G and Q: [x y] <- [x y] [[c, s e^{i phi}], [-s e^{-i phi}, c]]
-      if (act && lane < nc) {
-        T* gpr = G + lane * kLdG;
-        T* qr = Q + lane * kLdG;
-        if constexpr (CPLX) {
-          const double2 ep = make_double2(s * er, s * ei), em = make_double2(-s * er, s * ei);   // s e^{i phi}, -s e^{-i phi}
-          double2 x = gpr[p], y = gpr[q];
-          gpr[p] = cadd(make_double2(c * x.x, c * x.y), cmul(y, em));
-          gpr[q] = cadd(cmul(x, ep), make_double2(c * y.x, c * y.y));
-          x = qr[p]; y = qr[q];
-          qr[p] = cadd(make_double2(c * x.x, c * x.y), cmul(y, em));
-          qr[q] = cadd(cmul(x, ep), make_double2(c * y.x, c * y.y));
-        } else {
-          const double sg = s * er;
-          double x = gpr[p], y = gpr[q];
-          gpr[p] = c * x - sg * y;
-          gpr[q] = sg * x + c * y;
-          x = qr[p]; y = qr[q];
-          qr[p] = c * x - sg * y;
-          qr[q] = sg * x + c * y;
-        }
+      const double a = dg[p], b = dg[q];
+      T gpq = b00;
+      if (ahead)
+        gpq = rot_one(rot_one(b00, b01, rj, q_second, 0), rot_one(b10, b11, rj, q_second, 0), ri, p_second, 1);
+      const double gr = cre(gpq), gi = cim(gpq);
+      const double g2 = gr * gr + gi * gi;
+      // rotate when |g| > tol sqrt(ab), compared squared
+      const bool act = lane < np && q < nc && a * b > 0.0 && g2 > tol * tol * (a * b);
+      // the rotation before the test's outcome is known (unused where !act)
+      double c, sr, si = 0.0, tg;
+      if constexpr (CPLX) {
+        const double gn = sqrt(g2);
+        const double ig = 1.0 / gn;
+        double sn;
+        jacobi_rotation(a, b, gn, 1.0, c, sn, tg);
+        sr = sn * (gr * ig);
+        si = sn * (gi * ig);
+      } else {
+        jacobi_rotation(a, b, fabs(gr), gr >= 0.0 ? 1.0 : -1.0, c, sr, tg);
       }
-      __syncthreads();
-      // rows p, q of G: G <- J^H G; the rotated 2 x 2 block is set to its exact values
-      if (act && lane < nc) {
-        T* rp = G + p * kLdG;
-        T* rq = G + q * kLdG;
-        if constexpr (CPLX) {
-          const double2 x = rp[lane], y = rq[lane];
-          const double2 mp = make_double2(-s * er, -s * ei), pm = make_double2(s * er, -s * ei);   // -s e^{i phi}, s e^{-i phi}
-          rp[lane] = cadd(make_double2(c * x.x, c * x.y), cmul(mp, y));
-          rq[lane] = cadd(cmul(pm, x), make_double2(c * y.x, c * y.y));
-        } else {
-          const double sg = s * er;
-          const double x = rp[lane], y = rq[lane];
-          rp[lane] = c * x - sg * y;
-          rq[lane] = sg * x + c * y;
+      const unsigned on = __ballot_sync(0xffffffffu, act);
+      pend = act;
+      if (on == 0) {
+        if (ahead) {              // let the others finish the round before
+          buf ^= 1;
+          if (lane == 0) msg[buf] = 0;
+          sync();
+          swap_ptr(Gc, Gn);
+          ahead = false;
         }
-        if (lane == p) { rp[p] = czero<T>(); reinterpret_cast<double*>(rp + p)[0] = a - tg; }
-        if (lane == q) { rq[q] = czero<T>(); reinterpret_cast<double*>(rq + q)[0] = b + tg; }
-        if (lane == q) rp[q] = czero<T>();
-        if (lane == p) rq[p] = czero<T>();
+        continue;
       }
-      sr += __syncthreads_count(act && lane == 0);
+      if (ahead) swap_ptr(Gc, Gn);
+      buf ^= 1;
+      ahead = true;
+      if (lane < np) {
+        par_c[buf][lane] = c;
+        par_sr[buf][lane] = sr;
+        if constexpr (CPLX) par_si[buf][lane] = si;
+        par_pq[buf][lane] = p + 256 * q + (act ? 65536 : 0);
+      }
+      if (lane == 0) msg[buf] = rnd == N - 2 ? 2 : 1;
+      sync();
+      pp = p;                     // the rotated 2 x 2 block is set to its exact values
+      pq = q;
+      pa = __dsub_rn(a, tg);
+      pb = __dadd_rn(b, tg);
+      nrot += __popc(on);
     }
-    nrot += sr;
-    if (sr == 0) break;
+    if (lane == 0) {
+      msg[buf ^ 1] = -1;
+      nrot_sh = nrot;
+    }
+    sync();
+  } else if (tid < 32 + GT) {
+    const int e = tid - 32, bi = e / np, bj = e % np;   // rows of pair bi, columns of pair bj
+    T* Gc = G;
+    T* Gn = G2;
+    for (int buf = 1;; buf ^= 1) {
+      sync();
+      const int m = msg[buf];
+      if (m < 0) break;
+      if (m != 1 || bi >= np) continue;   // (nobody reads G after the last round)
+      const int pi = par_pq[buf][bi], pj = par_pq[buf][bj];
+      const SvdRot ri = rot_of(buf, bi), rj = rot_of(buf, bj);
+      const int r0 = (pi & 255) * kLdG, r1 = (pi >> 8 & 255) * kLdG, q0 = pj & 255, q1 = pj >> 8 & 255;
+      if (bi != bj) {
+        T b00 = Gc[r0 + q0], b01 = Gc[r0 + q1], b10 = Gc[r1 + q0], b11 = Gc[r1 + q1];
+        if (rj.on) {   // columns: [x y] <- [x y] [[c, s e^{i phi}], [-s e^{-i phi}, c]]
+          rot_cols(b00, b01, rj);
+          rot_cols(b10, b11, rj);
+        }
+        if (ri.on) {   // rows: G <- J^H G
+          rot_rows(b00, b10, ri);
+          rot_rows(b01, b11, ri);
+        }
+        Gn[r0 + q0] = b00;
+        Gn[r0 + q1] = b01;
+        Gn[r1 + q0] = b10;
+        Gn[r1 + q1] = b11;
+      } else {
+        Gn[r0 + q1] = ri.on ? czero<T>() : Gc[r0 + q1];
+        Gn[r1 + q0] = ri.on ? czero<T>() : Gc[r1 + q0];
+      }
+      swap_ptr(Gc, Gn);
+    }
+  } else if (tid < Gm::IT) {
+    constexpr int kG = Gm::QT / kNc, kU = B / kG;   // pairs at a time, and in turn
+    const int t = tid - 32 - GT;
+    T* const Qr = Q + t % kNc;                      // row t % kNc of Q
+    for (int buf = 1;; buf ^= 1) {
+      sync();
+      const int m = msg[buf];
+      if (m < 0) break;
+      if (m == 0) continue;
+      T x[kU], y[kU];
+      int pq[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int k = t / kNc + u * kG;
+        pq[u] = k < np ? par_pq[buf][k] : 0;
+        x[u] = Qr[(pq[u] & 255) * kLdG];
+        y[u] = Qr[(pq[u] >> 8 & 255) * kLdG];
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int k = t / kNc + u * kG;
+        if (k >= np) continue;
+        if (!(pq[u] >> 16)) continue;
+        rot_cols(x[u], y[u], rot_of(buf, k));
+        Qr[(pq[u] & 255) * kLdG] = x[u];
+        Qr[(pq[u] >> 8 & 255) * kLdG] = y[u];
+      }
+    }
   }
+  if (RES && tid >= Gm::IT) load_all(V, C, Vs, ldv, warp - Gm::IT / 32, kSvdWarps - Gm::IT / 32);
+  __syncthreads();
+  const int nrot = nrot_sh;
   if (nrot == 0) return;        // nothing moved: W and V stay as they are
 
-  if (res) {
-    // 3. Ws <- Ws Q and Vs <- Vs Q in place: warp w owns the 8-row tiles w, w + 16, ...
-    //    of the rows of Ws then Vs and computes all their output columns before it
-    //    writes them back; then every thread stores the new columns
-    const int ntw = (R + 7) / 8, ntv = (C + 7) / 8;
-    for (int t = warp; t < ntw + ntv; t += kSvdWarps) {
-      T* M = t < ntw ? Ws : Vs;
-      const int rows = t < ntw ? R : C, r = (t < ntw ? t : t - ntw) * 8 + fr;
-      double acc[kTD][4];
+  // 3. Wp <- Wp Q and Vp <- Vp Q: each warp takes RT 8-row tiles of W, then of V, at a
+  //    time, reads them whole (from shared memory: the next on their way) and writes their
+  //    new columns
+  const int ntw = (R + 7) / 8, nt = ntw + (C + 7) / 8;
+  constexpr int RT = CPLX || RES ? 1 : 2;
+  T x[RT][kNc / 4], xn[RES ? kNc / 4 : 1];
+  auto next = [&](int t) {
+    const bool isw = t < ntw;
+    const int r = (isw ? t : t - ntw) * 8 + fr, lds = isw ? ldw : ldv;
+    const bool in = t < nt && r < (isw ? R : C);
+    const T* sm = (isw ? Ws : Vs) + r + fk * lds;
 #pragma unroll
-      for (int jt = 0; jt < kTD; ++jt) acc[jt][0] = acc[jt][1] = acc[jt][2] = acc[jt][3] = 0.0;
-#pragma unroll
-      for (int k0 = 0; k0 < kNc; k0 += 4) {
-        const T x = r < rows ? M[r * kLdG + k0 + fk] : czero<T>();
-#pragma unroll
-        for (int jt = 0; jt < kTD; ++jt) {
-          const T y = Q[(k0 + fk) * kLdG + jt * 8 + fr];
-          if constexpr (CPLX) {
-            dmma(acc[jt][0], acc[jt][1], x.x, y.x);
-            dmma(acc[jt][0], acc[jt][1], -x.y, y.y);
-            dmma(acc[jt][2], acc[jt][3], x.x, y.y);
-            dmma(acc[jt][2], acc[jt][3], x.y, y.x);
-          } else {
-            dmma(acc[jt][0], acc[jt][1], x, y);
-          }
-        }
-      }
-      __syncwarp();
-      if (r < rows) {
-#pragma unroll
-        for (int jt = 0; jt < kTD; ++jt)
-          for (int i = 0; i < 2; ++i) {
-            T v;
-            if constexpr (CPLX) v = make_double2(acc[jt][i], acc[jt][2 + i]);
-            else v = acc[jt][i];
-            M[r * kLdG + jt * 8 + 2 * fk + i] = v;
-          }
-      }
-    }
-    __syncthreads();
-    for (int r0 = 0; r0 < R + C; r0 += kSvdThreads) {
-      const int rr = r0 + tid;
-      if (rr < R + C) {
-        const bool isw = rr < R;
-        const int r = isw ? rr : rr - R, ld = isw ? R : C;
-        T* M = isw ? W : V;
-        const T* S = (isw ? Ws : Vs) + r * kLdG;
-#pragma unroll
-        for (int c = 0; c < kNc; ++c)
-          if (c < nc) M[r + (long long)cols[c] * ld] = S[c];
-      }
-    }
-    __syncthreads();   // the next visit of this CTA reloads the shared arrays
-    if (tid == 0) atomicAdd(rotations, nrot);
-    return;
-  }
-
-  // 3. W_pair <- W_pair Q and V_pair <- V_pair Q, in row chunks (W's, then V's): each
-  //    chunk (128 x 2B, zero-filled) times Q on the FP64 tensor cores (warp w: output
-  //    tiles w, w + 16, ... of the chunk's 8 x 8 tile grid), the products stored
-  //    from registers; the chunk after next is copied in while one is multiplied
-  const int nw_chunks = (R + kChunk - 1) / kChunk, nv_chunks = (C + kChunk - 1) / kChunk;
-  const int nall = nw_chunks + nv_chunks;
-  auto chunk_of = [&](int k, T*& M, int& ld, int& r0, int& rows) {
-    if (k < nw_chunks) { M = W; ld = R; r0 = k * kChunk; }
-    else { M = V; ld = C; r0 = (k - nw_chunks) * kChunk; }
-    rows = min(kChunk, ld - r0);
+    for (int k = 0; k < kNc / 4; ++k) xn[k] = in ? sm[k * 4 * lds] : czero<T>();
   };
-  for (int k = 0; k < 2; ++k) {
-    if (k < nall) {
-      T* M; int ld, r0, rows;
-      chunk_of(k, M, ld, r0, rows);
-      issue(M, ld, r0, rows, k ? Cb1 : Cb0);
-    } else {
-      cp_async_commit();
+  if constexpr (RES) next(warp);
+  for (int t0 = warp * RT; t0 < nt; t0 += kSvdWarps * RT) {
+    T* base[RT];
+    int ld[RT];
+    bool in[RT];
+#pragma unroll
+    for (int u = 0; u < RT; ++u) {
+      const int t = t0 + u;
+      const bool isw = t < ntw;
+      const int r = (isw ? t : t - ntw) * 8 + fr;
+      ld[u] = isw ? R : C;
+      base[u] = (isw ? W : V) + r;
+      in[u] = t < nt && r < ld[u];
+      if constexpr (RES) {
+#pragma unroll
+        for (int k = 0; k < kNc / 4; ++k) x[u][k] = xn[k];
+        next(t + kSvdWarps);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kNc / 4; ++k)
+          x[u][k] = in[u] && k * 4 + fk < nc ? __ldcg(base[u] + (long long)cols[k * 4 + fk] * ld[u]) : czero<T>();
+      }
     }
-  }
-  for (int k = 0; k < nall; ++k) {
-    T* M; int ld, r0, rows;
-    chunk_of(k, M, ld, r0, rows);
-    cp_async_wait1();
-    __syncthreads();
-    const T* Cc = (k & 1) ? Cb1 : Cb0;
-    constexpr int kTiles = (kChunk / 8) * (kNc / 8) / kSvdWarps;   // output tiles per warp
+    double acc[RT][kTD][kE] = {};
 #pragma unroll
-    for (int u = 0; u < kTiles; ++u) {
-      const int t = warp + kSvdWarps * u, rt = t / kTD, jt = t % kTD;
-      double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
+    for (int k = 0; k < kNc / 4; ++k)
 #pragma unroll
-      for (int k0 = 0; k0 < kNc; k0 += 4) {
-        const T x = Cc[(rt * 8 + fr) * kLdG + k0 + fk];
-        const T y = Q[(k0 + fk) * kLdG + jt * 8 + fr];
-        if constexpr (CPLX) {
-          dmma(a0, a1, x.x, y.x);
-          dmma(a0, a1, -x.y, y.y);
-          dmma(b0, b1, x.x, y.y);
-          dmma(b0, b1, x.y, y.x);
-        } else {
-          dmma(a0, a1, x, y);
+      for (int j = 0; j < kTD; ++j) {
+        const T y = Q[(j * 8 + fr) * kLdG + k * 4 + fk];
+#pragma unroll
+        for (int u = 0; u < RT; ++u) {
+          if constexpr (CPLX) {
+            dmma(acc[u][j][0], acc[u][j][1], x[u][k].x, y.x);
+            dmma(acc[u][j][0], acc[u][j][1], -x[u][k].y, y.y);
+            dmma(acc[u][j][2], acc[u][j][3], x[u][k].x, y.y);
+            dmma(acc[u][j][2], acc[u][j][3], x[u][k].y, y.x);
+          } else {
+            dmma(acc[u][j][0], acc[u][j][1], x[u][k], y);
+          }
         }
       }
-      const int r = rt * 8 + fr;
-      if (r < rows) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int j = jt * 8 + 2 * fk + i;
-          if (j >= nc) continue;
+    for (int u = 0; u < RT; ++u) {
+      if (!in[u]) continue;
+#pragma unroll
+      for (int j = 0; j < kTD; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int c = j * 8 + 2 * fk + e;
           T v;
-          if constexpr (CPLX) v = make_double2(i ? a1 : a0, i ? b1 : b0);
-          else v = i ? a1 : a0;
-          M[(r0 + r) + (long long)cols[j] * ld] = v;
+          if constexpr (CPLX) v = make_double2(acc[u][j][e], acc[u][j][2 + e]);
+          else v = acc[u][j][e];
+          if (c < nc) base[u][(long long)cols[c] * ld[u]] = v;
         }
-      }
-    }
-    __syncthreads();   // every warp is done with this buffer
-    if (k + 2 < nall) {
-      T* M2; int ld2, r2, rows2;
-      chunk_of(k + 2, M2, ld2, r2, rows2);
-      issue(M2, ld2, r2, rows2, (k & 1) ? Cb1 : Cb0);
-    } else {
-      cp_async_commit();
     }
   }
   if (tid == 0) atomicAdd(rotations, nrot);
 }
 
-template <bool CPLX, int B>
-__global__ void __launch_bounds__(kSvdThreads) jacobi_pair_kernel(const SvdJob* __restrict__ jobs,
-                                                                  const SvdPair* __restrict__ pairs, void* work,
-                                                                  void* vmat, const int* perm, double tol,
-                                                                  int* rotations, int res) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const SvdPair P = pairs[blockIdx.x];
-  const SvdJob J = jobs[P.job];
-  jacobi_pair_visit<CPLX, B>(J, P, work, vmat, perm, tol, smem_raw, rotations, res != 0);
-}
-
-// ---------------------------------------------------------------------------
-// All sweeps in one cooperative launch.  Rounds are separated by a grid barrier
-// (bounded); rotations are counted per sector in three rotating counter sets
-// (sweep s adds into set s % 3, the set of sweep s + 1 is cleared during sweep
-// s, when nobody reads it any more), and a sector whose sweep made no rotation
-// is skipped from then on.  Every block takes the same decisions from the same
-// counts, read after the barrier that ends the sweep.
-constexpr int kSvdMaxJobsCoop = 256;
 constexpr unsigned long long kSvdBarrierNs = 2000000000ull;
 
 struct SvdCtl {
   unsigned count, gen;
-  int status;                 // 0, or 1 when a grid barrier ran out of time
-  int sweeps;                 // sweeps taken, -1 when max_sweeps was reached
+  int status;                 // 0, or 1 when a barrier ran out of time
+  int sweeps, failed;         // sweeps taken; 1 when max_sweeps was reached
   unsigned long long t0, t1;  // device clock (ns) at the start and end of block 0
 };
 
@@ -619,87 +762,138 @@ __device__ bool svd_grid_sync(SvdCtl* ctl) {
   return ok_sh != 0;
 }
 
-template <bool CPLX, int B>
-__global__ void __launch_bounds__(kSvdThreads) jacobi_coop_kernel(const SvdJob* __restrict__ jobs, int nj,
-                                                                  const SvdPair* __restrict__ pairs,
-                                                                  const int* __restrict__ roff, int max_rounds,
-                                                                  void* work, void* vmat, double* nrm, int* perm,
-                                                                  double tol, int* cnt, SvdCtl* ctl, int max_sweeps,
-                                                                  int res) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned char done[kSvdMaxJobsCoop];
-  __shared__ int all_done;
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->t0 = svd_gtime();
-  for (int j = threadIdx.x; j < nj; j += blockDim.x) done[j] = 0;
+// Barrier of the CTAs that share a sector: *count grows by one per CTA and phase.
+// Returns false when it ran out of time.
+__device__ bool svd_group_sync(unsigned* count, int size, unsigned& phase, SvdCtl* ctl) {
+  __shared__ int ok_sh;
   __syncthreads();
-  int sweeps = -1;
-  for (int sw = 0; sw < max_sweeps; ++sw) {
-    int* cur = cnt + (sw % 3) * nj;
-    if (blockIdx.x == 0)
-      for (int j = threadIdx.x; j < nj; j += blockDim.x) cnt[((sw + 1) % 3) * nj + j] = 0;
-    // column order of this sweep: decreasing norm (de Rijk), ties by index.  Norms
-    // one warp per column, then every column's rank counted over its sector.
-    {
-      using T = typename SvdT<CPLX>::T;
-      const int lane = threadIdx.x & 31;
-      const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-      for (int j = 0; j < nj; ++j) {
-        if (done[j]) continue;
-        const SvdJob J = jobs[j];
-        const int R = J.trans ? J.n : J.m, C = J.trans ? J.m : J.n;
-        const T* W = static_cast<const T*>(work) + J.woff;
-        for (int c = gw; c < C; c += nw) {
-          double a = 0.0;
-          for (int r = lane; r < R; r += 32) {
-            const T x = W[r + (long long)c * R];
-            if constexpr (CPLX) a += x.x * x.x + x.y * x.y;
-            else a += x * x;
-          }
-          a = wsum(a);
-          if (lane == 0) nrm[J.soff + c] = a;
-        }
+  if (size == 1) return true;
+  ++phase;
+  if (threadIdx.x == 0) {
+    ok_sh = 1;
+    __threadfence();
+    atomicAdd(count, 1u);
+    const unsigned want = phase * (unsigned)size;
+    const volatile unsigned* seen = count;
+    const unsigned long long t0 = svd_gtime();
+    for (long long it = 0; (int)(*seen - want) < 0; ++it) {
+      if (it > (1ll << 30) || ((it & 255) == 255 && svd_gtime() - t0 > kSvdBarrierNs)) {
+        ok_sh = 0;
+        atomicExch(&ctl->status, 1);
+        break;
       }
-      if (!svd_grid_sync(ctl)) return;
-      const int gt = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-      for (int j = 0; j < nj; ++j) {
-        if (done[j]) continue;
-        const SvdJob J = jobs[j];
-        const int C = J.trans ? J.m : J.n;
-        const double* nj_ = nrm + J.soff;
-        for (int c = gt; c < C; c += nt) {
-          const double v = nj_[c];
-          int rank = 0;
-          for (int k = 0; k < C; ++k) {
-            const double u = nj_[k];
-            rank += (u > v || (u == v && k < c)) ? 1 : 0;
-          }
-          perm[J.soff + rank] = c;
-        }
-      }
-      if (!svd_grid_sync(ctl)) return;
+      if (it > 16) __nanosleep(32);
     }
-    for (int r = 0; r < max_rounds; ++r) {
-      for (int p = roff[r] + blockIdx.x; p < roff[r + 1]; p += gridDim.x) {
-        const SvdPair P = pairs[p];
-        if (done[P.job]) continue;
-        const SvdJob J = jobs[P.job];
-        jacobi_pair_visit<CPLX, B>(J, P, work, vmat, perm, tol, smem_raw, cur + P.job, res != 0);
-      }
-      if (!svd_grid_sync(ctl)) return;
-    }
-    if (threadIdx.x == 0) all_done = 1;
-    __syncthreads();
-    for (int j = threadIdx.x; j < nj; j += blockDim.x) {
-      if (!done[j] && *((volatile int*)(cur + j)) == 0) done[j] = 1;
-      if (!done[j]) all_done = 0;
-    }
-    __syncthreads();
-    if (all_done) { sweeps = sw + 1; break; }
+    __threadfence();
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ctl->sweeps = sweeps;
-    ctl->t1 = svd_gtime();
+  __syncthreads();
+  return ok_sh != 0;
+}
+
+// All sweeps of all sectors in one cooperative launch.  Sectors are independent: each
+// has its own CTAs (SvdCta), its own barrier between rounds and its own end, so a round
+// of a narrow sector doesn't wait for the visits of the widest one (with one barrier
+// for all, waiting took 39,000 of 190,000 cycles a round at D = 2048; with its own
+// 11,500).  Rotations are counted in three rotating counter sets (sweep s adds into set s % 3; the set of sweep s + 1 is
+// cleared during sweep s, when nobody reads it any more); every CTA of a sector takes
+// the same decisions from the same counts, read after the barrier that ends the sweep.
+template <bool CPLX, int B, bool RES>
+__global__ void __launch_bounds__(kSvdThreads) jacobi_coop_kernel(const SvdJob* __restrict__ jobs, int nj,
+                                                                  const SvdCta* __restrict__ ctas,
+                                                                  const int* __restrict__ order, unsigned* bars,
+                                                                  void* work, void* vmat, double* nrm, int* perm,
+                                                                  double tol, int* cnt, SvdCtl* ctl, int max_sweeps) {
+  using T = typename SvdT<CPLX>::T;
+  constexpr int kNc = SvdGeom<CPLX, B>::Nc;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int cols[kNc];
+  __shared__ SvdLook looks[2 * B - 1][B];   // the rounds over looks_n columns
+  __shared__ int looks_n;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) {
+    looks_n = 0;
+    atomicMin(&ctl->t0, svd_gtime());
   }
+  const SvdCta me = ctas[blockIdx.x];
+  unsigned* bar = bars + me.group * 32;
+  unsigned phase = 0;
+  for (int jj = 0; jj < me.nj; ++jj) {
+    const int j = order[me.j0 + jj];
+    const SvdJob J = jobs[j];
+    const int R = J.trans ? J.n : J.m, C = J.trans ? J.m : J.n;
+    T* W = static_cast<T*>(work) + J.woff;
+    T* V = static_cast<T*>(vmat) + J.voff;
+    int* pj = perm + J.soff;
+    // rounds of the circle method over N blocks (odd nblk: the last is a dummy), npair
+    // pairs each
+    const int nblk = (C + B - 1) / B, N = nblk + (nblk & 1);
+    const int nr = nblk <= 1 ? 1 : N - 1, npair = nblk <= 1 ? 1 : nblk / 2;
+    // column of this thread (of the first kNc) in pair i of round r; nc: the pair's columns
+    int nc = 0;
+    auto column = [&](int r, int i) {
+      int b0 = 0, b1 = 0;
+      nc = min(B, C);
+      if (nblk > 1) {
+        circle_pair(N, r, i + (nblk & 1), b0, b1);
+        nc = B + min(B, C - b1 * B);
+      }
+      return tid < nc ? __ldcg(pj + (tid < B ? b0 * B + tid : b1 * B + tid - B)) : 0;
+    };
+    int sweeps = -1;
+    for (int sw = 0; sw < max_sweeps; ++sw) {
+      int* cur = cnt + (sw % 3) * nj + j;
+      if (me.rank == 0 && tid == 0) cnt[((sw + 1) % 3) * nj + j] = 0;
+      // column order of this sweep: decreasing norm (de Rijk), ties by index.  Norms
+      // one warp per column, then every column's rank counted by a warp.
+      const int gw = (me.rank * kSvdThreads + tid) >> 5, nw = me.size * kSvdWarps;
+      for (int c = gw; c < C; c += nw) {
+        double a = 0.0;
+        for (int r = lane; r < R; r += 32) {
+          const T x = __ldcg(W + r + (long long)c * R);
+          if constexpr (CPLX) a += x.x * x.x + x.y * x.y;
+          else a += x * x;
+        }
+        a = wsum(a);
+        if (lane == 0) nrm[J.soff + c] = a;
+      }
+      if (!svd_group_sync(bar, me.size, phase, ctl)) return;
+      for (int c = gw; c < C; c += nw) {
+        const double v = __ldcg(nrm + J.soff + c);
+        int rank = 0;
+        for (int k = lane; k < C; k += 32) {
+          const double u = __ldcg(nrm + J.soff + k);
+          rank += (u > v || (u == v && k < c)) ? 1 : 0;
+        }
+        rank = __reduce_add_sync(0xffffffffu, rank);
+        if (lane == 0) pj[rank] = c;
+      }
+      if (!svd_group_sync(bar, me.size, phase, ctl)) return;
+      int col = me.rank < npair ? column(0, me.rank) : 0;
+      for (int r = 0; r < nr; ++r) {
+        for (int i = me.rank; i < npair; i += me.size) {
+          if (i != me.rank) {
+            col = column(r, i);
+            __syncthreads();     // the visit before is done with cols
+          }
+          if (tid < nc) cols[tid] = col;
+          __syncthreads();
+          jacobi_pair_visit<CPLX, B, RES>(W, R, V, C, cols, nc, tol, smem_raw, looks, looks_n, cur);
+        }
+        // the next round's columns, on their way while the barrier is
+        if (r + 1 < nr && me.rank < npair) col = column(r + 1, me.rank);
+        if (!svd_group_sync(bar, me.size, phase, ctl)) return;
+      }
+      if (*reinterpret_cast<volatile int*>(cur) == 0) {
+        sweeps = sw + 1;
+        break;
+      }
+    }
+    if (me.rank == 0 && tid == 0) {
+      if (sweeps < 0) atomicExch(&ctl->failed, 1);
+      else atomicMax(&ctl->sweeps, sweeps);
+    }
+  }
+  if (tid == 0) atomicMax(&ctl->t1, svd_gtime());
 }
 
 // W = A (m >= n) or A^H (m < n); V = I (copy = 0: only the column order, when the
@@ -797,8 +991,6 @@ struct QrTile {
 
 __device__ __forceinline__ double cabs2(double a) { return a * a; }
 __device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x + a.y * a.y; }
-__device__ __forceinline__ double cim(double) { return 0.0; }
-__device__ __forceinline__ double cim(double2 a) { return a.y; }
 __device__ __forceinline__ double csub(double a, double b) { return a - b; }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 template <class T> __device__ __forceinline__ T cmake(double re, double im);
@@ -1131,126 +1323,138 @@ __global__ void qr_vout_kernel(const QrJob* jobs, const void* qbuf, void* vmat, 
   }
 }
 
-// Host driver.  Runs all sweeps in one cooperative launch when the device allows
-// it, otherwise one launch per round and one host synchronisation per sweep to
-// test convergence.  Returns the number of sweeps taken (or -1 when max_sweeps
-// was reached).
+// CTAs of the Jacobi kernel for nsect sectors with pairs[j] pairs per round, rounds[j]
+// rounds per sweep and visits of cost[j] each: of all shares of ncta CTAs the one whose
+// longest sector ends first (every sector taking as many sweeps).  A sector that ends in
+// time on one CTA may share it with others.  Fills the sectors' order and the CTAs.
+static void jacobi_shares(const std::vector<int>& pairs, const std::vector<int>& rounds, const std::vector<double>& cost,
+                          int ncta, std::vector<int>& order, std::vector<SvdCta>& ctas) {
+  const int nj = (int)pairs.size();
+  std::vector<int> by(nj);
+  for (int j = 0; j < nj; ++j) by[j] = j;
+  auto alone = [&](int j) { return rounds[j] * cost[j] * pairs[j]; };
+  std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return alone(a) > alone(b); });
+  std::vector<std::vector<int>> bins;
+  // CTAs needed to end by time t (> ncta: no)
+  auto fits = [&](double t) {
+    bins.clear();
+    std::vector<double> left;
+    long long n = 0;
+    for (const int j : by) {
+      const double turns = std::floor(t / (rounds[j] * cost[j]) * (1 + 1e-12));
+      if (turns < 1.0) return false;
+      const int size = (int)((pairs[j] + std::min(turns, 1e6) - 1) / std::floor(std::min(turns, 1e6)));
+      if (size > 1) {
+        n += size;
+        continue;
+      }
+      size_t b = 0;
+      while (b < bins.size() && left[b] < alone(j)) ++b;
+      if (b == bins.size()) {
+        bins.emplace_back();
+        left.push_back(t);
+      }
+      bins[b].push_back(j);
+      left[b] -= alone(j);
+    }
+    return n + (long long)bins.size() <= ncta;
+  };
+  double lo = 0.0, hi = 0.0;
+  for (int j = 0; j < nj; ++j) hi += alone(j);
+  for (int it = 0; it < 50; ++it) {
+    const double t = 0.5 * (lo + hi);
+    (fits(t) ? hi : lo) = t;
+  }
+  fits(hi);
+  int group = 0;
+  for (const int j : by) {
+    const double turns = std::min(std::floor(hi / (rounds[j] * cost[j]) * (1 + 1e-12)), 1e6);
+    const int size = (int)((pairs[j] + turns - 1) / turns);
+    if (size <= 1) continue;
+    for (int r = 0; r < size; ++r) ctas.push_back({group, r, size, (int)order.size(), 1});
+    order.push_back(j);
+    ++group;
+  }
+  for (const auto& b : bins) {
+    ctas.push_back({group++, 0, 1, (int)order.size(), (int)b.size()});
+    order.insert(order.end(), b.begin(), b.end());
+  }
+}
+
+// Host driver of the Jacobi: all sweeps in one cooperative launch.  Returns the number
+// of sweeps taken, or -1 when max_sweeps was reached.
 template <bool CPLX, int B>
 static int jacobi_run(const void* a, void* work, void* vmat, double* sv, const std::vector<SvdJob>& hjobs,
                       int max_sweeps, cudaStream_t s, double* kernel_ms, int copy = 1, int stream = 0) {
   const int nj = (int)hjobs.size();
-  std::vector<int> bsz(nj), nblk(nj), nrounds(nj);
-  int max_rounds = 0, maxR = 0;
-  long long maxRC = 0;
-  size_t smem = 0;
+  std::vector<int> pairs(nj), rounds(nj);
+  std::vector<double> cost(nj);
+  int maxR = 0;
+  long long nsv = 1;   // singular-value slots (the column order lives at the same offsets)
+  size_t smem = svd_smem_bytes<CPLX, B>(), res_smem = 0;
   for (int j = 0; j < nj; ++j) {
     const int R = hjobs[j].trans ? hjobs[j].n : hjobs[j].m;
     const int C = hjobs[j].trans ? hjobs[j].m : hjobs[j].n;
     maxR = std::max(maxR, R);
-    maxRC = std::max<long long>(maxRC, (long long)R + C);
-    bsz[j] = B;
-    nblk[j] = (C + bsz[j] - 1) / bsz[j];
-    const int N = nblk[j] + (nblk[j] & 1);
-    nrounds[j] = nblk[j] <= 1 ? 1 : N - 1;
-    max_rounds = std::max(max_rounds, nrounds[j]);
-    smem = svd_smem_bytes<CPLX, B>();
+    res_smem = std::max(res_smem, svd_res_smem_bytes<CPLX, B>(R, C));
+    nsv = std::max<long long>(nsv, hjobs[j].soff + C);
+    const int nblk = (C + B - 1) / B;
+    pairs[j] = std::max(nblk / 2, 1);
+    rounds[j] = std::max(nblk + (nblk & 1) - 1, 1);
+    // a visit's load, Gram and application take as long per row as 1,000 rows take for
+    // its inner sweep and barrier (b = 8: 17,000 cycles + 12 a row; b = 16: 35,000 + 40)
+    cost[j] = R + C + 1000.0;
   }
   // visits hold the pair's columns of W and V in shared memory when the largest fits
-  const int res = !stream && svd_res_smem_bytes<CPLX, B>(maxRC) <= kSvdResMax ? 1 : 0;
-  if (res) smem = std::max(smem, svd_res_smem_bytes<CPLX, B>(maxRC));
-  // pair lists per round
-  std::vector<std::vector<SvdPair>> rounds(max_rounds);
-  for (int j = 0; j < nj; ++j) {
-    if (nblk[j] <= 1) { rounds[0].push_back({j, 0, -1, bsz[j]}); continue; }
-    const int N = nblk[j] + (nblk[j] & 1);
-    for (int r = 0; r < N - 1; ++r)
-      for (int i = 0; i < N / 2; ++i) {
-        int p, q;
-        if (i == 0) { p = N - 1; q = r; }
-        else { p = (r + i) % (N - 1); q = (r - i + (N - 1)) % (N - 1); }
-        if (p >= nblk[j] || q >= nblk[j]) continue;
-        rounds[r].push_back({j, std::min(p, q), std::max(p, q), bsz[j]});
-      }
-  }
-  std::vector<int> roff(max_rounds + 1, 0);
-  std::vector<SvdPair> flat;
-  for (int r = 0; r < max_rounds; ++r) {
-    roff[r] = (int)flat.size();
-    flat.insert(flat.end(), rounds[r].begin(), rounds[r].end());
-  }
-  roff[max_rounds] = (int)flat.size();
-  long long nsv = 1;   // singular-value slots (the column order lives at the same offsets)
-  for (int j = 0; j < nj; ++j)
-    nsv = std::max<long long>(nsv, hjobs[j].soff + (hjobs[j].trans ? hjobs[j].m : hjobs[j].n));
-  DevBuf djobs(sizeof(SvdJob) * nj, s), dpairs(sizeof(SvdPair) * flat.size(), s), dcnt(sizeof(int), s),
-      dperm(sizeof(int) * nsv, s);
-  SADMRG_CUDA(cudaMemcpyAsync(djobs.get(), hjobs.data(), sizeof(SvdJob) * nj, cudaMemcpyHostToDevice, s));
-  SADMRG_CUDA(cudaMemcpyAsync(dpairs.get(), flat.data(), sizeof(SvdPair) * flat.size(), cudaMemcpyHostToDevice, s));
-  dim3 ig(nj, 16);
-  jacobi_init_kernel<CPLX><<<ig, 256, 0, s>>>(djobs.as<SvdJob>(), a, work, vmat, dperm.as<int>(), copy);
-  SADMRG_CUDA(cudaGetLastError());
-  SADMRG_CUDA(cudaFuncSetAttribute(jacobi_pair_kernel<CPLX, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const double tol = std::sqrt((double)std::max(maxR, 1)) * 2.220446049250313e-16;
-  int sweeps = -1;
-  int h_rot = 0;
-  // preferred: every sweep in one cooperative launch (no host round trip per sweep)
-  int dev = 0, coop = 0, nsm = 0, per_sm = 0;
+  const bool res = !stream && res_smem <= kSvdResMax;
+  if (res) smem = std::max(smem, res_smem);
+  const auto kernel = res ? jacobi_coop_kernel<CPLX, B, true> : jacobi_coop_kernel<CPLX, B, false>;
+  int dev = 0, nsm = 0, per_sm = 0;
   SADMRG_CUDA(cudaGetDevice(&dev));
-  SADMRG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   SADMRG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  SADMRG_CUDA(cudaFuncSetAttribute(jacobi_coop_kernel<CPLX, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  SADMRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, jacobi_coop_kernel<CPLX, B>, kSvdThreads, smem));
-  int max_pairs = 1;
-  for (int r = 0; r < max_rounds; ++r) max_pairs = std::max(max_pairs, roff[r + 1] - roff[r]);
-  if (coop && per_sm > 0 && nj <= kSvdMaxJobsCoop) {
-    const int grid = std::max(1, std::min(max_pairs, per_sm * nsm));
-    DevBuf droff(sizeof(int) * (max_rounds + 1), s), dcnt3(sizeof(int) * 3 * nj, s), dctl(sizeof(SvdCtl), s);
-    SADMRG_CUDA(cudaMemcpyAsync(droff.get(), roff.data(), sizeof(int) * (max_rounds + 1), cudaMemcpyHostToDevice, s));
-    SADMRG_CUDA(cudaMemsetAsync(dcnt3.get(), 0, sizeof(int) * 3 * nj, s));
-    SADMRG_CUDA(cudaMemsetAsync(dctl.get(), 0, sizeof(SvdCtl), s));
-    const SvdJob* pj = djobs.as<SvdJob>();
-    const SvdPair* pp = dpairs.as<SvdPair>();
-    const int* pr = droff.as<int>();
-    int* pc = dcnt3.as<int>();
-    SvdCtl* pctl = dctl.as<SvdCtl>();
-    int njv = nj, mr = max_rounds, ms = max_sweeps;
-    double tolv = tol;
-    int resv = res;
-    void* a_work = work;
-    void* a_vmat = vmat;
-    double* a_nrm = sv;   // column norms of each sweep; the final singular values overwrite them
-    int* a_perm = dperm.as<int>();
-    void* args[] = {(void*)&pj,     (void*)&njv,    (void*)&pp,   (void*)&pr, (void*)&mr,   (void*)&a_work,
-                    (void*)&a_vmat, (void*)&a_nrm, (void*)&a_perm, (void*)&tolv, (void*)&pc, (void*)&pctl,
-                    (void*)&ms, (void*)&resv};
-    SADMRG_CUDA(cudaLaunchCooperativeKernel((const void*)jacobi_coop_kernel<CPLX, B>, dim3(grid), dim3(kSvdThreads),
-                                            args, smem, s));
-    SvdCtl hctl{};
-    SADMRG_CUDA(cudaMemcpyAsync(&hctl, dctl.get(), sizeof(SvdCtl), cudaMemcpyDeviceToHost, s));
-    SADMRG_CUDA(cudaStreamSynchronize(s));
-    SADMRG_REQUIRE(hctl.status == 0, SADMRG_ERR_CUDA, "jacobi svd: a grid barrier ran out of time");
-    sweeps = hctl.sweeps;
-    if (kernel_ms) *kernel_ms = (double)(hctl.t1 - hctl.t0) * 1e-6;
-    jacobi_norms_kernel<CPLX><<<nj, 256, 0, s>>>(djobs.as<SvdJob>(), work, sv);
-    SADMRG_CUDA(cudaGetLastError());
-    return sweeps;
-  }
-  for (int sw = 0; sw < max_sweeps; ++sw) {
-    SADMRG_CUDA(cudaMemsetAsync(dcnt.get(), 0, sizeof(int), s));
-    for (int r = 0; r < max_rounds; ++r) {
-      const int np = roff[r + 1] - roff[r];
-      if (np == 0) continue;
-      jacobi_pair_kernel<CPLX, B><<<np, kSvdThreads, smem, s>>>(djobs.as<SvdJob>(), dpairs.as<SvdPair>() + roff[r],
-                                                                work, vmat, dperm.as<int>(), tol, dcnt.as<int>(), res);
-    }
-    SADMRG_CUDA(cudaGetLastError());
-    SADMRG_CUDA(cudaMemcpyAsync(&h_rot, dcnt.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
-    SADMRG_CUDA(cudaStreamSynchronize(s));
-    if (h_rot == 0) { sweeps = sw + 1; break; }
-  }
-  jacobi_norms_kernel<CPLX><<<nj, 256, 0, s>>>(djobs.as<SvdJob>(), work, sv);
+  SADMRG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SADMRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSvdThreads, smem));
+  SADMRG_REQUIRE(per_sm > 0, SADMRG_ERR_CUDA, "jacobi svd: the kernel does not fit on this device");
+  std::vector<int> order;
+  std::vector<SvdCta> ctas;
+  jacobi_shares(pairs, rounds, cost, per_sm * nsm, order, ctas);
+  // one copy: jobs, CTAs, order; one cleared area: control, counters, barriers
+  const size_t o_cta = sizeof(SvdJob) * nj, o_ord = o_cta + sizeof(SvdCta) * ctas.size();
+  std::vector<char> host(o_ord + sizeof(int) * nj);
+  std::memcpy(host.data(), hjobs.data(), o_cta);
+  std::memcpy(host.data() + o_cta, ctas.data(), o_ord - o_cta);
+  std::memcpy(host.data() + o_ord, order.data(), sizeof(int) * nj);
+  const size_t o_cnt = sizeof(SvdCtl), o_bar = (o_cnt + sizeof(int) * 3 * nj + 127) & ~(size_t)127;
+  const size_t nzero = o_bar + 128 * ctas.size();
+  DevBuf dlists(host.size(), s), dzero(nzero, s), dperm(sizeof(int) * nsv, s);
+  SADMRG_CUDA(cudaMemcpyAsync(dlists.get(), host.data(), host.size(), cudaMemcpyHostToDevice, s));
+  SADMRG_CUDA(cudaMemsetAsync(dzero.get(), 0, nzero, s));
+  char* lists = dlists.as<char>();
+  char* zero = dzero.as<char>();
+  SvdCtl* pctl = reinterpret_cast<SvdCtl*>(zero);
+  SADMRG_CUDA(cudaMemsetAsync(&pctl->t0, 0xff, sizeof(pctl->t0), s));
+  const SvdJob* pj = reinterpret_cast<const SvdJob*>(lists);
+  const SvdCta* pcta = reinterpret_cast<const SvdCta*>(lists + o_cta);
+  const int* pord = reinterpret_cast<const int*>(lists + o_ord);
+  int* pcnt = reinterpret_cast<int*>(zero + o_cnt);
+  unsigned* pbar = reinterpret_cast<unsigned*>(zero + o_bar);
+  int* pperm = dperm.as<int>();
+  jacobi_init_kernel<CPLX><<<dim3(nj, 16), 256, 0, s>>>(pj, a, work, vmat, pperm, copy);
   SADMRG_CUDA(cudaGetLastError());
-  return sweeps;
+  double tol = std::sqrt((double)std::max(maxR, 1)) * 2.220446049250313e-16;
+  int njv = nj;
+  double* nrm = sv;   // column norms of each sweep; the final singular values overwrite them
+  void* args[] = {(void*)&pj,   (void*)&njv, (void*)&pcta,  (void*)&pord, (void*)&pbar, (void*)&work,       (void*)&vmat,
+                  (void*)&nrm,  (void*)&pperm, (void*)&tol, (void*)&pcnt, (void*)&pctl, (void*)&max_sweeps};
+  SADMRG_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)ctas.size()), dim3(kSvdThreads), args, smem, s));
+  SvdCtl hctl{};
+  SADMRG_CUDA(cudaMemcpyAsync(&hctl, pctl, sizeof(SvdCtl), cudaMemcpyDeviceToHost, s));
+  jacobi_norms_kernel<CPLX><<<nj, 256, 0, s>>>(pj, work, sv);
+  SADMRG_CUDA(cudaGetLastError());
+  SADMRG_CUDA(cudaStreamSynchronize(s));
+  SADMRG_REQUIRE(hctl.status == 0, SADMRG_ERR_CUDA, "jacobi svd: a barrier ran out of time");
+  if (kernel_ms) *kernel_ms = (double)(hctl.t1 - hctl.t0) * 1e-6;
+  return hctl.failed ? -1 : hctl.sweeps;
 }
 
 // Column blocks of the Jacobi for these jobs: 8 when the widest round of
