@@ -6,7 +6,7 @@
 // one operator buffer and one scratch buffer, so every batched matvec is one
 // launch per stage for all instances (mma.sync for FP64, tcgen05 for 3xTF32).
 // The Krylov recurrence runs segment-wise (krylov.cu: every segment cut into
-// ranges, a block each), and the host keeps one tridiagonal problem per instance; the
+// ranges, a block each), and every instance has its own tridiagonal problem; the
 // recurrence and its checks are those of lanczos1 (Lanczos::lanczos1,
 // src/dmrg_inst.cpp:1286-1348), applied per instance.
 #include <algorithm>
@@ -126,6 +126,8 @@ struct BatchKrylov {
   S* h_dots = nullptr;          // 2 per segment
   double* h_cdev = nullptr;     // Ritz coefficients (ns x (mlanc + 1))
   int* h_mask = nullptr;
+  double* h_e0 = nullptr;       // lowest Ritz values
+  int* h_n = nullptr;           // rows of the tridiagonals of a check, then their status
   int* h_active = nullptr;      // instances whose matvec work still runs (written only after a stream sync)
   BatchKrylov(Ctx& cc, const HeffBatch<S>& B, int ml) : c(cc), N(B.merged.n), ns(B.nseg()), mlanc(ml), all(B.span) {
     ff.alloc(sizeof(S) * N * (mlanc + 1), c.stream);
@@ -142,12 +144,16 @@ struct BatchKrylov {
     SADMRG_CUDA(cudaMemsetAsync(beta.get(), 0, beta.bytes(), c.stream));
     SADMRG_CUDA(cudaMemsetAsync(counter.get(), 0, counter.bytes(), c.stream));
     SADMRG_CUDA(cudaMemsetAsync(norm.get(), 0, norm.bytes(), c.stream));
-    SADMRG_CUDA(cudaMallocHost(&h_a, sizeof(double) * (size_t)ns * (mlanc + 1)));
-    SADMRG_CUDA(cudaMallocHost(&h_beta, sizeof(double) * (size_t)ns * (mlanc + 2)));
-    SADMRG_CUDA(cudaMallocHost(&h_dots, sizeof(S) * (size_t)ns * 2));
-    SADMRG_CUDA(cudaMallocHost(&h_cdev, sizeof(double) * (size_t)ns * (mlanc + 1)));
-    SADMRG_CUDA(cudaMallocHost(&h_mask, sizeof(int) * ns));
-    SADMRG_CUDA(cudaMallocHost(&h_active, sizeof(int) * ns));
+    // page-locked scalars, one allocation
+    const size_t na = (size_t)ns * (mlanc + 1), nb = (size_t)ns * (mlanc + 2), nd = sizeof(S) / sizeof(double) * 2 * ns;
+    SADMRG_CUDA(cudaMallocHost(&h_a, sizeof(double) * (na + nb + nd + na + ns) + sizeof(int) * (3 * (size_t)ns + 1)));
+    h_beta = h_a + na;
+    h_dots = reinterpret_cast<S*>(h_beta + nb);
+    h_cdev = h_beta + nb + nd;
+    h_e0 = h_cdev + na;
+    h_mask = reinterpret_cast<int*>(h_e0 + ns);
+    h_active = h_mask + ns;
+    h_n = h_active + ns;
     // an instance without elements has no block to write its scalars: they read as zero
     std::memset(h_a, 0, sizeof(double) * (size_t)ns * (mlanc + 1));
     std::memset(h_beta, 0, sizeof(double) * (size_t)ns * (mlanc + 2));
@@ -158,11 +164,6 @@ struct BatchKrylov {
   ~BatchKrylov() {
     cudaStreamSynchronize(c.stream);
     cudaFreeHost(h_a);
-    cudaFreeHost(h_beta);
-    cudaFreeHost(h_dots);
-    cudaFreeHost(h_cdev);
-    cudaFreeHost(h_mask);
-    cudaFreeHost(h_active);
   }
   S* F(int i) { return ff.as<S>() + (size_t)i * N; }
   VecSpan on(const DevBuf& m) const {   // the segments whose flag in m is set
@@ -190,7 +191,6 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
   st.energy.assign(ns, 0.0);
   st.matvecs.assign(ns, 0);
   std::vector<char> done(ns, 0);
-  std::vector<std::vector<double>> aal(ns, std::vector<double>(mlanc, 0.0)), nnl(ns, std::vector<double>(mlanc + 1, 0.0));
   // Converged instances are switched off in the matvec (their jobs skip all
   // work; their segments of the output keep stale values that nothing reads).
   auto matvec = [&](const S* in, S* out) {
@@ -210,11 +210,36 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
   to_norm.op = VO_NORM;
   to_norm.scal = K.norm.get();
   to_norm.sstride = 1;
-  // Ritz vectors of the masked segments into v (coefficients in h_cdev, row stride
-  // mlanc + 1) and their norms
+  // Lowest Ritz pair of the masked segments, whose tridiagonals have K.h_n[s] <= nv rows
+  // (0 elsewhere): the Ritz vectors into v and their norms.  Tridiagonals of at least
+  // kTridiagDev instances are solved on the device (0.2 us a rotation, all at once), of
+  // fewer on the host (0.04 us, one after another): 8 of 40 rows 0.52 ms against 0.8.
+  constexpr int kTridiagDev = 8;
+  std::vector<double> eig, z;
   auto ritz = [&](int nv) {
-    SADMRG_CUDA(cudaMemcpyAsync(K.cdev.get(), K.h_cdev, sizeof(double) * (size_t)ns * (mlanc + 1),
-                                cudaMemcpyHostToDevice, c.stream));
+    int open = 0;
+    for (int s = 0; s < ns; ++s) open += K.h_mask[s] != 0;
+    K.h_n[ns] = 0;
+    if (open >= kTridiagDev && nv <= kTridiagMax) {
+      launch_tridiag_lowest(ns, K.h_n, nv, K.h_a, K.h_beta, K.cdev.template as<double>(), mlanc + 1, K.h_e0, K.h_n + ns,
+                            c.stream);
+      ++c.launches;
+    } else {
+      std::fill(K.h_cdev, K.h_cdev + (size_t)ns * (mlanc + 1), 0.0);
+      for (int s = 0; s < ns; ++s) {
+        const int m = K.h_n[s];
+        if (m == 0) continue;
+        eig.resize(m);
+        std::vector<double> e(m, 0.0);
+        for (int i = 0; i < m; ++i) eig[i] = K.h_a[(size_t)i * ns + s];
+        for (int i = 0; i + 1 < m; ++i) e[i] = K.h_beta[(size_t)(i + 1) * ns + s];
+        tridiag_eig(m, eig, e, z);
+        K.h_e0[s] = eig[0];
+        std::copy(z.begin(), z.begin() + m, K.h_cdev + (size_t)s * (mlanc + 1));
+      }
+      SADMRG_CUDA(cudaMemcpyAsync(K.cdev.get(), K.h_cdev, sizeof(double) * (size_t)ns * (mlanc + 1),
+                                  cudaMemcpyHostToDevice, c.stream));
+    }
     SADMRG_CUDA(cudaMemcpyAsync(K.mask.get(), K.h_mask, sizeof(int) * ns, cudaMemcpyHostToDevice, c.stream));
     launch_vec_lincomb(CX, K.on(K.mask), v, K.F(0), N, nv, K.cdev.template as<double>(), mlanc + 1,
                        K.partial.template as<double>(), K.counter.template as<unsigned>(), to_norm, c.stream);
@@ -236,19 +261,13 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
     o.hstride = 2;
     K.mdot(m, vv, 2, hv, o);
     SADMRG_CUDA(cudaStreamSynchronize(c.stream));
+    if (K.h_n[ns]) throw Error(SADMRG_ERR_NUMERIC, "tridiagonal QL did not converge");
     for (int s = 0; s < ns; ++s) {
       if (!K.h_mask[s]) continue;
       const double prod = std::sqrt(std::fabs(real_of(K.h_dots[2 * s + 1])));
       ov[s] = prod > 0 ? std::abs(K.h_dots[2 * s]) / prod : 0.0;
     }
   };
-  auto tridiag = [&](int s, int m, std::vector<double>& eig, std::vector<double>& z) {
-    eig.assign(aal[s].begin(), aal[s].begin() + m);
-    std::vector<double> e(m, 0.0);
-    for (int i = 0; i + 1 < m; ++i) e[i] = nnl[s][i + 1];
-    tridiag_eig(m, eig, e, z);
-  };
-
   // F(0) = normalised v
   K.mdot(K.all, v, 1, v, to_norm);
   launch_vec_div(CX, K.all, v, K.F(0), nullptr, K.norm.template as<double>(), 1, 1e-12, c.stream);
@@ -290,17 +309,13 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
     for (int s = 0; s < ns; ++s) {
       if (done[s]) continue;
       for (int j = synced + 1; j <= m; ++j) {
-        aal[s][j - 1] = K.h_a[(size_t)(j - 1) * ns + s];
-        nnl[s][j] = K.h_beta[(size_t)j * ns + s];
-        if (!brk[s] && j >= 2 && nnl[s][j] < tol) brk[s] = j;
+        if (!brk[s] && j >= 2 && K.h_beta[(size_t)j * ns + s] < tol) brk[s] = j;
       }
     }
     synced = m;
   };
 
-  std::vector<double> eig, z;
   std::vector<int> brk;
-  std::vector<double> e0(ns, 0.0);
   std::vector<int> finishing(ns, 0);
   step(1);
   if (mlanc > 2) {
@@ -310,15 +325,12 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
       sync_to(m, brk);
       bool any = false;
       std::fill(K.h_mask, K.h_mask + ns, 0);
-      std::fill(K.h_cdev, K.h_cdev + (size_t)ns * (mlanc + 1), 0.0);
+      std::fill(K.h_n, K.h_n + ns, 0);
       for (int s = 0; s < ns; ++s) {
         finishing[s] = 0;
         if (done[s]) continue;
-        const int mm = brk[s] ? brk[s] : m;
         if (!brk[s] && m % 4 != 0) continue;
-        tridiag(s, mm, eig, z);
-        e0[s] = eig[0];
-        for (int j = 0; j < mm; ++j) K.h_cdev[(size_t)s * (mlanc + 1) + j] = z[j];
+        K.h_n[s] = brk[s] ? brk[s] : m;
         K.h_mask[s] = 1;
         finishing[s] = brk[s] ? 1 : 0;
         any = true;
@@ -330,7 +342,7 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
       for (int s = 0; s < ns; ++s) {
         if (K.h_mask[s] && (finishing[s] || std::fabs(ov[s] - 1.0) < c.lanczos_ov_tol)) {
           done[s] = 1;
-          st.energy[s] = e0[s];
+          st.energy[s] = K.h_e0[s];
           K.h_active[s] = 0;
           changed = true;
         }
@@ -351,13 +363,11 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
   K.mdot(K.on(K.active), K.F(last), 1, K.F(last + 1), od);
   SADMRG_CUDA(cudaStreamSynchronize(c.stream));
   std::fill(K.h_mask, K.h_mask + ns, 0);
-  std::fill(K.h_cdev, K.h_cdev + (size_t)ns * (mlanc + 1), 0.0);
+  std::fill(K.h_n, K.h_n + ns, 0);
   for (int s = 0; s < ns; ++s) {
     if (done[s]) continue;
-    aal[s][last] = real_of(K.h_dots[s]);
-    tridiag(s, last + 1, eig, z);
-    e0[s] = eig[0];
-    for (int j = 0; j <= last; ++j) K.h_cdev[(size_t)s * (mlanc + 1) + j] = z[j];
+    K.h_a[(size_t)last * ns + s] = real_of(K.h_dots[s]);
+    K.h_n[s] = last + 1;
     K.h_mask[s] = 1;
   }
   ritz(last + 1);
@@ -365,7 +375,7 @@ BatchStats batch_lanczos1(Ctx& c, const HeffBatch<S>& B, S* v, int mlanc, int pr
   for (int s = 0; s < ns; ++s)
     if (!done[s]) {
       done[s] = 1;
-      st.energy[s] = e0[s];
+      st.energy[s] = K.h_e0[s];
     }
   return st;
 }

@@ -245,6 +245,15 @@ void launch_vec_lincomb(bool cplx, const VecSpan& v, void* y, const void* V, lon
 void launch_vec_div(bool cplx, const VecSpan& v, const void* x, void* y, void* y2, const double* scal, int sstride,
                     double floor, cudaStream_t s);
 
+// Lowest eigenvalue (e0[s]) and its vector (z0[s * zstride + i], zeros to i = nmax) of ns
+// symmetric tridiagonals of n[s] <= nmax <= kTridiagMax rows (0: none), diagonal a[i * ns + s],
+// coupling of i and i + 1 b[(i + 1) * ns + s]; as tridiag_eig (dmrg.cpp) bit for bit.
+// *status = 1 where one did not converge.  n, a, b, e0 and status may be page-locked host
+// memory.
+constexpr int kTridiagMax = 128;
+void launch_tridiag_lowest(int ns, const int* n, int nmax, const double* a, const double* b, double* z0, int zstride,
+                           double* e0, int* status, cudaStream_t s);
+
 // ---- one-sided Jacobi SVD of sector blocks --------------------------------
 struct SvdJob {
   long long aoff;             // input block (m x n, lda = m) in the input buffer
