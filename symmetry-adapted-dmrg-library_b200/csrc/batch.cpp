@@ -144,12 +144,15 @@ struct BatchKrylov {
     SADMRG_CUDA(cudaMemsetAsync(beta.get(), 0, beta.bytes(), c.stream));
     SADMRG_CUDA(cudaMemsetAsync(counter.get(), 0, counter.bytes(), c.stream));
     SADMRG_CUDA(cudaMemsetAsync(norm.get(), 0, norm.bytes(), c.stream));
-    // page-locked scalars, one allocation
-    const size_t na = (size_t)ns * (mlanc + 1), nb = (size_t)ns * (mlanc + 2), nd = sizeof(S) / sizeof(double) * 2 * ns;
-    SADMRG_CUDA(cudaMallocHost(&h_a, sizeof(double) * (na + nb + nd + na + ns) + sizeof(int) * (3 * (size_t)ns + 1)));
+    // page-locked scalars, one allocation: the dots, which may be complex, first (16-byte
+    // aligned), then doubles, then ints
+    const size_t na = (size_t)ns * (mlanc + 1), nb = (size_t)ns * (mlanc + 2);
+    void* pinned = nullptr;
+    SADMRG_CUDA(cudaMallocHost(&pinned, sizeof(S) * 2 * ns + sizeof(double) * (2 * na + nb + ns) + sizeof(int) * (3 * (size_t)ns + 1)));
+    h_dots = static_cast<S*>(pinned);
+    h_a = reinterpret_cast<double*>(h_dots + 2 * ns);
     h_beta = h_a + na;
-    h_dots = reinterpret_cast<S*>(h_beta + nb);
-    h_cdev = h_beta + nb + nd;
+    h_cdev = h_beta + nb;
     h_e0 = h_cdev + na;
     h_mask = reinterpret_cast<int*>(h_e0 + ns);
     h_active = h_mask + ns;
@@ -163,7 +166,7 @@ struct BatchKrylov {
   }
   ~BatchKrylov() {
     cudaStreamSynchronize(c.stream);
-    cudaFreeHost(h_a);
+    cudaFreeHost(h_dots);
   }
   S* F(int i) { return ff.as<S>() + (size_t)i * N; }
   VecSpan on(const DevBuf& m) const {   // the segments whose flag in m is set
