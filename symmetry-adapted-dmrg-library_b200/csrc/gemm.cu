@@ -19,6 +19,7 @@
 #include <mutex>
 
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace sadmrg {
 
@@ -364,6 +365,7 @@ template <bool CX>
 __global__ void __launch_bounds__(kThreads, 3) items_f64(const __grid_constant__ ItemArgs args) {
   using T = typename GTile<CX>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  chain_begin();
   const WorkItem it = args.items[blockIdx.x];
   if (args.mask && !args.mask[it.tag]) return;   // instance switched off for this launch
   T* const smem = reinterpret_cast<T*>(smem_raw);
@@ -390,7 +392,7 @@ template <bool CX>
 static void launch_items_t(const ItemArgs& a, int nitems, cudaStream_t s) {
   static unsigned char attr[kMaxDevices] = {0};
   ensure_smem_attr((const void*)items_f64<CX>, GSmem<CX>::bytes, attr);
-  items_f64<CX><<<nitems, kThreads, GSmem<CX>::bytes, s>>>(a);
+  launch_chained(items_f64<CX>, nitems, kThreads, GSmem<CX>::bytes, s, a);
 }
 
 void launch_items(bool cplx, const WorkItem* items, const ItemSeg* segs, int nitems, const Bases& b, void* work,

@@ -7,6 +7,7 @@
 #include <cstdio>
 
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace sadmrg {
 
@@ -14,6 +15,7 @@ namespace sadmrg {
 // block utilities
 template <bool CPLX>
 __global__ void seg_axpy_kernel(void* y, const void* x, const Seg* segs) {
+  chain_begin();
   const Seg sg = segs[blockIdx.x];
   const long long stride = (long long)blockDim.x * gridDim.y;
   for (long long i = (long long)blockIdx.y * blockDim.x + threadIdx.x; i < sg.n; i += stride) {
@@ -31,12 +33,13 @@ __global__ void seg_axpy_kernel(void* y, const void* x, const Seg* segs) {
 void launch_seg_axpy(bool cplx, void* y, const void* x, const Seg* segs, int nseg, cudaStream_t s) {
   if (nseg <= 0) return;
   dim3 grid(nseg, 16);
-  if (cplx) seg_axpy_kernel<true><<<grid, 256, 0, s>>>(y, x, segs);
-  else seg_axpy_kernel<false><<<grid, 256, 0, s>>>(y, x, segs);
+  if (cplx) launch_chained(seg_axpy_kernel<true>, grid, 256, 0, s, y, x, segs);
+  else launch_chained(seg_axpy_kernel<false>, grid, 256, 0, s, y, x, segs);
 }
 
 template <class T>
 __global__ void block_transpose_kernel(T* dst, const T* src, const Transp* jobs) {
+  chain_begin();
   __shared__ T tile[32][33];
   const Transp tj = jobs[blockIdx.x];
   const int tr = (tj.rows + 31) / 32, tc = (tj.cols + 31) / 32;
@@ -59,8 +62,8 @@ __global__ void block_transpose_kernel(T* dst, const T* src, const Transp* jobs)
 void launch_block_transpose(bool cplx, void* dst, const void* src, const Transp* t, int nt, cudaStream_t s) {
   if (nt <= 0) return;
   dim3 grid(nt, 32);
-  if (cplx) block_transpose_kernel<double2><<<grid, 256, 0, s>>>((double2*)dst, (const double2*)src, t);
-  else block_transpose_kernel<double><<<grid, 256, 0, s>>>((double*)dst, (const double*)src, t);
+  if (cplx) launch_chained(block_transpose_kernel<double2>, grid, 256, 0, s, (double2*)dst, (const double2*)src, t);
+  else launch_chained(block_transpose_kernel<double>, grid, 256, 0, s, (double*)dst, (const double*)src, t);
 }
 
 // leg permutation of 3-leg blocks: one block of threads per tensor block, every
@@ -68,6 +71,7 @@ void launch_block_transpose(bool cplx, void* dst, const void* src, const Transp*
 // projected lower states of an excited-state sweep, are small)
 template <class T>
 __global__ void permute3_kernel(T* dst, const T* src, const Perm3* jobs) {
+  chain_begin();
   const Perm3 J = jobs[blockIdx.x];
   const long long nd0 = J.d[J.p[0]], nd1 = J.d[J.p[1]], n = (long long)J.d[0] * J.d[1] * J.d[2];
   const long long st[3] = {1, J.d[0], (long long)J.d[0] * J.d[1]};   // source strides
@@ -80,12 +84,13 @@ __global__ void permute3_kernel(T* dst, const T* src, const Perm3* jobs) {
 void launch_permute3(bool cplx, void* dst, const void* src, const Perm3* t, int nt, cudaStream_t s) {
   if (nt <= 0) return;
   dim3 grid(nt, 8);
-  if (cplx) permute3_kernel<double2><<<grid, 256, 0, s>>>((double2*)dst, (const double2*)src, t);
-  else permute3_kernel<double><<<grid, 256, 0, s>>>((double*)dst, (const double*)src, t);
+  if (cplx) launch_chained(permute3_kernel<double2>, grid, 256, 0, s, (double2*)dst, (const double2*)src, t);
+  else launch_chained(permute3_kernel<double>, grid, 256, 0, s, (double*)dst, (const double*)src, t);
 }
 
 template <bool CPLX>
 __global__ void fuse_fill_kernel(void* data, const FuseFill* f) {
+  chain_begin();
   const FuseFill ff = f[blockIdx.x];
   const long long plane = (long long)ff.d0 * ff.d1;
   for (long long e = threadIdx.x; e < plane; e += blockDim.x) {
@@ -98,12 +103,13 @@ __global__ void fuse_fill_kernel(void* data, const FuseFill* f) {
 
 void launch_fuse_fill(bool cplx, void* data, const FuseFill* f, int nf, cudaStream_t s) {
   if (nf <= 0) return;
-  if (cplx) fuse_fill_kernel<true><<<nf, 256, 0, s>>>(data, f);
-  else fuse_fill_kernel<false><<<nf, 256, 0, s>>>(data, f);
+  if (cplx) launch_chained(fuse_fill_kernel<true>, nf, 256, 0, s, data, f);
+  else launch_chained(fuse_fill_kernel<false>, nf, 256, 0, s, data, f);
 }
 
 template <bool CPLX>
 __global__ void gather_kernel(void* dst, const void* src, const double* w, const int* perm, const Gather* g) {
+  chain_begin();
   const Gather G = g[blockIdx.x];
   const long long total = (long long)G.rows * G.kept;
   for (long long e = (long long)blockIdx.y * blockDim.x + threadIdx.x; e < total; e += (long long)blockDim.x * gridDim.y) {
@@ -127,12 +133,13 @@ void launch_gather(bool cplx, void* dst, const void* src, const double* w, const
                    cudaStream_t s) {
   if (ng <= 0) return;
   dim3 grid(ng, 8);
-  if (cplx) gather_kernel<true><<<grid, 256, 0, s>>>(dst, src, w, perm, g);
-  else gather_kernel<false><<<grid, 256, 0, s>>>(dst, src, w, perm, g);
+  if (cplx) launch_chained(gather_kernel<true>, grid, 256, 0, s, dst, src, w, perm, g);
+  else launch_chained(gather_kernel<false>, grid, 256, 0, s, dst, src, w, perm, g);
 }
 
 template <bool CPLX>
 __global__ void scale_kernel(void* x, double ar, double ai, long long n) {
+  chain_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)blockDim.x * gridDim.x) {
     if (CPLX) {
       const double2 v = static_cast<double2*>(x)[i];
@@ -146,8 +153,8 @@ __global__ void scale_kernel(void* x, double ar, double ai, long long n) {
 void launch_scale(bool cplx, void* x, double ar, double ai, long long n, cudaStream_t s) {
   if (n <= 0) return;
   const int blocks = (int)min((n + 255) / 256, 148LL * 8);
-  if (cplx) scale_kernel<true><<<blocks, 256, 0, s>>>(x, ar, ai, n);
-  else scale_kernel<false><<<blocks, 256, 0, s>>>(x, ar, ai, n);
+  if (cplx) launch_chained(scale_kernel<true>, blocks, 256, 0, s, x, ar, ai, n);
+  else launch_chained(scale_kernel<false>, blocks, 256, 0, s, x, ar, ai, n);
 }
 
 // Reads bytes (a multiple of 16) of x; writes sink only when the xor of all
@@ -168,6 +175,7 @@ void launch_read(const void* x, long long bytes, unsigned* sink, cudaStream_t s)
 
 template <bool CPLX>
 __global__ void fill_kernel(void* x, double vr, double vi, long long n) {
+  chain_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)blockDim.x * gridDim.x) {
     if (CPLX) static_cast<double2*>(x)[i] = make_double2(vr, vi);
     else static_cast<double*>(x)[i] = vr;
@@ -177,8 +185,8 @@ __global__ void fill_kernel(void* x, double vr, double vi, long long n) {
 void launch_fill(bool cplx, void* x, double vr, double vi, long long n, cudaStream_t s) {
   if (n <= 0) return;
   const int blocks = (int)min((n + 255) / 256, 148LL * 8);
-  if (cplx) fill_kernel<true><<<blocks, 256, 0, s>>>(x, vr, vi, n);
-  else fill_kernel<false><<<blocks, 256, 0, s>>>(x, vr, vi, n);
+  if (cplx) launch_chained(fill_kernel<true>, blocks, 256, 0, s, x, vr, vi, n);
+  else launch_chained(fill_kernel<false>, blocks, 256, 0, s, x, vr, vi, n);
 }
 
 }  // namespace sadmrg

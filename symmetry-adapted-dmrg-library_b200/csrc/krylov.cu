@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace sadmrg {
 namespace {
@@ -127,13 +128,14 @@ __device__ __forceinline__ void norm_out(const VecOut& o, int seg, double sum) {
 // out[seg * nv + j] = <V_j | x>, after x -= uc[0] u0 + uc[1] u1 when u1 is given
 // (u0 may be null).  See VecOut for what the last block does with the sums.
 template <bool CX>
-__global__ void __launch_bounds__(kVT) vec_dots(VecSpan v, const typename VT_<CX>::T* __restrict__ V, long long ldv,
+__global__ void __launch_bounds__(kVT) vec_dots(VecSpan v, const typename VT_<CX>::T* V, long long ldv,
                                                 int nv, typename VT_<CX>::T* x, const typename VT_<CX>::T* u0,
                                                 const typename VT_<CX>::T* u1, const typename VT_<CX>::T* uc,
                                                 double* partial, typename VT_<CX>::T* out, unsigned* counter,
                                                 VecOut o) {
   using T = typename VT_<CX>::T;
   __shared__ double red[2][CX ? 2 : 1][kVW][kG];
+  chain_begin();
   Range r;
   if (!block_range(v, r)) return;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -223,13 +225,14 @@ __global__ void __launch_bounds__(kVT) vec_dots(VecSpan v, const typename VT_<CX
 // to o.scal and o.host (as VO_NORM).
 template <bool CX>
 __global__ void __launch_bounds__(kVT) vec_axpy(VecSpan v, typename VT_<CX>::T* x,
-                                                const typename VT_<CX>::T* __restrict__ V, long long ldv, int nv,
+                                                const typename VT_<CX>::T* V, long long ldv, int nv,
                                                 const typename VT_<CX>::T* c, int cstride, double* partial,
                                                 unsigned* counter, VecOut o) {
   using T = typename VT_<CX>::T;
   extern __shared__ __align__(16) unsigned char csm[];
   __shared__ double red[kVW];
   T* cs = reinterpret_cast<T*>(csm);
+  chain_begin();
   Range r;
   if (!block_range(v, r)) return;
   for (int j = threadIdx.x; j < nv; j += kVT) cs[j] = c[(long long)r.seg * cstride + j];
@@ -271,13 +274,14 @@ __global__ void __launch_bounds__(kVT) vec_axpy(VecSpan v, typename VT_<CX>::T* 
 // y = sum_j c[seg * cstride + j] V_j (real c); with a partial buffer also |y| (as VO_NORM)
 template <bool CX>
 __global__ void __launch_bounds__(kVT) vec_lincomb(VecSpan v, typename VT_<CX>::T* y,
-                                                   const typename VT_<CX>::T* __restrict__ V, long long ldv, int nv,
+                                                   const typename VT_<CX>::T* V, long long ldv, int nv,
                                                    const double* c, int cstride, double* partial, unsigned* counter,
                                                    VecOut o) {
   using T = typename VT_<CX>::T;
   extern __shared__ __align__(16) unsigned char csm[];
   __shared__ double red[kVW];
   double* cs = reinterpret_cast<double*>(csm);
+  chain_begin();
   Range r;
   if (!block_range(v, r)) return;
   for (int j = threadIdx.x; j < nv; j += kVT) cs[j] = c[(long long)r.seg * cstride + j];
@@ -320,6 +324,7 @@ __global__ void __launch_bounds__(kVT) vec_lincomb(VecSpan v, typename VT_<CX>::
 template <bool CX>
 __global__ void __launch_bounds__(kVT) vec_div(VecSpan v, const typename VT_<CX>::T* x, typename VT_<CX>::T* y,
                                                typename VT_<CX>::T* y2, const double* scal, int sstride, double floor) {
+  chain_begin();
   Range r;
   if (!block_range(v, r)) return;
   const double d = scal[(long long)r.seg * sstride];
@@ -350,10 +355,10 @@ void launch_vec_dots(bool cplx, const VecSpan& v, const void* V, long long ldv, 
                      cudaStream_t s) {
   if (nv <= 0 || v.nblk <= 0) return;
   if (cplx)
-    vec_dots<true><<<v.nblk, kVT, 0, s>>>(v, (const double2*)V, ldv, nv, (double2*)x, (const double2*)u0,
+    launch_chained(vec_dots<true>, v.nblk, kVT, 0, s, v, (const double2*)V, ldv, nv, (double2*)x, (const double2*)u0,
                                           (const double2*)u1, (const double2*)uc, partial, (double2*)out, counter, o);
   else
-    vec_dots<false><<<v.nblk, kVT, 0, s>>>(v, (const double*)V, ldv, nv, (double*)x, (const double*)u0,
+    launch_chained(vec_dots<false>, v.nblk, kVT, 0, s, v, (const double*)V, ldv, nv, (double*)x, (const double*)u0,
                                            (const double*)u1, (const double*)uc, partial, (double*)out, counter, o);
 }
 
@@ -361,10 +366,10 @@ void launch_vec_axpy(bool cplx, const VecSpan& v, void* x, const void* V, long l
                      int cstride, double* partial, unsigned* counter, const VecOut& o, cudaStream_t s) {
   if (v.nblk <= 0) return;
   if (cplx)
-    vec_axpy<true><<<v.nblk, kVT, nv * sizeof(double2), s>>>(v, (double2*)x, (const double2*)V, ldv, nv,
+    launch_chained(vec_axpy<true>, v.nblk, kVT, nv * sizeof(double2), s, v, (double2*)x, (const double2*)V, ldv, nv,
                                                               (const double2*)c, cstride, partial, counter, o);
   else
-    vec_axpy<false><<<v.nblk, kVT, nv * sizeof(double), s>>>(v, (double*)x, (const double*)V, ldv, nv,
+    launch_chained(vec_axpy<false>, v.nblk, kVT, nv * sizeof(double), s, v, (double*)x, (const double*)V, ldv, nv,
                                                               (const double*)c, cstride, partial, counter, o);
 }
 
@@ -372,10 +377,10 @@ void launch_vec_lincomb(bool cplx, const VecSpan& v, void* y, const void* V, lon
                         int cstride, double* partial, unsigned* counter, const VecOut& o, cudaStream_t s) {
   if (v.nblk <= 0) return;
   if (cplx)
-    vec_lincomb<true><<<v.nblk, kVT, nv * sizeof(double), s>>>(v, (double2*)y, (const double2*)V, ldv, nv, c, cstride,
+    launch_chained(vec_lincomb<true>, v.nblk, kVT, nv * sizeof(double), s, v, (double2*)y, (const double2*)V, ldv, nv, c, cstride,
                                                                 partial, counter, o);
   else
-    vec_lincomb<false><<<v.nblk, kVT, nv * sizeof(double), s>>>(v, (double*)y, (const double*)V, ldv, nv, c, cstride,
+    launch_chained(vec_lincomb<false>, v.nblk, kVT, nv * sizeof(double), s, v, (double*)y, (const double*)V, ldv, nv, c, cstride,
                                                                  partial, counter, o);
 }
 
@@ -383,9 +388,9 @@ void launch_vec_div(bool cplx, const VecSpan& v, const void* x, void* y, void* y
                     double floor, cudaStream_t s) {
   if (v.nblk <= 0) return;
   if (cplx)
-    vec_div<true><<<v.nblk, kVT, 0, s>>>(v, (const double2*)x, (double2*)y, (double2*)y2, scal, sstride, floor);
+    launch_chained(vec_div<true>, v.nblk, kVT, 0, s, v, (const double2*)x, (double2*)y, (double2*)y2, scal, sstride, floor);
   else
-    vec_div<false><<<v.nblk, kVT, 0, s>>>(v, (const double*)x, (double*)y, (double*)y2, scal, sstride, floor);
+    launch_chained(vec_div<false>, v.nblk, kVT, 0, s, v, (const double*)x, (double*)y, (double*)y2, scal, sstride, floor);
 }
 
 }  // namespace sadmrg

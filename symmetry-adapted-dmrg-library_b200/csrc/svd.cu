@@ -22,6 +22,7 @@
 
 #include "common.hpp"
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace sadmrg {
 
@@ -900,6 +901,7 @@ __global__ void __launch_bounds__(kSvdThreads) jacobi_coop_kernel(const SvdJob* 
 // caller has set W and V itself)
 template <bool CPLX>
 __global__ void jacobi_init_kernel(const SvdJob* jobs, const void* a, void* work, void* vmat, int* perm, int copy) {
+  chain_begin();
   using T = typename SvdT<CPLX>::T;
   const SvdJob J = jobs[blockIdx.x];
   const int R = J.trans ? J.n : J.m, C = J.trans ? J.m : J.n;
@@ -929,6 +931,7 @@ __global__ void jacobi_init_kernel(const SvdJob* jobs, const void* a, void* work
 
 template <bool CPLX>
 __global__ void jacobi_norms_kernel(const SvdJob* jobs, const void* work, double* sv) {
+  chain_begin();
   using T = typename SvdT<CPLX>::T;
   const SvdJob J = jobs[blockIdx.x];
   const int R = J.trans ? J.n : J.m, C = J.trans ? J.m : J.n;
@@ -1010,6 +1013,7 @@ __device__ __forceinline__ T op_a(const T* A, int m, int trans, int r, int c) {
 // Column norms of op(A) and their order (decreasing, ties by index): P.
 template <bool CPLX>
 __global__ void qr_order_kernel(const QrJob* jobs, const void* a, double* nrm, int* perm) {
+  chain_begin();
   using T = typename SvdT<CPLX>::T;
   const QrJob J = jobs[blockIdx.x];
   const T* A = static_cast<const T*>(a) + J.aoff;
@@ -1036,6 +1040,7 @@ __global__ void qr_order_kernel(const QrJob* jobs, const void* a, double* nrm, i
 // W0 = op(A) P
 template <bool CPLX>
 __global__ void qr_gather_kernel(const QrJob* jobs, const void* a, void* qbuf, const int* perm) {
+  chain_begin();
   using T = typename SvdT<CPLX>::T;
   const QrJob J = jobs[blockIdx.x];
   const T* A = static_cast<const T*>(a) + J.aoff;
@@ -1280,6 +1285,7 @@ __global__ void __launch_bounds__(kSvdThreads) qr_unmq_kernel(const QrJob* __res
 // (to_jacobi = 0), or into dst's Jacobi W with V = I (to_jacobi = 1).
 template <bool CPLX>
 __global__ void qr_rh_kernel(const QrJob* src, const QrJob* dst, void* qbuf, int to_jacobi) {
+  chain_begin();
   using T = typename SvdT<CPLX>::T;
   const QrJob S = src[blockIdx.x], D = dst[blockIdx.x];
   const T* A = static_cast<const T*>(qbuf) + S.qoff;
@@ -1297,6 +1303,7 @@ __global__ void qr_rh_kernel(const QrJob* src, const QrJob* dst, void* qbuf, int
 // Before the Q applications: the output W = [R1^H V2; 0] (R x C).
 template <bool CPLX>
 __global__ void qr_wout_kernel(const QrJob* jobs, const void* qbuf, void* work) {
+  chain_begin();
   using T = typename SvdT<CPLX>::T;
   const QrJob J = jobs[blockIdx.x];
   const T* Wj = static_cast<const T*>(qbuf) + J.jwoff;
@@ -1311,6 +1318,7 @@ __global__ void qr_wout_kernel(const QrJob* jobs, const void* qbuf, void* work) 
 // After them: the output V = P (Q1 V2), rows put back in the order of op(A)'s columns.
 template <bool CPLX>
 __global__ void qr_vout_kernel(const QrJob* jobs, const void* qbuf, void* vmat, const int* perm) {
+  chain_begin();
   using T = typename SvdT<CPLX>::T;
   const QrJob J = jobs[blockIdx.x];
   const T* Vj = static_cast<const T*>(qbuf) + J.jvoff;
@@ -1439,7 +1447,7 @@ static int jacobi_run(const void* a, void* work, void* vmat, double* sv, const s
   int* pcnt = reinterpret_cast<int*>(zero + o_cnt);
   unsigned* pbar = reinterpret_cast<unsigned*>(zero + o_bar);
   int* pperm = dperm.as<int>();
-  jacobi_init_kernel<CPLX><<<dim3(nj, 16), 256, 0, s>>>(pj, a, work, vmat, pperm, copy);
+  launch_chained(jacobi_init_kernel<CPLX>, dim3(nj, 16), 256, 0, s, pj, a, work, vmat, pperm, copy);
   SADMRG_CUDA(cudaGetLastError());
   double tol = std::sqrt((double)std::max(maxR, 1)) * 2.220446049250313e-16;
   int njv = nj;
@@ -1449,7 +1457,7 @@ static int jacobi_run(const void* a, void* work, void* vmat, double* sv, const s
   SADMRG_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)ctas.size()), dim3(kSvdThreads), args, smem, s));
   SvdCtl hctl{};
   SADMRG_CUDA(cudaMemcpyAsync(&hctl, pctl, sizeof(SvdCtl), cudaMemcpyDeviceToHost, s));
-  jacobi_norms_kernel<CPLX><<<nj, 256, 0, s>>>(pj, work, sv);
+  launch_chained(jacobi_norms_kernel<CPLX>, nj, 256, 0, s, pj, work, sv);
   SADMRG_CUDA(cudaGetLastError());
   SADMRG_CUDA(cudaStreamSynchronize(s));
   SADMRG_REQUIRE(hctl.status == 0, SADMRG_ERR_CUDA, "jacobi svd: a barrier ran out of time");
@@ -1600,8 +1608,8 @@ static int qr_jacobi_run(const void* a, void* work, void* vmat, double* sv, cons
   // P and W0 = op(A) P need the job array on the device: the first QR's copy
   L1.dj.alloc(sizeof(QrJob) * nj, s);
   SADMRG_CUDA(cudaMemcpyAsync(L1.dj.get(), q1.data(), sizeof(QrJob) * nj, cudaMemcpyHostToDevice, s));
-  qr_order_kernel<CPLX><<<nj, kSvdThreads, 0, s>>>(static_cast<const QrJob*>(L1.dj.get()), a, sv, dperm.as<int>());
-  qr_gather_kernel<CPLX><<<dim3(nj, 32), 256, 0, s>>>(static_cast<const QrJob*>(L1.dj.get()), a, qbuf.get(), dperm.as<int>());
+  launch_chained(qr_order_kernel<CPLX>, nj, kSvdThreads, 0, s, static_cast<const QrJob*>(L1.dj.get()), a, sv, dperm.as<int>());
+  launch_chained(qr_gather_kernel<CPLX>, dim3(nj, 32), 256, 0, s, static_cast<const QrJob*>(L1.dj.get()), a, qbuf.get(), dperm.as<int>());
   SADMRG_CUDA(cudaGetLastError());
   if (!L1.run(q1, false, qbuf.get(), work, ctl, s)) {
     *fallback = true;
@@ -1609,11 +1617,11 @@ static int qr_jacobi_run(const void* a, void* work, void* vmat, double* sv, cons
   }
   L2.dj.alloc(sizeof(QrJob) * nj, s);
   SADMRG_CUDA(cudaMemcpyAsync(L2.dj.get(), q2.data(), sizeof(QrJob) * nj, cudaMemcpyHostToDevice, s));
-  qr_rh_kernel<CPLX><<<dim3(nj, 16), 256, 0, s>>>(static_cast<const QrJob*>(L1.dj.get()), static_cast<const QrJob*>(L2.dj.get()), qbuf.get(), 0);
+  launch_chained(qr_rh_kernel<CPLX>, dim3(nj, 16), 256, 0, s, static_cast<const QrJob*>(L1.dj.get()), static_cast<const QrJob*>(L2.dj.get()), qbuf.get(), 0);
   SADMRG_CUDA(cudaGetLastError());
   SADMRG_REQUIRE(L2.run(q2, false, qbuf.get(), work, ctl + 1, s), SADMRG_ERR_CUDA,
                  "svd: the second cooperative QR cannot be launched");
-  qr_rh_kernel<CPLX><<<dim3(nj, 16), 256, 0, s>>>(static_cast<const QrJob*>(L2.dj.get()), static_cast<const QrJob*>(L2.dj.get()), qbuf.get(), 1);
+  launch_chained(qr_rh_kernel<CPLX>, dim3(nj, 16), 256, 0, s, static_cast<const QrJob*>(L2.dj.get()), static_cast<const QrJob*>(L2.dj.get()), qbuf.get(), 1);
   SADMRG_CUDA(cudaGetLastError());
   // the Jacobi on R1^H (C x C, W and V in qbuf)
   std::vector<SvdJob> jj(nj);
@@ -1633,13 +1641,13 @@ static int qr_jacobi_run(const void* a, void* work, void* vmat, double* sv, cons
                          : jacobi_run<CPLX, 16>(nullptr, qbuf.get(), qbuf.get(), sv, jj, max_sweeps, s, &jms, 0, stream);
   if (sweeps <= 0) return sweeps;
   // W = Q [R1^H V2; 0] and Q1 V2, both Q applications in one launch, then V = P (Q1 V2)
-  qr_wout_kernel<CPLX><<<dim3(nj, 16), 256, 0, s>>>(static_cast<const QrJob*>(L1.dj.get()), qbuf.get(), work);
+  launch_chained(qr_wout_kernel<CPLX>, dim3(nj, 16), 256, 0, s, static_cast<const QrJob*>(L1.dj.get()), qbuf.get(), work);
   SADMRG_CUDA(cudaGetLastError());
   std::vector<QrJob> qu(q1);
   qu.insert(qu.end(), q2.begin(), q2.end());
   SADMRG_REQUIRE(LU.run(qu, true, qbuf.get(), work, ctl + 2, s), SADMRG_ERR_CUDA,
                  "svd: the cooperative Q application cannot be launched");
-  qr_vout_kernel<CPLX><<<dim3(nj, 16), 256, 0, s>>>(static_cast<const QrJob*>(L1.dj.get()), qbuf.get(), vmat, dperm.as<int>());
+  launch_chained(qr_vout_kernel<CPLX>, dim3(nj, 16), 256, 0, s, static_cast<const QrJob*>(L1.dj.get()), qbuf.get(), vmat, dperm.as<int>());
   SADMRG_CUDA(cudaGetLastError());
   SvdCtl hctl[3];
   SADMRG_CUDA(cudaMemcpyAsync(hctl, dctl.get(), 3 * sizeof(SvdCtl), cudaMemcpyDeviceToHost, s));

@@ -17,6 +17,7 @@
 
 #include "common.hpp"
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace sadmrg {
 namespace {
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(32) tridiag_lowest_kernel(int ns, const int* n
                                                             const double* b, double* z0, int zstride, double* e0,
                                                             int* status) {
   extern __shared__ double sm[];
+  chain_begin();
   const int s = blockIdx.x, n = nn[s], lane = threadIdx.x;
   if (n <= 0) return;
   double* d = sm;               // a of row i: a[i * ns + s]; coupling of i and i + 1: b[(i + 1) * ns + s]
@@ -182,7 +184,7 @@ void launch(int ns, const int* n, int nmax, const double* a, const double* b, do
             int* status, cudaStream_t s) {
   const size_t smem = smem_of(nmax);
   SADMRG_CUDA(cudaFuncSetAttribute(tridiag_lowest_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  tridiag_lowest_kernel<NR><<<ns, 32, smem, s>>>(ns, n, nmax, a, b, z0, zstride, e0, status);
+  launch_chained(tridiag_lowest_kernel<NR>, ns, 32, smem, s, ns, n, nmax, a, b, z0, zstride, e0, status);
   SADMRG_CUDA(cudaGetLastError());
 }
 
