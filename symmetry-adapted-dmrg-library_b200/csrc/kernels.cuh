@@ -62,11 +62,12 @@ void launch_items(bool cplx, const WorkItem* items, const ItemSeg* segs, int nit
 
 // ---- tcgen05 3xTF32 over TF32 hi/lo operand panels (umma.cu) --------------
 // An operand (rows x K after op) is stored as panels: panel (p, s) holds rows
-// [p*T, p*T + T) and k [32 s, 32 s + 32) as a hi plane then a lo plane, each
-// [kg = 0..7][row = 0..T-1][4 consecutive k] of TF32 bit patterns (x ~ hi + lo),
-// zero padded; it starts at dst + (p * nslab + s) * T * 256 bytes.  This is the
-// K-major, no-swizzle core-matrix layout tcgen05.mma reads, so a panel moves
-// into shared memory as one contiguous bulk copy.
+// [p*T, p*T + T) and k [32 s, 32 s + 32) as groups of 8 rows, each a hi plane then a lo
+// plane, each [kg = 0..7][row = 0..7][4 consecutive k] of TF32 bit patterns (x ~ hi + lo),
+// zero padded in k; it starts at dst + (p * nslab + s) * T * 256 bytes.  This is the
+// K-major, no-swizzle core-matrix layout tcgen05.mma reads, and the rows that a block has
+// are the first bytes of its panel: one contiguous bulk copy of them moves into shared
+// memory, whatever the tile is padded to.
 // Complex products run as real ones of twice the size: C = A B (complex m x n,
 // k) is Ch = Ah Bh with Ch (2m x n) and Bh (2k x n) the interleaved storage of
 // C and B read as real column-major matrices (no copy), and Ah (2m x 2k) the
@@ -87,10 +88,10 @@ struct PackJob {              // FP64 matrix -> panels
   int sparse;                 // 1: chunks of the real rows and k only (the padding of the
                               // panels is zero already and never written), 0: whole panels
 };
-struct UTerm {                // a term's operands as panel sets: A (T = 128), B (T = BN)
-  long long a, b;             // byte offsets of panel (0, 0)
-  int abuf, bbuf;             // 0: constant panels, 1: per-apply panels
-  int nslab, klast;           // k slabs, k of the last slab (1..32)
+struct USlab {                // one slab of a job's concatenated reduction
+  long long a, b;             // byte offsets of its A and B panels of tile row / column 0
+  int nslab;                  // slabs of its term: panels of tile row p start p * nslab panels further on
+  int info;                   // its k (1..32), + 256 (+ 512): the A (B) panel is a per-apply one, else constant
   int adep, bdep;             // dependency counter of the A / B panels written in the same launch, or -1
 };
 struct UJob {                 // output tile grid of one job
@@ -98,15 +99,16 @@ struct UJob {                 // output tile grid of one job
   long long pack;             // >= 0: the result becomes A panels (T = 128) at this byte offset of the
                               // per-apply buffer, scaled by alpha, with pack_nslab slabs per panel
   double alpha;
-  int cbuf, m, n, ldc, flags, t0, nt, pack_nslab;
+  int cbuf, m, n, ldc, flags, pack_nslab;
   int dep;                    // counter bumped per finished tile (results read as panels later), or -1
   int tag;                    // as GemmJob::tag
   int cx;                     // complex plan: the tile is a real-form block (rows 2i, 2i+1 = Re, Im of
                               // row i); panels of the result are written in the real form Xh (cmode 1)
 };
 struct UItem {                // one output tile x a run of consecutive slabs
-  int job, tm, tn, t0, s0, nslab, slot;   // t0: first term (absolute), s0: its first slab; slot < 0: direct
+  int job, tm, tn, q0, nslab, slot;   // q0: first slab (absolute); slot < 0: direct
   int red;                    // split items: their tile's URed
+  int arows, brows;           // rows of the A and B panels that the tile's block has, to a multiple of 8
 };
 struct URed {                 // C tile = sum of FP32 partial slots [slot0, slot0 + nslot) in fixed order
   int job, tm, tn, slot0, nslot;
@@ -138,7 +140,7 @@ void launch_pack(const PackJob* jobs, const int* blk_job, int nblocks, const Bas
 // One launch of the tcgen05 executor: optional psi packing, then the items.  With
 // ph.wait_deps the whole matvec (pack, stage 0, stage 1) runs as one cooperative
 // launch, every item waiting (bounded) for the panels it reads.
-void launch_umma_items(int bn, const UTerm* terms, const UJob* jobs, const UItem* items, const URed* reds, int nitems,
+void launch_umma_items(int bn, const USlab* slabs, const UJob* jobs, const UItem* items, const URed* reds, int nitems,
                        const Bases& b, const UBufs& u, const UPhase& ph, cudaStream_t s);
 // status word of the tcgen05 kernels: 0 = fine, otherwise a bounded wait ran out
 // (the tiles it guarded were not written); reset clears it.  -1 if unreadable.

@@ -414,23 +414,26 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
     if (packs[pi].cls == 2) return xdep[packs[pi].k.src];
     return -1;
   };
-  U->terms.resize(flat_terms.size());
-  for (size_t t = 0; t < flat_terms.size(); ++t) {
-    UTerm u{};
-    u.adep = u.bdep = -1;
-    const int K = (cplx ? 2 : 1) * flat_terms[t].k;
-    if (K > 0) {
+  // slabs of every job's reduction, and where they start
+  std::vector<int> slab0(jobs.size() + 1, 0);
+  for (size_t j = 0; j < jobs.size(); ++j) {
+    slab0[j] = (int)U->slabs.size();
+    for (int t = jobs[j].t0; t < jobs[j].t0 + jobs[j].nt; ++t) {
+      const int K = (cplx ? 2 : 1) * flat_terms[t].k;
+      if (K <= 0) continue;
+      USlab u{};
       u.adep = dep_of(ta[t]);
       u.bdep = dep_of(tb[t]);
-      u.a = packs[ta[t]].dst;
-      u.b = packs[tb[t]].dst;
-      u.abuf = packs[ta[t]].cls ? 1 : 0;
-      u.bbuf = packs[tb[t]].cls ? 1 : 0;
       u.nslab = nslab_of(K);
-      u.klast = K - (u.nslab - 1) * kPanelK;
+      for (int q = 0; q < u.nslab; ++q) {
+        u.a = packs[ta[t]].dst + (long long)q * kUmmaTileM * 256;
+        u.b = packs[tb[t]].dst + (long long)q * BN * 256;
+        u.info = std::min(kPanelK, K - q * kPanelK) + (packs[ta[t]].cls ? 256 : 0) + (packs[tb[t]].cls ? 512 : 0);
+        U->slabs.push_back(u);
+      }
     }
-    U->terms[t] = u;
   }
+  slab0[jobs.size()] = (int)U->slabs.size();
   // jobs: stage-0 results become the A panels their readers use
   std::map<long long, int> xreader;   // stage-0 result offset -> its pack
   for (size_t i = 0; i < packs.size(); ++i)
@@ -453,8 +456,6 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
     u.ldc = xm * J.ldc;
     u.cx = cplx ? 1 : 0;
     u.flags = J.flags;
-    u.t0 = J.t0;
-    u.nt = J.nt;
     u.tag = J.tag;
     u.dep = -1;
     if (J.cbuf == 3) {
@@ -492,8 +493,7 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
     long long total = 0, ntile = 0;
     for (size_t j = 0; j < jobs.size(); ++j) {
       if (job_stage[j] != s) continue;
-      long long ns = 0;
-      for (int t = jobs[j].t0; t < jobs[j].t0 + jobs[j].nt; ++t) ns += U->terms[t].nslab;
+      const long long ns = slab0[j + 1] - slab0[j];
       const long long tiles = (long long)((U->jobs[j].m + kUmmaTileM - 1) / kUmmaTileM) * ((jobs[j].n + BN - 1) / BN);
       ntile += tiles;
       total += tiles * std::max<long long>(ns, 1);
@@ -508,29 +508,23 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
     for (size_t j = 0; j < jobs.size(); ++j) {
       if (job_stage[j] != s) continue;
       const GemmJob& J = jobs[j];
-      long long ns = 0;
-      for (int t = J.t0; t < J.t0 + J.nt; ++t) ns += U->terms[t].nslab;
+      const long long ns = slab0[j + 1] - slab0[j];
       if (ns == 0 && (J.flags & JF_ACCUM)) continue;
       const int tm = (U->jobs[j].m + kUmmaTileM - 1) / kUmmaTileM, tn = (J.n + BN - 1) / BN;
       const long long nch = std::max<long long>(1, (ns + kc - 1) / kc);
       for (int a = 0; a < tm; ++a)
         for (int b = 0; b < tn; ++b) {
+          const int ar = (std::min(kUmmaTileM, U->jobs[j].m - a * kUmmaTileM) + 7) & ~7;
+          const int br = (std::min(BN, J.n - b * BN) + 7) & ~7;
           if (nch == 1) {
-            its.push_back({ns, UItem{(int)j, a, b, J.t0, 0, (int)ns, -1, -1}});
+            its.push_back({ns, UItem{(int)j, a, b, slab0[j], (int)ns, -1, -1, ar, br}});
             continue;
           }
           const int slot0 = nslot, red = (int)U->reds.size();
           long long pos = 0;
-          int t = J.t0, s0 = 0;
           for (long long ch = 0; ch < nch; ++ch) {
             const long long len = std::min(kc, ns - pos);
-            its.push_back({len, UItem{(int)j, a, b, t, s0, (int)len, nslot++, red}});
-            long long left = len;
-            while (left > 0) {
-              const int avail = U->terms[t].nslab - s0;
-              if (left < avail) { s0 += (int)left; left = 0; }
-              else { left -= avail; ++t; s0 = 0; }
-            }
+            its.push_back({len, UItem{(int)j, a, b, slab0[j] + (int)pos, (int)len, nslot++, red, ar, br}});
             pos += len;
           }
           U->reds.push_back(URed{(int)j, a, b, slot0, (int)nch});
@@ -551,10 +545,10 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
   }
   U->nslot = nslot;
 
-  // device copies: [cpack | vpack | terms | jobs | items | reds | cblk | vblk]
+  // device copies: [cpack | vpack | slabs | jobs | items | reds | cblk | vblk]
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t b0 = sizeof(PackJob) * U->cpack.size(), b1 = sizeof(PackJob) * U->vpack.size(),
-               b2 = sizeof(UTerm) * U->terms.size(), b3 = sizeof(UJob) * U->jobs.size(),
+               b2 = sizeof(USlab) * U->slabs.size(), b3 = sizeof(UJob) * U->jobs.size(),
                b4 = sizeof(UItem) * U->items.size(), b5 = sizeof(URed) * U->reds.size(),
                b6 = sizeof(int) * U->cblk.size(), b7 = sizeof(int) * U->vblk.size(),
                b8 = sizeof(int) * U->dep_target.size();
@@ -563,7 +557,7 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
   std::vector<unsigned char> h(total, 0);
   if (b0) std::memcpy(h.data(), U->cpack.data(), b0);
   if (b1) std::memcpy(h.data() + o1, U->vpack.data(), b1);
-  if (b2) std::memcpy(h.data() + o2, U->terms.data(), b2);
+  if (b2) std::memcpy(h.data() + o2, U->slabs.data(), b2);
   if (b3) std::memcpy(h.data() + o3, U->jobs.data(), b3);
   if (b4) std::memcpy(h.data() + o4, U->items.data(), b4);
   if (b5) std::memcpy(h.data() + o5, U->reds.data(), b5);
@@ -575,7 +569,7 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
   unsigned char* base = U->dev->as<unsigned char>();
   const PackJob* d_cpack = reinterpret_cast<PackJob*>(base);
   U->d_vpack = reinterpret_cast<PackJob*>(base + o1);
-  U->d_terms = reinterpret_cast<UTerm*>(base + o2);
+  U->d_slabs = reinterpret_cast<USlab*>(base + o2);
   U->d_jobs = reinterpret_cast<UJob*>(base + o3);
   U->d_items = reinterpret_cast<UItem*>(base + o4);
   U->d_reds = reinterpret_cast<URed*>(base + o5);
@@ -683,7 +677,7 @@ void GemmPlan::run_starved(Ctx& c, bool cplx, const Bases& b, int starve, long l
   ph.wait_ns = wait_ns;
   ph.ctas_per_sm = U.ctas;
   const int ni = U.stage_items[nstage] - U.stage_items[0];
-  launch_umma_items(U.bn, U.d_terms, U.d_jobs, U.d_items, U.d_reds, ni, b, ub, ph, c.stream);
+  launch_umma_items(U.bn, U.d_slabs, U.d_jobs, U.d_items, U.d_reds, ni, b, ub, ph, c.stream);
   ++c.launches;
   SADMRG_CUDA(cudaGetLastError());
   SADMRG_CUDA(cudaStreamSynchronize(c.stream));   // dt must outlive the launch
@@ -724,7 +718,7 @@ void GemmPlan::run(Ctx& c, bool cplx, int prec, const Bases& b, int stage_lo, in
       ph.npk_blocks = (int)U.vblk.size();
       ph.wait_deps = 1;
       const int ni = U.stage_items[nstage] - U.stage_items[0];
-      launch_umma_items(U.bn, U.d_terms, U.d_jobs, U.d_items, U.d_reds, ni, b, ub, ph, c.stream);
+      launch_umma_items(U.bn, U.d_slabs, U.d_jobs, U.d_items, U.d_reds, ni, b, ub, ph, c.stream);
       ++c.launches;
       mark(c, 5);
     } else {
@@ -736,7 +730,7 @@ void GemmPlan::run(Ctx& c, bool cplx, int prec, const Bases& b, int stage_lo, in
       for (int s = stage_lo; s < stage_hi; ++s) {
         const int ni = U.stage_items[s + 1] - U.stage_items[s];
         if (ni > 0) {
-          launch_umma_items(U.bn, U.d_terms, U.d_jobs, U.d_items + U.stage_items[s], U.d_reds, ni, b, ub, ph,
+          launch_umma_items(U.bn, U.d_slabs, U.d_jobs, U.d_items + U.stage_items[s], U.d_reds, ni, b, ub, ph,
                             c.stream);
           ++c.launches;
           mark(c, 1 + 2 * s);

@@ -131,7 +131,7 @@ struct UmmaSchedule {
   std::vector<PackJob> cpack, vpack;       // constant panels (packed once), psi panels (every apply)
   long long cchunks = 0, vchunks = 0;      // multiples of 256 (one block per 256 chunks)
   std::vector<int> cblk, vblk;             // block -> pack job
-  std::vector<UTerm> terms;
+  std::vector<USlab> slabs;
   std::vector<UJob> jobs;
   std::vector<UItem> items;
   std::vector<URed> reds;
@@ -141,7 +141,7 @@ struct UmmaSchedule {
   int* d_dep_target = nullptr;
   PackJob* d_vpack = nullptr;
   int* d_vblk = nullptr;
-  UTerm* d_terms = nullptr;
+  USlab* d_slabs = nullptr;
   UJob* d_jobs = nullptr;
   UItem* d_items = nullptr;
   URed* d_reds = nullptr;

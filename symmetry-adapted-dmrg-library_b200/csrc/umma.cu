@@ -7,14 +7,15 @@
 // intermediate X = op1^T psi directly by the epilogue of the stage that makes
 // it.  The GEMM then does no per-element work in its main loop:
 //
-//   warp 0 (one lane)  producer: per slab, two cp.async.bulk copies (A panel
-//                      128 x 32, B panel BN x 32, hi + lo) into a ring of
-//                      shared-memory stages, completion tracked by the stage's
-//                      mbarrier (expect_tx);
-//   warp 1 (one lane)  issuer: per 8-wide k step three tcgen05.mma (lo*hi,
-//                      hi*lo, hi*hi) into the item's accumulator; tcgen05.commit
-//                      frees the stage, and after the item's last slab signals
-//                      the accumulator full;
+//   warp 0             producer: per slab, two cp.async.bulk copies (of the rows that
+//                      the tile's blocks have, of an A panel 128 x 32 and a B panel
+//                      BN x 32, hi + lo) into a ring of shared-memory stages, completion
+//                      tracked by the stage's mbarrier (expect_tx); a lane per slab, 32
+//                      slabs at a time;
+//   warp 1             issuer: per 8-wide k step three tcgen05.mma (lo*hi, hi*lo, hi*hi),
+//                      as wide as the tile's block, into the item's accumulator;
+//                      tcgen05.commit frees the stage, and after the item's last slab
+//                      signals the accumulator full;
 //   warps 2-5          epilogue: tcgen05.ld of the 128 x BN accumulator (each
 //                      warp its 32 lanes), then FP64 store (optionally adding)
 //                      or hi/lo panels of X; a split-K item writes an FP32
@@ -24,6 +25,16 @@
 // the MMAs of the next; the kernel is persistent (one CTA per SM -- or two,
 // with a 2-stage ring each, at tile width 64 -- static round-robin over the
 // longest-first item list).
+//
+// What bounds it: panels from L2, 8 bytes per element (64 KB a slab of a full tile, 1,000 to
+// 1,170 cycles with all SMs at it; its mma take 800), and where blocks are few the chain of a
+// launch: packing 13 us, the items' slabs, the last sums.  Panels are copied to the rows the
+// block has, the mma issued from uniform registers (550 cycles a slab, from a branch of one
+// lane 950), a slab's entry, dependencies and copies taken by a lane of their own (one lane
+// for all: four loads after one another per slab).  SU(2) ladder centre 97.8 -> 78.8 us,
+// complex U(1) D = 1024 337 -> 300, matvecs back to back.  Tried and no faster: the 128-byte
+// swizzle (panels are then written in scattered pieces), 8 epilogue warps (168 registers), the
+// longest item to the least loaded CTA, 4 groups at a time in the packing.
 //
 // Every mbarrier wait is bounded (time and iterations) and also gives up when
 // another role has failed.  A wait that runs out sets a device status word
@@ -53,10 +64,6 @@ __device__ __forceinline__ void split_hl(double v, uint32_t& hi, uint32_t& lo) {
   hi = tf32_rna(f);
   lo = tf32_rna(f - __uint_as_float(hi));
 }
-__device__ __forceinline__ void split_hl_f(float f, uint32_t& hi, uint32_t& lo) {
-  hi = tf32_rna(f);
-  lo = tf32_rna(f - __uint_as_float(hi));
-}
 
 // shared-memory matrix descriptor: K-major, no swizzle, version 1
 __device__ __forceinline__ uint64_t kmajor_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
@@ -75,6 +82,20 @@ __device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t da, uint64_t
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(da), "l"(db), "r"(idesc), "r"(acc)
       : "memory");
+}
+
+// one k step of 8: low x high, high x low, high x high parts (16-byte units between planes)
+__device__ __forceinline__ void umma_step(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+  umma_tf32(d_tmem, a + 64, b, idesc, acc ? 1u : 0u);
+  umma_tf32(d_tmem, a, b + 64, idesc, 1u);
+  umma_tf32(d_tmem, a, b, idesc, 1u);
+}
+
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -110,6 +131,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 
 __device__ __forceinline__ void st_global_v4(void* p, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   *reinterpret_cast<uint4*>(p) = make_uint4(x, y, z, w);
+}
+
+// Offset in a panel of the 16 bytes of row r, k 4 kg .. 4 kg + 3, high parts: groups of 8
+// rows after one another, in a group the high then the low plane, in a plane the 8 kg.
+constexpr unsigned kRowGroup = 2048, kPlane = 1024;
+__device__ __forceinline__ unsigned panel_off(unsigned r, unsigned kg) {
+  return (r >> 3) * kRowGroup + kg * 128u + (r & 7u) * 16u;
 }
 
 // ---------------------------------------------------------------------------
@@ -171,9 +199,9 @@ __device__ __forceinline__ void pack_chunk(const PackJob& P, unsigned local, con
     }
   }
   unsigned char* panel = dst + P.dst + ((long long)p * nslab + s) * (T * 256u);
-  const unsigned off = (kg * T + rr) * 16u;
-  st_global_v4(panel + off, h[0], h[1], h[2], h[3]);
-  st_global_v4(panel + T * 128u + off, l[0], l[1], l[2], l[3]);
+  unsigned char* o = panel + panel_off(rr, kg);
+  st_global_v4(o, h[0], h[1], h[2], h[3]);
+  st_global_v4(o + kPlane, l[0], l[1], l[2], l[3]);
 }
 
 __global__ void __launch_bounds__(256) pack_kernel(const PackJob* __restrict__ jobs, const int* __restrict__ blk_job,
@@ -201,7 +229,7 @@ struct UG {
 
 template <int BN, int ST, int MINB>
 __global__ void __launch_bounds__(kGThreads, MINB)
-    umma_gemm(const UTerm* __restrict__ terms, const UJob* __restrict__ jobs, const UItem* __restrict__ items,
+    umma_gemm(const USlab* __restrict__ slabs, const UJob* __restrict__ jobs, const UItem* __restrict__ items,
               const URed* __restrict__ reds, int nitems, Bases bases, UBufs ub, UPhase ph) {
   using G = UG<BN, ST>;
   constexpr int BM = kUmmaTileM;
@@ -265,141 +293,167 @@ __global__ void __launch_bounds__(kGThreads, MINB)
 
   if (warp == 0) {
     // ---------------- producer ----------------
-    if (lane == 0) {
-      long long g = 0;
-      uint32_t last_bar = 0, last_par = 0;
-      bool issued_any = false;
-      int ready_term = -1;
-      // bounded wait until dependency counter d reaches its target
-      auto dep_wait = [&](int d) -> bool {
-        if (d < 0) return true;
-        const int target = ub.dep_target[d];
-        const unsigned long long t0 = gtime();
-        for (long long i = 0; i < kWaitIters; ++i) {
-          if (ld_acquire(ub.deps + d) >= target) return true;
-          if ((i & 63) == 63 && (abort_sh || gtime() - t0 > wlim)) return false;
-          __nanosleep(64);
-        }
-        return false;
-      };
-      for (int ii = blockIdx.x; ii < nitems && !abort_sh; ii += gridDim.x) {
-        const UItem it = items[ii];
-        if (ub.mask && !ub.mask[jobs[it.job].tag]) continue;   // instance switched off for this launch
-        int t = it.t0, s = it.s0;
-        for (int q = 0; q < it.nslab; ++q) {
-          while (s >= terms[t].nslab) { ++t; s = 0; }
-          const UTerm T = terms[t];
-          if (ph.wait_deps && t != ready_term) {
-            // the panels this term reads are written in this launch: wait for them
-            if (!dep_wait(T.adep) || !dep_wait(T.bdep)) {
-              if (!abort_sh) atomicExch(&g_umma_status, 9);
-              abort_sh = 1;
+    // Lane q of the warp has slab q of the next 32: it loads the slab's entry, polls its
+    // dependencies and issues its copies in turn.  (One lane that did all this took a chain of
+    // four loads per slab, 1,900 cycles where the mma of a slab take 800.)
+    long long g = 0;
+    bool ok = true;
+    UItem nx{};
+    if ((int)blockIdx.x < nitems) nx = items[blockIdx.x];
+    for (int ii = blockIdx.x; ii < nitems && ok; ii += gridDim.x) {
+      const UItem it = nx;
+      if (ii + (int)gridDim.x < nitems) nx = items[ii + gridDim.x];
+      if (ub.mask && !ub.mask[jobs[it.job].tag]) continue;   // instance switched off for this launch
+      const uint32_t abytes = (uint32_t)it.arows * 256u, bbytes = (uint32_t)it.brows * 256u;
+      for (int q0 = 0; q0 < it.nslab && ok; q0 += 32) {
+        const int n = min(32, it.nslab - q0);
+        const USlab S = slabs[it.q0 + q0 + min(lane, n - 1)];
+        bool ready = !ph.wait_deps || (S.adep < 0 && S.bdep < 0);
+        const int atgt = !ready && S.adep >= 0 ? ub.dep_target[S.adep] : 0;
+        const int btgt = !ready && S.bdep >= 0 ? ub.dep_target[S.bdep] : 0;
+        const unsigned char* A = ((S.info & 256) ? ub.pvar : ub.pconst) + S.a + (long long)it.tm * S.nslab * G::ABYTES;
+        const unsigned char* B = ((S.info & 512) ? ub.pvar : ub.pconst) + S.b + (long long)it.tn * S.nslab * G::BBYTES;
+        for (int q = 0; q < n; ++q) {
+          if (!(__ballot_sync(0xffffffffu, ready) >> q & 1u)) {
+            // the panels this slab reads are written in this launch: bounded wait
+            const unsigned long long t0 = gtime();
+            bool late = true;
+            for (long long i = 0; i < kWaitIters; ++i) {
+              if (!ready) {
+                ready = (S.adep < 0 || ld_acquire(ub.deps + S.adep) >= atgt) &&
+                        (S.bdep < 0 || ld_acquire(ub.deps + S.bdep) >= btgt);
+                if (ready) fence_proxy_async_global();
+              }
+              if (__ballot_sync(0xffffffffu, ready) >> q & 1u) {
+                late = false;
+                break;
+              }
+              const bool stop = (i & 63) == 63 && (abort_sh || gtime() - t0 > wlim);
+              if (__any_sync(0xffffffffu, stop)) break;
+              __nanosleep(64);
+            }
+            if (late) {
+              if (lane == 0) {
+                if (!abort_sh) atomicExch(&g_umma_status, 9);
+                abort_sh = 1;
+              }
+              ok = false;
               break;
             }
-            fence_proxy_async_global();
-            ready_term = t;
           }
           const int st = (int)(g % ST);
-          const uint32_t n = (uint32_t)(g / ST);
-          if (!mbar_wait(saddr(&empty[st]), (n & 1u) ^ 1u, &abort_sh, wlim)) {
-            if (!abort_sh) atomicExch(&g_umma_status, 3);
-            abort_sh = 1;
-            break;
+          bool mine = true;
+          if (lane == q) {
+            mine = mbar_wait(saddr(&empty[st]), ((uint32_t)(g / ST) & 1u) ^ 1u, &abort_sh, wlim);
+            if (mine) {
+              const uint32_t fb = saddr(&full[st]), sa = sbase + (uint32_t)st * G::SBYTES;
+              mbar_expect_tx(fb, abytes + bbytes);
+              bulk_g2s(sa, A, abytes, fb);
+              bulk_g2s(sa + G::ABYTES, B, bbytes, fb);
+            } else {
+              if (!abort_sh) atomicExch(&g_umma_status, 3);
+              abort_sh = 1;
+            }
           }
-          const uint32_t fb = saddr(&full[st]);
-          mbar_expect_tx(fb, G::SBYTES);
-          const unsigned char* A = (T.abuf ? ub.pvar : ub.pconst) + T.a + ((long long)it.tm * T.nslab + s) * G::ABYTES;
-          const unsigned char* B = (T.bbuf ? ub.pvar : ub.pconst) + T.b + ((long long)it.tn * T.nslab + s) * G::BBYTES;
-          const uint32_t sa = sbase + (uint32_t)st * G::SBYTES;
-          bulk_g2s(sa, A, G::ABYTES, fb);
-          bulk_g2s(sa + G::ABYTES, B, G::BBYTES, fb);
-          last_bar = fb;
-          last_par = n & 1u;
-          issued_any = true;
+          ok = __all_sync(0xffffffffu, mine);
+          if (!ok) break;
           ++g;
-          ++s;
         }
       }
-      // every copy this thread issued has landed before the CTA can exit: the last
-      // copy into each stage (bulk copies may complete out of order, and after an
-      // abort the issuer has not consumed them all)
-      (void)last_bar;
-      (void)last_par;
-      if (issued_any)
-        for (long long j = g > ST ? g - ST : 0; j < g; ++j)
-          if (!mbar_wait(saddr(&full[(int)(j % ST)]), (uint32_t)(j / ST) & 1u, nullptr))
-            atomicExch(&g_umma_status, 4);
+      ok = !__any_sync(0xffffffffu, ok && abort_sh) && ok;
+    }
+    if (lane == 0) {
+      // every copy this warp issued has landed before the CTA can exit: the last copy into
+      // each stage (bulk copies may complete out of order, and after an abort the issuer has
+      // not consumed them all)
+      for (long long j = g > ST ? g - ST : 0; j < g; ++j)
+        if (!mbar_wait(saddr(&full[(int)(j % ST)]), (uint32_t)(j / ST) & 1u, nullptr))
+          atomicExch(&g_umma_status, 4);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = tf32_idesc(BM, BN);
-      long long g = 0;
-      int il = 0;
-      uint32_t last_bar = 0, last_par = 0;
-      bool committed = false;
-      for (int ii = blockIdx.x; ii < nitems && !abort_sh; ii += gridDim.x) {
-        const UItem it = items[ii];
-        if (ub.mask && !ub.mask[jobs[it.job].tag]) continue;
-        const int acc = il & 1;
-        if (!mbar_wait(saddr(&tempty[acc]), (((uint32_t)il >> 1) & 1u) ^ 1u, &abort_sh, wlim)) {
-          if (!abort_sh) atomicExch(&g_umma_status, 5);
+    // The whole warp runs the loop and one elected lane issues, so that the descriptors stay
+    // in uniform registers: issued from a branch of one lane an mma took 79 cycles at any
+    // width, more than its work.  The next item, its first slab's k and the next slab's k are
+    // loaded ahead.
+    long long g = 0;
+    int il = 0;
+    uint32_t last_bar = 0, last_par = 0;
+    bool committed = false, ok = true;
+    const bool leader = elect_one();
+    UItem nx{};
+    int kn = 0;                                            // info of the next slab
+    if ((int)blockIdx.x < nitems) {
+      nx = items[blockIdx.x];
+      if (nx.nslab > 0) kn = slabs[nx.q0].info;
+    }
+    for (int ii = blockIdx.x; ii < nitems && ok; ii += gridDim.x) {
+      const UItem it = nx;
+      if (ii + (int)gridDim.x < nitems) nx = items[ii + gridDim.x];
+      const bool on = !ub.mask || ub.mask[jobs[it.job].tag];
+      if (!on) {
+        if (nx.nslab > 0) kn = slabs[nx.q0].info;
+        continue;
+      }
+      const int acc = il & 1;
+      const uint32_t idesc = tf32_idesc(BM, (it.brows + 15) & ~15);
+      const uint32_t d = tmem + (uint32_t)(acc * BN);
+      ok = __all_sync(0xffffffffu, mbar_wait(saddr(&tempty[acc]), (((uint32_t)il >> 1) & 1u) ^ 1u, &abort_sh, wlim));
+      if (!ok) {
+        if (leader && !abort_sh) atomicExch(&g_umma_status, 5);
+        abort_sh = 1;
+        break;
+      }
+      fence_after();
+      for (int q = 0; q < it.nslab; ++q) {
+        const int kt = kn & 255;
+        if (q + 1 < it.nslab) kn = slabs[it.q0 + q + 1].info;
+        else if (nx.nslab > 0) kn = slabs[nx.q0].info;
+        const int st = (int)(g % ST);
+        const uint32_t n = (uint32_t)(g / ST);
+        ok = __all_sync(0xffffffffu, mbar_wait(saddr(&full[st]), n & 1u, &abort_sh, wlim));
+        if (!ok) {
+          if (leader && !abort_sh) atomicExch(&g_umma_status, 6);
           abort_sh = 1;
           break;
         }
         fence_after();
-        const uint32_t d = tmem + (uint32_t)(acc * BN);
-        int t = it.t0, s = it.s0;
-        bool ok = true;
-        for (int q = 0; q < it.nslab; ++q) {
-          while (s >= terms[t].nslab) { ++t; s = 0; }
-          const UTerm T = terms[t];
-          const int kt = (s == T.nslab - 1) ? T.klast : kPanelK;
-          const int st = (int)(g % ST);
-          const uint32_t n = (uint32_t)(g / ST);
-          if (!mbar_wait(saddr(&full[st]), n & 1u, &abort_sh, wlim)) {
-            if (!abort_sh) atomicExch(&g_umma_status, 6);
-            abort_sh = 1;
-            ok = false;
-            break;
-          }
-          fence_after();
-          const uint32_t a0 = sbase + (uint32_t)st * G::SBYTES, b0 = a0 + G::ABYTES;
-          const int nks = (kt + 7) >> 3;
-          for (int ks = 0; ks < nks; ++ks) {
-            const uint32_t ao = (uint32_t)ks * 2u * BM * 16u, bo = (uint32_t)ks * 2u * BN * 16u;
-            const uint64_t ah = kmajor_desc(a0 + ao, BM * 16, 128);
-            const uint64_t al = kmajor_desc(a0 + BM * 128 + ao, BM * 16, 128);
-            const uint64_t bh = kmajor_desc(b0 + bo, BN * 16, 128);
-            const uint64_t bl = kmajor_desc(b0 + BN * 128 + bo, BN * 16, 128);
-            umma_tf32(d, al, bh, idesc, (q > 0 || ks > 0) ? 1u : 0u);
-            umma_tf32(d, ah, bl, idesc, 1u);
-            umma_tf32(d, ah, bh, idesc, 1u);
+        const uint32_t a0 = sbase + (uint32_t)st * G::SBYTES;
+        const uint64_t da = kmajor_desc(a0, 128, kRowGroup), db = kmajor_desc(a0 + G::ABYTES, 128, kRowGroup);
+        if (leader) {
+          if (kt > 24) {
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) umma_step(d, da + ks * 16, db + ks * 16, idesc, ks > 0 || q > 0);
+          } else {
+            for (int ks = 0; ks < (kt + 7) >> 3; ++ks) umma_step(d, da + ks * 16, db + ks * 16, idesc, ks > 0 || q > 0);
           }
           umma_commit(saddr(&empty[st]));
-          last_bar = saddr(&empty[st]);
-          last_par = n & 1u;
-          committed = true;
-          ++g;
-          ++s;
         }
-        if (!ok) break;
-        umma_commit(saddr(&tfull[acc]));
-        last_bar = saddr(&tfull[acc]);
-        last_par = ((uint32_t)il >> 1) & 1u;
+        __syncwarp();
+        last_bar = saddr(&empty[st]);
+        last_par = n & 1u;
         committed = true;
-        ++il;
+        ++g;
       }
-      // every MMA this thread issued has finished before tensor memory is freed
-      if (committed && !mbar_wait(last_bar, last_par, nullptr)) atomicExch(&g_umma_status, 7);
+      if (!ok) break;
+      if (it.nslab == 0 && nx.nslab > 0) kn = slabs[nx.q0].info;
+      if (leader) umma_commit(saddr(&tfull[acc]));
+      __syncwarp();
+      last_bar = saddr(&tfull[acc]);
+      last_par = ((uint32_t)il >> 1) & 1u;
+      committed = true;
+      ++il;
+      ok = !__any_sync(0xffffffffu, abort_sh != 0);
     }
+    // every MMA this warp issued has finished before tensor memory is freed
+    if (committed && !mbar_wait(last_bar, last_par, nullptr)) atomicExch(&g_umma_status, 7);
   } else {
     // ---------------- epilogue: warps 2..5 ----------------
     const int quarter = warp & 3;           // TMEM lanes 32*quarter .. +31
     const int r = 32 * quarter + lane;      // tile row
     int il = 0;
-    const int et = tid - 64;                // 0..127 within the epilogue warps
-    // The four epilogue warps take every decision together: a failed wait is
+    const int et = tid - 64;                // within the epilogue warps
+    // The epilogue warps take every decision together: a failed wait is
     // posted to ep_fail and read by all after the same named barrier (id 1).
     for (int ii = blockIdx.x; ii < nitems; ii += gridDim.x) {
       const UItem it = items[ii];
@@ -416,7 +470,13 @@ __global__ void __launch_bounds__(kGThreads, MINB)
       fence_after();
       const int row0 = it.tm * BM, col0 = it.tn * BN;
       // 32 columns [cb, cb + 32) of row r of the finished tile -> C, or -> A panels of X
-      auto emit = [&](int cb, const double (&x)[32]) {
+      // (columns past the block hold whatever was there: zeros in the panels, where they are
+      // the padding of the reduction)
+      const int ncol = min(BN, J.n - col0);
+      auto emit = [&](int cb, double (&x)[32]) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (cb + j >= ncol) x[j] = 0.0;
         if (J.pack >= 0 && J.cx) {
           // real form Xh of the complex result: this thread holds Re (r even) or Im (r odd)
           // of row r/2, its lane neighbour the other part; columns [cb, cb + 32) feed
@@ -427,36 +487,40 @@ __global__ void __launch_bounds__(kGThreads, MINB)
           for (int hs = 0; hs < 2; ++hs) {
             const int s = s0 + hs;
             unsigned char* panel = ub.pvar + J.pack + ((long long)it.tm * J.pack_nslab + s) * (BM * 256);
-            const bool live = s < J.pack_nslab;   // the same for every lane
+            const bool live = s < J.pack_nslab && r < it.arows;
 #pragma unroll
             for (int kg = 0; kg < 8; ++kg) {
               uint32_t h[4], l[4];
 #pragma unroll
               for (int w = 0; w < 2; ++w) {
-                const int j = 16 * hs + 2 * kg + w;
-                const double own = x[j];
-                const double nb = __shfl_xor_sync(0xffffffffu, own, 1);
-                const double v0 = own, v1 = odd ? nb : -nb;   // (Re, -Im) on row 2i, (Im, Re) on 2i + 1
-                split_hl(J.alpha * v0, h[2 * w], l[2 * w]);
-                split_hl(J.alpha * v1, h[2 * w + 1], l[2 * w + 1]);
+                // (Re, -Im) on row 2i, (Im, Re) on 2i + 1; a split changes sign with its number
+                uint32_t oh, ol;
+                split_hl(J.alpha * x[16 * hs + 2 * kg + w], oh, ol);
+                const uint32_t sign = odd ? 0u : 0x80000000u;
+                h[2 * w] = oh;
+                l[2 * w] = ol;
+                h[2 * w + 1] = __shfl_xor_sync(0xffffffffu, oh, 1) ^ sign;
+                l[2 * w + 1] = __shfl_xor_sync(0xffffffffu, ol, 1) ^ sign;
               }
               if (live) {
-                st_global_v4(panel + (kg * BM + r) * 16, h[0], h[1], h[2], h[3]);
-                st_global_v4(panel + BM * 128 + (kg * BM + r) * 16, l[0], l[1], l[2], l[3]);
+                unsigned char* o = panel + panel_off(r, kg);
+                st_global_v4(o, h[0], h[1], h[2], h[3]);
+                st_global_v4(o + kPlane, l[0], l[1], l[2], l[3]);
               }
             }
           }
         } else if (J.pack >= 0) {
           const int s = (col0 + cb) / kPanelK;
-          if (s < J.pack_nslab) {
+          if (s < J.pack_nslab && r < it.arows) {
             unsigned char* panel = ub.pvar + J.pack + ((long long)it.tm * J.pack_nslab + s) * (BM * 256);
 #pragma unroll
             for (int kg = 0; kg < 8; ++kg) {
               uint32_t h[4], l[4];
 #pragma unroll
               for (int u = 0; u < 4; ++u) split_hl(J.alpha * x[4 * kg + u], h[u], l[u]);
-              st_global_v4(panel + (kg * BM + r) * 16, h[0], h[1], h[2], h[3]);
-              st_global_v4(panel + BM * 128 + (kg * BM + r) * 16, l[0], l[1], l[2], l[3]);
+              unsigned char* o = panel + panel_off(r, kg);
+              st_global_v4(o, h[0], h[1], h[2], h[3]);
+              st_global_v4(o + kPlane, l[0], l[1], l[2], l[3]);
             }
           }
         } else if (row0 + r < J.m) {
@@ -473,7 +537,7 @@ __global__ void __launch_bounds__(kGThreads, MINB)
         }
       };
 #pragma unroll 1
-      for (int cb = 0; cb < BN; cb += 32) {
+      for (int cb = 0; cb < ncol; cb += 32) {
         uint32_t v[32];
         if (it.nslab > 0) {
           tmem_ld32(tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(acc * BN + cb), v);
@@ -482,9 +546,10 @@ __global__ void __launch_bounds__(kGThreads, MINB)
           for (int j = 0; j < 32; ++j) v[j] = 0u;
         }
         if (it.slot >= 0) {
-          float* S = ub.slots + (long long)it.slot * BM * BN;
+          // partial tile: four columns of a row together, rows next to one another
+          uint4* S = reinterpret_cast<uint4*>(ub.slots + (long long)it.slot * BM * BN) + (cb / 4) * BM + r;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) S[r + (cb + j) * BM] = __uint_as_float(v[j]);
+          for (int j = 0; j < 8; ++j) S[j * BM] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         } else {
           double x[32];
 #pragma unroll
@@ -514,14 +579,31 @@ __global__ void __launch_bounds__(kGThreads, MINB)
         if (last_sh) {
           __threadfence();
 #pragma unroll 1
-          for (int cb = 0; cb < BN; cb += 32) {
+          for (int cb = 0; cb < ncol; cb += 32) {
             double x[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) x[j] = 0.0;
-            for (int k = 0; k < R.nslot; ++k) {
-              const float* S = ub.slots + (long long)(R.slot0 + k) * BM * BN;
+            // (kSl slots' loads in flight: one slot at a time, 4 bytes a load, the sum of ten
+            // slots took 32,000 cycles, longer than the mma of 29 slabs)
+            constexpr int kSl = MINB == 1 ? 3 : 1;
+            const float4* S = reinterpret_cast<const float4*>(ub.slots + (long long)R.slot0 * BM * BN) + (cb / 4) * BM + r;
+            for (int k0 = 0; k0 < R.nslot; k0 += kSl) {
+              float4 w[kSl][8];
 #pragma unroll
-              for (int j = 0; j < 32; ++j) x[j] += (double)__ldcg(S + r + (cb + j) * BM);
+              for (int u = 0; u < kSl; ++u)
+                if (k0 + u < R.nslot)
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) w[u][j] = __ldcg(S + (long long)(k0 + u) * (BM * BN / 4) + j * BM);
+#pragma unroll
+              for (int u = 0; u < kSl; ++u)
+                if (k0 + u < R.nslot)
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) {
+                    x[4 * j] += (double)w[u][j].x;
+                    x[4 * j + 1] += (double)w[u][j].y;
+                    x[4 * j + 2] += (double)w[u][j].z;
+                    x[4 * j + 3] += (double)w[u][j].w;
+                  }
             }
             emit(cb, x);
           }
@@ -554,7 +636,7 @@ __global__ void __launch_bounds__(kGThreads, MINB)
 }
 
 template <int BN, int ST, int MINB>
-void launch_gemm_t(const UTerm* terms, const UJob* jobs, const UItem* items, const URed* reds, int nitems,
+void launch_gemm_t(const USlab* slabs, const UJob* jobs, const UItem* items, const URed* reds, int nitems,
                    const Bases& b, const UBufs& u, const UPhase& ph, cudaStream_t s) {
   static unsigned char attr[kMaxDevices] = {0};
   static int occ[kMaxDevices] = {0};   // resident CTAs per SM the device grants this kernel
@@ -580,12 +662,12 @@ void launch_gemm_t(const UTerm* terms, const UJob* jobs, const UItem* items, con
     UBufs uu = u;
     UPhase pp = ph;
     int ni = nitems;
-    void* args[] = {(void*)&terms, (void*)&jobs, (void*)&items, (void*)&reds, (void*)&ni, (void*)&bb, (void*)&uu,
+    void* args[] = {(void*)&slabs, (void*)&jobs, (void*)&items, (void*)&reds, (void*)&ni, (void*)&bb, (void*)&uu,
                     (void*)&pp};
     cudaLaunchCooperativeKernel((const void*)umma_gemm<BN, ST, MINB>, dim3(grid), dim3(kGThreads), args,
                                 UG<BN, ST>::SMEM, s);
   } else {
-    umma_gemm<BN, ST, MINB><<<grid, kGThreads, UG<BN, ST>::SMEM, s>>>(terms, jobs, items, reds, nitems, b, u, ph);
+    umma_gemm<BN, ST, MINB><<<grid, kGThreads, UG<BN, ST>::SMEM, s>>>(slabs, jobs, items, reds, nitems, b, u, ph);
   }
 }
 
@@ -622,12 +704,12 @@ void launch_pack(const PackJob* jobs, const int* blk_job, int nblocks, const Bas
   pack_kernel<<<nblocks, 256, 0, s>>>(jobs, blk_job, b, dst);
 }
 
-void launch_umma_items(int bn, const UTerm* terms, const UJob* jobs, const UItem* items, const URed* reds, int nitems,
+void launch_umma_items(int bn, const USlab* slabs, const UJob* jobs, const UItem* items, const URed* reds, int nitems,
                        const Bases& b, const UBufs& u, const UPhase& ph, cudaStream_t s) {
   if (nitems <= 0 && ph.npk_blocks <= 0) return;
-  if (bn == 128) launch_gemm_t<128, 3, 1>(terms, jobs, items, reds, nitems, b, u, ph, s);
-  else if (ph.ctas_per_sm == 2) launch_gemm_t<64, 2, 2>(terms, jobs, items, reds, nitems, b, u, ph, s);
-  else launch_gemm_t<64, 4, 1>(terms, jobs, items, reds, nitems, b, u, ph, s);
+  if (bn == 128) launch_gemm_t<128, 3, 1>(slabs, jobs, items, reds, nitems, b, u, ph, s);
+  else if (ph.ctas_per_sm == 2) launch_gemm_t<64, 2, 2>(slabs, jobs, items, reds, nitems, b, u, ph, s);
+  else launch_gemm_t<64, 4, 1>(slabs, jobs, items, reds, nitems, b, u, ph, s);
 }
 
 int umma_status(bool reset) {
