@@ -722,7 +722,7 @@ __device__ __forceinline__ void jacobi_pair_visit(typename SvdT<CPLX>::T* W, int
 constexpr unsigned long long kSvdBarrierNs = 2000000000ull;
 
 struct SvdCtl {
-  unsigned count, gen;
+  unsigned count;             // of the QR kernels' barrier
   int status;                 // 0, or 1 when a barrier ran out of time
   int sweeps, failed;         // sweeps taken; 1 when max_sweeps was reached
   unsigned long long t0, t1;  // device clock (ns) at the start and end of block 0
@@ -734,36 +734,8 @@ __device__ __forceinline__ unsigned long long svd_gtime() {
   return t;
 }
 
-__device__ bool svd_grid_sync(SvdCtl* ctl) {
-  __shared__ int ok_sh;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok_sh = 1;
-    volatile unsigned* gen = &ctl->gen;
-    const unsigned g = *gen;
-    __threadfence();
-    if (atomicAdd(&ctl->count, 1u) == gridDim.x - 1) {
-      atomicExch(&ctl->count, 0u);
-      __threadfence();
-      atomicAdd(&ctl->gen, 1u);
-    } else {
-      const unsigned long long t0 = svd_gtime();
-      for (long long it = 0; *gen == g; ++it) {
-        if (it > (1ll << 30) || ((it & 255) == 255 && svd_gtime() - t0 > kSvdBarrierNs)) {
-          ok_sh = 0;
-          atomicExch(&ctl->status, 1);
-          break;
-        }
-        __nanosleep(32);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return ok_sh != 0;
-}
-
-// Barrier of the CTAs that share a sector: *count grows by one per CTA and phase.
+// Barrier of `size` CTAs (those that share a sector, or all): *count grows by one per CTA
+// and phase.
 // Returns false when it ran out of time.
 __device__ bool svd_group_sync(unsigned* count, int size, unsigned& phase, SvdCtl* ctl) {
   __shared__ int ok_sh;
@@ -937,7 +909,7 @@ __global__ void jacobi_norms_kernel(const SvdJob* jobs, const void* work, double
   const int R = J.trans ? J.n : J.m, C = J.trans ? J.m : J.n;
   const T* W = static_cast<const T*>(work) + J.woff;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int c = warp; c < C; c += nw) {
+  for (int c = blockIdx.y * nw + warp; c < C; c += gridDim.y * nw) {
     double s = 0.0;
     for (int r = lane; r < R; r += 32) {
       if (CPLX) { const double2 v = reinterpret_cast<const double2*>(W)[r + (long long)c * R]; s += v.x * v.x + v.y * v.y; }
@@ -1010,30 +982,38 @@ __device__ __forceinline__ T op_a(const T* A, int m, int trans, int r, int c) {
   return trans ? cconj(A[c + (long long)r * m]) : A[r + (long long)c * m];
 }
 
-// Column norms of op(A) and their order (decreasing, ties by index): P.
+// Column norms of op(A).  (One block per sector for these, the order and jacobi_norms took
+// 1.8 ms at D = 2048: 7 of 148 SMs.)
 template <bool CPLX>
-__global__ void qr_order_kernel(const QrJob* jobs, const void* a, double* nrm, int* perm) {
+__global__ void qr_norms_kernel(const QrJob* jobs, const void* a, double* nrm) {
   chain_begin();
   using T = typename SvdT<CPLX>::T;
   const QrJob J = jobs[blockIdx.x];
   const T* A = static_cast<const T*>(a) + J.aoff;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double* nj = nrm + J.soff;
-  for (int c = warp; c < J.C; c += nw) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int c = blockIdx.y * nw + (threadIdx.x >> 5); c < J.C; c += gridDim.y * nw) {
     double s = 0.0;
     for (int r = lane; r < J.R; r += 32) s += cabs2(op_a(A, J.m, J.trans, r, c));
     s = wsum(s);
-    if (lane == 0) nj[c] = s;
+    if (lane == 0) nrm[J.soff + c] = s;
   }
-  __syncthreads();
-  for (int c = threadIdx.x; c < J.C; c += blockDim.x) {
-    const double v = nj[c];
+}
+// Their order (decreasing, ties by index): P; a warp counts a column's rank.
+template <bool CPLX>
+__global__ void qr_order_kernel(const QrJob* jobs, const double* nrm, int* perm) {
+  chain_begin();
+  const QrJob J = jobs[blockIdx.x];
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const double* nj = nrm + J.soff;
+  for (int c = blockIdx.y * nw + (threadIdx.x >> 5); c < J.C; c += gridDim.y * nw) {
+    const double v = fmax(nj[c], -1.0);   // (a NaN counts as -1: a permutation whatever the input)
     int rank = 0;
-    for (int k = 0; k < J.C; ++k) {
-      const double u = nj[k];
+    for (int k = lane; k < J.C; k += 32) {
+      const double u = fmax(nj[k], -1.0);
       rank += (u > v || (u == v && k < c)) ? 1 : 0;
     }
-    perm[J.soff + rank] = c;
+    rank = __reduce_add_sync(0xffffffffu, rank);
+    if (lane == 0) perm[J.soff + rank] = c;
   }
 }
 
@@ -1248,16 +1228,17 @@ __global__ void __launch_bounds__(kSvdThreads) qr_coop_kernel(const QrJob* __res
                                                               const QrTile* __restrict__ tiles, const int* __restrict__ toff,
                                                               int steps, void* qbuf, SvdCtl* ctl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned phase = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->t0 = svd_gtime();
   for (int k = 0; k < steps; ++k) {
     for (int p = poff[k] + blockIdx.x; p < poff[k + 1]; p += gridDim.x) qr_panel<CPLX>(jobs[panels[p]], k, qbuf, smem_raw);
-    if (!svd_grid_sync(ctl)) return;
+    if (!svd_group_sync(&ctl->count, gridDim.x, phase, ctl)) return;
     for (int t = toff[k] + blockIdx.x; t < toff[k + 1]; t += gridDim.x) {
       const QrTile tl = tiles[t];
       const QrJob& J = jobs[tl.job];
       qr_apply_tile<CPLX>(J, k, tl.c1, J.C, 1, qbuf, qbuf, J.qoff, smem_raw);
     }
-    if (!svd_grid_sync(ctl)) return;
+    if (!svd_group_sync(&ctl->count, gridDim.x, phase, ctl)) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->t1 = svd_gtime();
 }
@@ -1269,6 +1250,7 @@ __global__ void __launch_bounds__(kSvdThreads) qr_unmq_kernel(const QrJob* __res
                                                               const QrTile* __restrict__ tiles, const int* __restrict__ toff,
                                                               int steps, void* qbuf, void* out, SvdCtl* ctl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned phase = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->t0 = svd_gtime();
   for (int k = steps - 1; k >= 0; --k) {
     for (int t = toff[k] + blockIdx.x; t < toff[k + 1]; t += gridDim.x) {
@@ -1276,7 +1258,7 @@ __global__ void __launch_bounds__(kSvdThreads) qr_unmq_kernel(const QrJob* __res
       const QrJob& J = jobs[tl.job];
       qr_apply_tile<CPLX>(J, k, tl.c1, J.C, 0, qbuf, J.x_in_q ? qbuf : out, J.woff, smem_raw);
     }
-    if (k > 0 && !svd_grid_sync(ctl)) return;
+    if (k > 0 && !svd_group_sync(&ctl->count, gridDim.x, phase, ctl)) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->t1 = svd_gtime();
 }
@@ -1457,7 +1439,7 @@ static int jacobi_run(const void* a, void* work, void* vmat, double* sv, const s
   SADMRG_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)ctas.size()), dim3(kSvdThreads), args, smem, s));
   SvdCtl hctl{};
   SADMRG_CUDA(cudaMemcpyAsync(&hctl, pctl, sizeof(SvdCtl), cudaMemcpyDeviceToHost, s));
-  launch_chained(jacobi_norms_kernel<CPLX>, nj, 256, 0, s, pj, work, sv);
+  launch_chained(jacobi_norms_kernel<CPLX>, dim3(nj, 16), 256, 0, s, pj, work, sv);
   SADMRG_CUDA(cudaGetLastError());
   SADMRG_CUDA(cudaStreamSynchronize(s));
   SADMRG_REQUIRE(hctl.status == 0, SADMRG_ERR_CUDA, "jacobi svd: a barrier ran out of time");
@@ -1608,7 +1590,8 @@ static int qr_jacobi_run(const void* a, void* work, void* vmat, double* sv, cons
   // P and W0 = op(A) P need the job array on the device: the first QR's copy
   L1.dj.alloc(sizeof(QrJob) * nj, s);
   SADMRG_CUDA(cudaMemcpyAsync(L1.dj.get(), q1.data(), sizeof(QrJob) * nj, cudaMemcpyHostToDevice, s));
-  launch_chained(qr_order_kernel<CPLX>, nj, kSvdThreads, 0, s, static_cast<const QrJob*>(L1.dj.get()), a, sv, dperm.as<int>());
+  launch_chained(qr_norms_kernel<CPLX>, dim3(nj, 32), 256, 0, s, static_cast<const QrJob*>(L1.dj.get()), a, sv);
+  launch_chained(qr_order_kernel<CPLX>, dim3(nj, 32), 256, 0, s, static_cast<const QrJob*>(L1.dj.get()), (const double*)sv, dperm.as<int>());
   launch_chained(qr_gather_kernel<CPLX>, dim3(nj, 32), 256, 0, s, static_cast<const QrJob*>(L1.dj.get()), a, qbuf.get(), dperm.as<int>());
   SADMRG_CUDA(cudaGetLastError());
   if (!L1.run(q1, false, qbuf.get(), work, ctl, s)) {
