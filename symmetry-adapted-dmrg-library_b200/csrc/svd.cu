@@ -1039,6 +1039,11 @@ __global__ void qr_gather_kernel(const QrJob* jobs, const void* a, void* qbuf, c
 // when the column below the diagonal is zero and alpha is real), each applied as
 // H^H to the panel's later columns; then T of the compact WY form (forward,
 // columnwise).  Writes R's panel rows, the reflectors and T back.
+// The panel is what bounds a step: a chain of columns (norm, scale, dots, update) in one
+// CTA while the other SMs wait.  Cycles of a panel of 172 x 16 on average (D = 512): load
+// 1,900, columns 33,400, S 5,200, T 3,200, after 67,800 with one element in flight per lane, a
+// dot at a time and T's sums through shared memory; a QR of D = 512 blocks 1.18 -> 0.83 ms, of
+// D = 2048 10.1 -> 7.1.  The order of every sum is as it was (see jacobi_pair_visit on signs).
 template <bool CPLX>
 __device__ void qr_panel(const QrJob& J, int k, void* qbuf, unsigned char* smem) {
   using T = typename SvdT<CPLX>::T;
@@ -1049,16 +1054,35 @@ __device__ void qr_panel(const QrJob& J, int k, void* qbuf, unsigned char* smem)
   __shared__ T tau_sh[NB];
   __shared__ T S_sh[NB * NB];          // S(k, j) = v_k^H v_j, k < j
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < nr * w; e += blockDim.x) {
-    const int i = e % nr, l = e / nr;
-    P[e] = A[(r0 + i) + (long long)(r0 + l) * J.R];
+  // kU elements of a column from i on, every 32nd (zeros past the rows): read together, as a
+  // column is a chain of four passes over it and each element's latency would add to it (one
+  // element at a time a column of 172 rows took 4,200 cycles)
+  constexpr int kU = CPLX ? 4 : 8;
+  auto take = [&](const T* x, int i, T (&a)[kU]) {
+#pragma unroll
+    for (int u = 0; u < kU; ++u) a[u] = i + 32 * u < nr ? x[i + 32 * u] : czero<T>();
+  };
+  for (int l = warp; l < w; l += kSvdWarps) {
+    const T* src = A + r0 + (long long)(r0 + l) * J.R;
+    for (int i = lane; i < nr; i += 32 * kU) {
+      T a[kU];
+      take(src, i, a);
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (i + 32 * u < nr) P[l * nr + i + 32 * u] = a[u];
+    }
   }
   __syncthreads();
   for (int j = 0; j < w; ++j) {
     T* x = P + (long long)j * nr;
     if (warp == 0) {
       double s2 = 0.0;
-      for (int i = j + 1 + lane; i < nr; i += 32) s2 += cabs2(x[i]);
+      for (int i = j + 1 + lane; i < nr; i += 32 * kU) {
+        T a[kU];
+        take(x, i, a);
+#pragma unroll
+        for (int u = 0; u < kU; ++u) s2 += cabs2(a[u]);
+      }
       s2 = wsum(s2);
       const T alpha = x[j];
       T tau = czero<T>();
@@ -1075,7 +1099,13 @@ __device__ void qr_panel(const QrJob& J, int k, void* qbuf, unsigned char* smem)
         } else {
           scale = 1.0 / (alpha - beta);
         }
-        for (int i = j + 1 + lane; i < nr; i += 32) x[i] = cmul(x[i], scale);
+        for (int i = j + 1 + lane; i < nr; i += 32 * kU) {
+          T a[kU];
+          take(x, i, a);
+#pragma unroll
+          for (int u = 0; u < kU; ++u)
+            if (i + 32 * u < nr) x[i + 32 * u] = cmul(a[u], scale);
+        }
       }
       __syncwarp();
       if (lane == 0) {
@@ -1088,49 +1118,79 @@ __device__ void qr_panel(const QrJob& J, int k, void* qbuf, unsigned char* smem)
     if (warp < w - 1 - j && cabs2(tau) != 0.0) {
       T* y = P + (long long)(j + 1 + warp) * nr;
       T d = lane == 0 ? y[j] : czero<T>();   // v_j = 1
-      for (int i = j + 1 + lane; i < nr; i += 32) d = cadd(d, cj_mul(x[i], y[i]));
+      for (int i = j + 1 + lane; i < nr; i += 32 * kU) {
+        T a[kU], b[kU];
+        take(x, i, a);
+        take(y, i, b);
+#pragma unroll
+        for (int u = 0; u < kU; ++u) d = cadd(d, cj_mul(a[u], b[u]));
+      }
       d = wsum_t(d);
       const T f = cmul(cconj(tau), d);
       if (lane == 0) y[j] = csub(y[j], f);
-      for (int i = j + 1 + lane; i < nr; i += 32) y[i] = csub(y[i], cmul(x[i], f));
+      for (int i = j + 1 + lane; i < nr; i += 32 * kU) {
+        T a[kU], b[kU];
+        take(x, i, a);
+        take(y, i, b);
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+          if (i + 32 * u < nr) y[i + 32 * u] = csub(b[u], cmul(a[u], f));
+      }
     }
     __syncthreads();
   }
-  // S(q, j) = v_q^H v_j for q < j (rows j .. nr-1; v_j(j) = 1, v_q(j) = P(j, q))
-  for (int pr = warp; pr < w * w; pr += kSvdWarps) {
-    const int q = pr / w, j = pr % w;
-    if (q >= j) continue;
-    const T* vq = P + (long long)q * nr;
-    const T* vj = P + (long long)j * nr;
-    T d = lane == 0 ? cconj(vq[j]) : czero<T>();
-    for (int i = j + 1 + lane; i < nr; i += 32) d = cadd(d, cj_mul(vq[i], vj[i]));
-    d = wsum_t(d);
-    if (lane == 0) S_sh[q + j * NB] = d;
-  }
+  // S(q, j) = v_q^H v_j for q < j (rows j .. nr-1; v_j(j) = 1, v_q(j) = P(j, q)); a warp
+  // takes a j, kQ of its sums side by side
+  constexpr int kQ = CPLX ? 2 : 4;
+  for (int j = warp; j < w; j += kSvdWarps)
+    for (int q0 = 0; q0 < j; q0 += kQ) {
+      const T* vj = P + (long long)j * nr;
+      T d[kQ];
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) d[q] = lane == 0 ? cconj(P[(long long)min(q0 + q, j - 1) * nr + j]) : czero<T>();
+      for (int i = j + 1 + lane; i < nr; i += 32 * kU) {
+        T b[kU];
+        take(vj, i, b);
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+          T a[kU];
+          take(P + (long long)min(q0 + q, j - 1) * nr, i, a);
+#pragma unroll
+          for (int u = 0; u < kU; ++u) d[q] = cadd(d[q], cj_mul(a[u], b[u]));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) d[q] = wsum_t(d[q]);
+#pragma unroll
+      for (int q = 0; q < kQ; ++q)
+        if (lane == 0 && q0 + q < j) S_sh[q0 + q + j * NB] = d[q];
+    }
   __syncthreads();
   // T: T(j, j) = tau_j, T(0:j, j) = -tau_j T(0:j, 0:j) S(0:j, j)
   T* Tm = static_cast<T*>(qbuf) + J.toff + (long long)k * NB * NB;
   if (warp == 0) {
-    __shared__ T T_sh[NB * NB];
-    for (int e = lane; e < NB * NB; e += 32) T_sh[e] = czero<T>();
-    __syncwarp();
-    for (int j = 0; j < w; ++j) {
-      const T tj = tau_sh[j];
-      T v = czero<T>();
-      if (lane < j) {
-        for (int q = lane; q < j; ++q) v = cadd(v, cmul(T_sh[lane + q * NB], S_sh[q + j * NB]));
-        v = cmul(cscale(tj, -1.0), v);
+    T row[NB];                           // lane's row of T
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      row[j] = czero<T>();
+      if (j < w) {
+        const T tj = tau_sh[j];
+        T v = czero<T>();
+#pragma unroll
+        for (int q = 0; q < j; ++q)
+          if (q >= lane) v = cadd(v, cmul(row[q], S_sh[q + j * NB]));
+        if (lane < j) row[j] = cmul(cscale(tj, -1.0), v);
+        if (lane == j) row[j] = tj;
       }
-      __syncwarp();
-      if (lane < j) T_sh[lane + j * NB] = v;
-      if (lane == j) T_sh[j + j * NB] = tj;
-      __syncwarp();
     }
-    for (int e = lane; e < NB * NB; e += 32) Tm[e] = T_sh[e];
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (lane < NB) Tm[lane + j * NB] = row[j];
   }
-  for (int e = tid; e < nr * w; e += blockDim.x) {
-    const int i = e % nr, l = e / nr;
-    A[(r0 + i) + (long long)(r0 + l) * J.R] = P[e];
+  for (int l = warp; l < w; l += kSvdWarps) {
+    T* dst = A + r0 + (long long)(r0 + l) * J.R;
+#pragma unroll 4
+    for (int i = lane; i < nr; i += 32) dst[i] = P[l * nr + i];
   }
   __syncthreads();   // P, tau_sh and S_sh are reused by the next panel this CTA takes
 }
@@ -1156,23 +1216,34 @@ __device__ void qr_apply_tile(const QrJob& J, int k, int c1, int ncols, int adj,
   const int tid = threadIdx.x;
   const int g = tid / NT, l = (tid % NT) / NB, t = tid % NB;
   const int nch = (nr + RC - 1) / RC;
+  // (four elements of each at a time: their latencies one after another were half of a tile)
   auto load = [&](int rr0, int rows) {
-    for (int e = tid; e < RC * NB; e += kSvdThreads) {
-      const int i = e % RC, c = e / RC, gi = rr0 + i;
-      T v = czero<T>(), x = czero<T>();
-      if (i < rows) {
-        if (c < w) v = gi < c ? czero<T>() : (gi == c ? cmake<T>(1.0, 0.0) : A[(r0 + gi) + (long long)(r0 + c) * J.R]);
-        if (c < tw) x = X[(r0 + gi) + (long long)(c1 + c) * J.R];
+    constexpr int U = 4;
+    for (int e0 = tid; e0 < RC * NB; e0 += U * kSvdThreads) {
+      T v[U], x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = e0 + u * kSvdThreads, i = e % RC, c = e / RC, gi = rr0 + i;
+        v[u] = czero<T>();
+        x[u] = czero<T>();
+        if (i < rows && c < w && gi >= c) v[u] = gi == c ? cmake<T>(1.0, 0.0) : A[(r0 + gi) + (long long)(r0 + c) * J.R];
+        if (i < rows && c < tw) x[u] = X[(r0 + gi) + (long long)(c1 + c) * J.R];
       }
-      Vs[i + c * LD] = v;
-      Xs[i + c * LD] = x;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = e0 + u * kSvdThreads, i = e % RC, c = e / RC;
+        Vs[i + c * LD] = v[u];
+        Xs[i + c * LD] = x[u];
+      }
     }
   };
+  static_assert(RC * NB % (4 * kSvdThreads) == 0, "whole groups of four");
   T acc = czero<T>();
   for (int ch = 0; ch < nch; ++ch) {
     const int rr0 = ch * RC, rows = min(RC, nr - rr0);
     load(rr0, rows);
     __syncthreads();
+#pragma unroll 8
     for (int i = g; i < rows; i += G) acc = cadd(acc, cj_mul(Vs[i + l * LD], Xs[i + t * LD]));
     __syncthreads();
   }
@@ -1223,7 +1294,7 @@ constexpr size_t qr_tile_smem() {
 // then updates every NB-column tile right of it; a bounded grid barrier after
 // each phase.
 template <bool CPLX>
-__global__ void __launch_bounds__(kSvdThreads) qr_coop_kernel(const QrJob* __restrict__ jobs,
+__global__ void __launch_bounds__(kSvdThreads, 1) qr_coop_kernel(const QrJob* __restrict__ jobs,
                                                               const int* __restrict__ panels, const int* __restrict__ poff,
                                                               const QrTile* __restrict__ tiles, const int* __restrict__ toff,
                                                               int steps, void* qbuf, SvdCtl* ctl) {
