@@ -794,6 +794,10 @@ __global__ void __launch_bounds__(kSvdThreads) jacobi_coop_kernel(const SvdJob* 
     const int j = order[me.j0 + jj];
     const SvdJob J = jobs[j];
     const int R = J.trans ? J.n : J.m, C = J.trans ? J.m : J.n;
+    if (C <= 0) {                // an empty sector: nothing to rotate
+      if (me.rank == 0 && tid == 0) atomicMax(&ctl->sweeps, 1);
+      continue;
+    }
     T* W = static_cast<T*>(work) + J.woff;
     T* V = static_cast<T*>(vmat) + J.voff;
     int* pj = perm + J.soff;
