@@ -147,8 +147,11 @@ void launch_umma_items(int bn, const USlab* slabs, const UJob* jobs, const UItem
 int umma_status(bool reset);
 int device_sm_count();
 constexpr int kMaxDevices = 64;
-// cudaFuncSetAttribute(fn, MaxDynamicSharedMemorySize, bytes) once per device
-// (the attribute is per device); done[] holds one flag per device ordinal
+// cudaFuncSetAttribute(fn, MaxDynamicSharedMemorySize, bytes) once per device (the
+// attribute belongs to the kernel on a device and holds for every host thread, so bytes is
+// the most that any launch of it takes); done[] holds one flag per device ordinal
+void ensure_smem_limit(const void* fn, int bytes, unsigned char* done);
+// the same, and the largest shared-memory carve-out
 void ensure_smem_attr(const void* fn, int bytes, unsigned char* done);
 // Fixed device scratch of the allocation-free H_eff*psi entry point (gemm.cu).
 constexpr size_t kNoAllocScratchBytes = (size_t)32 << 20;

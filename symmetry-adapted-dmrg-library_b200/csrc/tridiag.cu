@@ -182,9 +182,10 @@ size_t smem_of(int n) { return sizeof(double) * ((size_t)n * n + 2 * (size_t)n);
 template <int NR>
 void launch(int ns, const int* n, int nmax, const double* a, const double* b, double* z0, int zstride, double* e0,
             int* status, cudaStream_t s) {
-  const size_t smem = smem_of(nmax);
-  SADMRG_CUDA(cudaFuncSetAttribute(tridiag_lowest_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_chained(tridiag_lowest_kernel<NR>, ns, 32, smem, s, ns, n, nmax, a, b, z0, zstride, e0, status);
+  // the limit belongs to the kernel, for every thread that launches it: its largest size, once
+  static unsigned char attr[kMaxDevices] = {0};
+  ensure_smem_limit((const void*)tridiag_lowest_kernel<NR>, (int)smem_of(32 * NR), attr);
+  launch_chained(tridiag_lowest_kernel<NR>, ns, 32, smem_of(nmax), s, ns, n, nmax, a, b, z0, zstride, e0, status);
   SADMRG_CUDA(cudaGetLastError());
 }
 

@@ -684,19 +684,18 @@ int device_sm_count() {
   return n[dev];
 }
 
-void ensure_smem_attr(const void* fn, int bytes, unsigned char* done) {
+static void smem_attr(const void* fn, int bytes, unsigned char* done, bool carveout) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    return;
-  }
-  if (!done[dev]) {
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    // the largest shared-memory carve-out, so that as many CTAs as the smem allows are resident
-    cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-    done[dev] = 1;
-  }
+  const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices;
+  if (known && done[dev]) return;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  // the largest carve-out: as many CTAs as the shared memory allows are resident
+  if (carveout) cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+  if (known) done[dev] = 1;
 }
+
+void ensure_smem_limit(const void* fn, int bytes, unsigned char* done) { smem_attr(fn, bytes, done, false); }
+void ensure_smem_attr(const void* fn, int bytes, unsigned char* done) { smem_attr(fn, bytes, done, true); }
 
 void launch_pack(const PackJob* jobs, const int* blk_job, int nblocks, const Bases& b, unsigned char* dst,
                  cudaStream_t s) {
