@@ -1474,10 +1474,11 @@ static int jacobi_run(const void* a, void* work, void* vmat, double* sv, const s
   const bool res = !stream && res_smem <= kSvdResMax;
   if (res) smem = std::max(smem, res_smem);
   const auto kernel = res ? jacobi_coop_kernel<CPLX, B, true> : jacobi_coop_kernel<CPLX, B, false>;
+  static unsigned char limit[2][kMaxDevices] = {{0}};
+  ensure_smem_limit((const void*)kernel, (int)std::max(svd_smem_bytes<CPLX, B>(), res ? kSvdResMax : 0), limit[res]);
   int dev = 0, nsm = 0, per_sm = 0;
   SADMRG_CUDA(cudaGetDevice(&dev));
   SADMRG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  SADMRG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   SADMRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSvdThreads, smem));
   SADMRG_REQUIRE(per_sm > 0, SADMRG_ERR_CUDA, "jacobi svd: the kernel does not fit on this device");
   std::vector<int> order;
@@ -1537,14 +1538,13 @@ static bool narrow_blocks(const std::vector<SvdJob>& hjobs) {
   return 2 * pairs16 < nsm;
 }
 
-// Launches a cooperative kernel on the largest grid the device keeps resident,
-// capped at `want` CTAs.  Returns false (nothing launched) when it cannot.
+// Launches a cooperative kernel (whose shared-memory limit is set) on the largest grid the
+// device keeps resident, capped at `want` CTAs.  Returns false (nothing launched) when it cannot.
 static bool coop_launch(const void* fn, int want, size_t smem, void** args, cudaStream_t s) {
   int dev = 0, coop = 0, nsm = 0, per_sm = 0;
   SADMRG_CUDA(cudaGetDevice(&dev));
   SADMRG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   SADMRG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  SADMRG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   SADMRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSvdThreads, smem));
   if (!coop || per_sm <= 0) return false;
   const int grid = std::max(1, std::min(want, per_sm * nsm));
@@ -1613,11 +1613,14 @@ struct QrLaunch {
     void* qb = qbuf;
     void* o = out;
     SvdCtl* pc = ctl;
+    static unsigned char limit[2][kMaxDevices] = {{0}};
     if (unmq) {
+      ensure_smem_limit((const void*)qr_unmq_kernel<CPLX>, (int)qr_tile_smem<CPLX>(), limit[1]);
       void* args[] = {(void*)&pj, (void*)&pt, (void*)&pto, (void*)&st, (void*)&qb, (void*)&o, (void*)&pc};
       return coop_launch((const void*)qr_unmq_kernel<CPLX>, L.want, qr_tile_smem<CPLX>(), args, s);
     }
     const size_t smem = std::max((size_t)maxR * NB * sizeof(typename SvdT<CPLX>::T), qr_tile_smem<CPLX>());
+    ensure_smem_limit((const void*)qr_coop_kernel<CPLX>, (int)std::max(kQrSmemMax, qr_tile_smem<CPLX>()), limit[0]);
     void* args[] = {(void*)&pj, (void*)&pp, (void*)&ppo, (void*)&pt, (void*)&pto, (void*)&st, (void*)&qb, (void*)&pc};
     return coop_launch((const void*)qr_coop_kernel<CPLX>, L.want, smem, args, s);
   }
