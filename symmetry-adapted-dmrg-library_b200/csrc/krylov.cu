@@ -16,6 +16,7 @@
 // 1,000 to 43,000 elements, 40 steps: one block per segment took 82 ms for the
 // vector kernels of a solve).
 #include <cuda_runtime.h>
+#include <algorithm>
 
 #include "kernels.cuh"
 #include "ptx.cuh"
@@ -26,6 +27,9 @@ namespace {
 constexpr int kVT = 256;             // threads per block
 constexpr int kVW = kVT / 32;
 constexpr int kG = 8;                // dots per pass over a block's range
+// coefficients that a block keeps in shared memory (complex 32 KB); those of further
+// vectors, which no solve has in earnest, are read where they are
+constexpr int kStaged = 2048;
 
 template <bool CX> struct VT_;
 template <> struct VT_<false> { using T = double; };
@@ -235,20 +239,23 @@ __global__ void __launch_bounds__(kVT) vec_axpy(VecSpan v, typename VT_<CX>::T* 
   chain_begin();
   Range r;
   if (!block_range(v, r)) return;
-  for (int j = threadIdx.x; j < nv; j += kVT) cs[j] = c[(long long)r.seg * cstride + j];
+  const auto* cg = c + (long long)r.seg * cstride;
+  const int ns = min(nv, kStaged);
+  for (int j = threadIdx.x; j < ns; j += kVT) cs[j] = cg[j];
   __syncthreads();
   double s2 = 0.0;
   for (long long i = r.lo + threadIdx.x; i < r.hi; i += kVT) {
     T a = x[i];
     int j = 0;
-    for (; j + kG <= nv; j += kG) {
+    for (; j + kG <= ns; j += kG) {
       T t[kG];
 #pragma unroll
       for (int u = 0; u < kG; ++u) t[u] = V[(j + u) * ldv + i];
 #pragma unroll
       for (int u = 0; u < kG; ++u) a = sub_mul(a, cs[j + u], t[u]);
     }
-    for (; j < nv; ++j) a = sub_mul(a, cs[j], V[j * ldv + i]);
+    for (; j < ns; ++j) a = sub_mul(a, cs[j], V[j * ldv + i]);
+    for (; j < nv; ++j) a = sub_mul(a, cg[j], V[j * ldv + i]);
     x[i] = a;
     s2 += vabs2(a);
   }
@@ -284,20 +291,23 @@ __global__ void __launch_bounds__(kVT) vec_lincomb(VecSpan v, typename VT_<CX>::
   chain_begin();
   Range r;
   if (!block_range(v, r)) return;
-  for (int j = threadIdx.x; j < nv; j += kVT) cs[j] = c[(long long)r.seg * cstride + j];
+  const auto* cg = c + (long long)r.seg * cstride;
+  const int ns = min(nv, kStaged);
+  for (int j = threadIdx.x; j < ns; j += kVT) cs[j] = cg[j];
   __syncthreads();
   double s2 = 0.0;
   for (long long i = r.lo + threadIdx.x; i < r.hi; i += kVT) {
     T a = vzero(T());
     int j = 0;
-    for (; j + kG <= nv; j += kG) {
+    for (; j + kG <= ns; j += kG) {
       T t[kG];
 #pragma unroll
       for (int u = 0; u < kG; ++u) t[u] = V[(j + u) * ldv + i];
 #pragma unroll
       for (int u = 0; u < kG; ++u) a = add_rmul(a, cs[j + u], t[u]);
     }
-    for (; j < nv; ++j) a = add_rmul(a, cs[j], V[j * ldv + i]);
+    for (; j < ns; ++j) a = add_rmul(a, cs[j], V[j * ldv + i]);
+    for (; j < nv; ++j) a = add_rmul(a, cg[j], V[j * ldv + i]);
     y[i] = a;
     s2 += vabs2(a);
   }
@@ -365,23 +375,25 @@ void launch_vec_dots(bool cplx, const VecSpan& v, const void* V, long long ldv, 
 void launch_vec_axpy(bool cplx, const VecSpan& v, void* x, const void* V, long long ldv, int nv, const void* c,
                      int cstride, double* partial, unsigned* counter, const VecOut& o, cudaStream_t s) {
   if (v.nblk <= 0) return;
+  const size_t smem = std::min(nv, kStaged) * (cplx ? sizeof(double2) : sizeof(double));
   if (cplx)
-    launch_chained(vec_axpy<true>, v.nblk, kVT, nv * sizeof(double2), s, v, (double2*)x, (const double2*)V, ldv, nv,
-                                                              (const double2*)c, cstride, partial, counter, o);
+    launch_chained(vec_axpy<true>, v.nblk, kVT, smem, s, v, (double2*)x, (const double2*)V, ldv, nv,
+                   (const double2*)c, cstride, partial, counter, o);
   else
-    launch_chained(vec_axpy<false>, v.nblk, kVT, nv * sizeof(double), s, v, (double*)x, (const double*)V, ldv, nv,
-                                                              (const double*)c, cstride, partial, counter, o);
+    launch_chained(vec_axpy<false>, v.nblk, kVT, smem, s, v, (double*)x, (const double*)V, ldv, nv,
+                   (const double*)c, cstride, partial, counter, o);
 }
 
 void launch_vec_lincomb(bool cplx, const VecSpan& v, void* y, const void* V, long long ldv, int nv, const double* c,
                         int cstride, double* partial, unsigned* counter, const VecOut& o, cudaStream_t s) {
   if (v.nblk <= 0) return;
+  const size_t smem = std::min(nv, kStaged) * sizeof(double);
   if (cplx)
-    launch_chained(vec_lincomb<true>, v.nblk, kVT, nv * sizeof(double), s, v, (double2*)y, (const double2*)V, ldv, nv, c, cstride,
-                                                                partial, counter, o);
+    launch_chained(vec_lincomb<true>, v.nblk, kVT, smem, s, v, (double2*)y, (const double2*)V, ldv, nv, c, cstride,
+                   partial, counter, o);
   else
-    launch_chained(vec_lincomb<false>, v.nblk, kVT, nv * sizeof(double), s, v, (double*)y, (const double*)V, ldv, nv, c, cstride,
-                                                                 partial, counter, o);
+    launch_chained(vec_lincomb<false>, v.nblk, kVT, smem, s, v, (double*)y, (const double*)V, ldv, nv, c, cstride,
+                   partial, counter, o);
 }
 
 void launch_vec_div(bool cplx, const VecSpan& v, const void* x, void* y, void* y2, const double* scal, int sstride,
