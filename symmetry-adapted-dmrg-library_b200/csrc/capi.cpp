@@ -612,7 +612,7 @@ int sadmrg_heff_launches_per_matvec(sadmrg_handle* h, int precision, int* n) {
     const HeffPlan<S>& H = *S_.heff;
     *n = H.plan.launches_per_run(ScalarInfo<S>::cplx, precision,
                                  H.plan.runs_fused(h->ctx, ScalarInfo<S>::cplx, precision)) +
-         (H.npen > 0 ? 3 : 0);
+         (H.npen > 0 ? 2 : 0);   // its dots and its update
   });
 }
 
