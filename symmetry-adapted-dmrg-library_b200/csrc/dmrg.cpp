@@ -1,5 +1,6 @@
 // dmrg.cpp -- H_eff plans, Lanczos, block SVD truncation and the sweep driver.
 #include "dmrg.hpp"
+#include "hypot.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -333,14 +334,14 @@ void tridiag_eig(int n, std::vector<double>& d, std::vector<double> e, std::vect
       if (m != l) {
         if (iter++ == 100) throw Error(SADMRG_ERR_NUMERIC, "tridiagonal QL did not converge");
         double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-        double r = std::hypot(g, 1.0);
+        double r = rn::hypot(g, 1.0);
         g = d[m] - d[l] + e[l] / (g + (g >= 0.0 ? std::fabs(r) : -std::fabs(r)));
         double s = 1.0, cc = 1.0, pp = 0.0;
         int i;
         bool deflated = false;
         for (i = m - 1; i >= l; --i) {
           double f = s * e[i], b = cc * e[i];
-          e[i + 1] = (r = std::hypot(f, g));
+          e[i + 1] = (r = rn::hypot(f, g));
           if (r == 0.0) { d[i + 1] -= pp; e[m] = 0.0; deflated = true; break; }
           s = f / r;
           cc = g / r;

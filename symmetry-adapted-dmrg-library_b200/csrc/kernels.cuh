@@ -252,7 +252,7 @@ void launch_vec_div(bool cplx, const VecSpan& v, const void* x, void* y, void* y
 
 // Lowest eigenvalue (e0[s]) and its vector (z0[s * zstride + i], zeros to i = nmax) of ns
 // symmetric tridiagonals of n[s] <= nmax <= kTridiagMax rows (0: none), diagonal a[i * ns + s],
-// coupling of i and i + 1 b[(i + 1) * ns + s]; as tridiag_eig (dmrg.cpp) bit for bit.
+// coupling of i and i + 1 b[(i + 1) * ns + s]; as tridiag_eig (dmrg.cpp) bit for bit (tridiag.cu).
 // *status = 1 where one did not converge.  n, a, b, e0 and status may be page-locked host
 // memory.
 constexpr int kTridiagMax = 128;

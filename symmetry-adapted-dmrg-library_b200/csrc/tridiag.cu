@@ -3,10 +3,10 @@
 // A batched Lanczos diagonalises one tridiagonal per instance at every check point
 // (replaces LAPACK dstev, src/dmrg_inst.cpp:1216-1231).  One warp per matrix runs the
 // implicit QL of tridiag_eig (dmrg.cpp) with the same operations and roundings in the same
-// order, so the eigenvalues and vectors are those of the host's solver to the last bit:
-// the sign of a vector depends on how often an almost converged coupling is swept, which
-// the roundings decide.  hypot is Borges' corrected form without fma ("An improved
-// algorithm for hypot(a, b)", 2019), which is what the host's C library computes.
+// order and one hypot (hypot.hpp), so the eigenvalues and vectors are those of the host's
+// solver to the last bit (but for the rare quotient named at `rotation`): the sign of a
+// vector depends on how often an almost converged coupling is swept, which the roundings
+// decide.
 //
 // The time is the chain of a rotation, 0.2 us.  All lanes compute it, and each lane
 // rotates its own rows of the eigenvectors in shared memory while the next one is on its
@@ -16,47 +16,26 @@
 #include <algorithm>
 
 #include "common.hpp"
+#include "hypot.hpp"
 #include "kernels.cuh"
 #include "ptx.cuh"
 
 namespace sadmrg {
 namespace {
 
-__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+using rn::add;
+using rn::mul;
+using rn::sub;
 
-// h = sqrt(x^2 + y^2) less (h^2 - x^2 - y^2) / (2 h), x >= y >= 0, the numerator from
-// differences that are exact or nearly so
-__device__ __forceinline__ double hypot_core(double x, double y) {
-  const double h = __dsqrt_rn(add(mul(x, x), mul(y, y)));
-  double num;
-  if (h <= mul(2.0, y)) {
-    const double t = sub(h, y);
-    num = add(mul(x, sub(mul(2.0, t), x)), mul(sub(t, mul(2.0, sub(x, y))), t));
-  } else {
-    const double t = sub(h, x);
-    num = add(mul(mul(2.0, t), sub(x, mul(2.0, y))), add(mul(sub(mul(4.0, t), y), y), mul(t, t)));
-  }
-  return sub(h, __ddiv_rn(num, mul(2.0, h)));
-}
-__device__ __forceinline__ double hypot2(double a, double b) {
-  const double x = fmax(fabs(a), fabs(b)), y = fmin(fabs(a), fabs(b));
-  if (y <= mul(x, 0x1p-54)) return add(x, y);
-  // squares that would overflow or underflow: scaled by a power of two
-  if (x > 0x1p511) return mul(hypot_core(mul(x, 0x1p-600), mul(y, 0x1p-600)), 0x1p600);
-  if (y < 0x1p-459) return mul(hypot_core(mul(x, 0x1p600), mul(y, 0x1p600)), 0x1p-600);
-  return hypot_core(x, y);
-}
-
-// r = hypot2(f, g), s = f / r, c = g / r.  In the usual range without CUDA's division and
+// r = hypot(f, g), s = f / r, c = g / r.  In the usual range without CUDA's division and
 // square root after one another (0.39 us a rotation, 0.21 like this): from one inverse
 // square root y of x^2 + y^2, the square root and the quotients by Markstein's final
-// corrections (IBM J. Res. Dev. 34, 1990), which round as the exact results do; the
-// numerator's quotient is a correction below an ulp of h, for which y does.
+// corrections (IBM J. Res. Dev. 34, 1990).  They round as the exact results do but where an
+// exact quotient lies within about 2^-52 of an ulp from halfway between two numbers (so does
+// the correction of h, which is below an ulp of it): one in some 10^15.
 __device__ __forceinline__ void rotation(double f, double g, double& r, double& s, double& c) {
   const double af = fabs(f), ag = fabs(g), x = fmax(af, ag), y = fmin(af, ag);
-  if (y > mul(x, 0x1p-54) && x <= 0x1p511 && y >= 0x1p-459) {
+  if (y >= rn::kHypotLo && x <= rn::kHypotHi) {
     const double q = add(mul(x, x), mul(y, y)), i0 = rsqrt(q), h0 = mul(q, i0);
     const double h = fma(fma(-h0, h0, q), mul(0.5, i0), h0);
     const double t = sub(h, y), u = sub(h, x);
@@ -67,9 +46,9 @@ __device__ __forceinline__ void rotation(double f, double g, double& r, double& 
     s = fma(fma(-s0, r, f), ir, s0);
     c = fma(fma(-c0, r, g), ir, c0);
   } else {
-    r = hypot2(f, g);
-    s = __ddiv_rn(f, r);
-    c = __ddiv_rn(g, r);
+    r = rn::hypot(f, g);
+    s = rn::div(f, r);
+    c = rn::div(g, r);
   }
 }
 
@@ -114,9 +93,9 @@ __global__ void __launch_bounds__(32) tridiag_lowest_kernel(int ns, const int* n
         break;
       }
       const double el = e[l], dl = d[l];
-      double g = __ddiv_rn(sub(d[l + 1], dl), mul(2.0, el));
-      const double r0 = hypot2(g, 1.0);
-      g = add(sub(d[m], dl), __ddiv_rn(el, add(g, g >= 0.0 ? r0 : -r0)));
+      double g = rn::div(sub(d[l + 1], dl), mul(2.0, el));
+      const double r0 = rn::hypot(g, 1.0);
+      g = add(sub(d[m], dl), rn::div(el, add(g, g >= 0.0 ? r0 : -r0)));
       double sn = 1.0, cc = 1.0, pp = 0.0;
       double col[NR];           // the eigenvectors' column i + 1
 #pragma unroll

@@ -16,7 +16,7 @@ def load():
     lib = sadmrg.LIB_PATH
     src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "native_calls.cpp")
     out = os.path.join(tempfile.mkdtemp(prefix="sadmrg_native_"), "native_calls.so")
-    r = subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-I" + os.path.join(PKG, "csrc"),
+    r = subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fPIC", "-shared", "-I" + os.path.join(PKG, "csrc"),
                         "-I" + os.path.join(CUDA, "include"), src, lib,
                         "-Wl,-rpath," + os.path.dirname(os.path.abspath(lib)), "-o", out], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <vector>
 
+#include "hypot.hpp"
 #include "kernels.cuh"
 
 namespace sadmrg {
@@ -22,6 +23,10 @@ static int call(F f) {
 }
 
 extern "C" {
+
+void nc_hypot(long long n, const double* a, const double* b, double* out) {
+  for (long long i = 0; i < n; ++i) out[i] = rn::hypot(a[i], b[i]);
+}
 
 // d: n diagonal, e: n - 1 couplings; the lowest eigenvalue and its vector
 int nc_tridiag_host(int n, const double* d, const double* e, double* e0, double* z0) {
