@@ -821,7 +821,9 @@ __global__ void __launch_bounds__(kSvdThreads) jacobi_coop_kernel(const SvdJob* 
       int* cur = cnt + (sw % 3) * nj + j;
       if (me.rank == 0 && tid == 0) cnt[((sw + 1) % 3) * nj + j] = 0;
       // column order of this sweep: decreasing norm (de Rijk), ties by index.  Norms
-      // one warp per column, then every column's rank counted by a warp.
+      // one warp per column, then every column's rank counted by a warp.  A NaN counts as
+      // -1: the order is a permutation whatever the input, so no two visits of a round
+      // share a column.
       const int gw = (me.rank * kSvdThreads + tid) >> 5, nw = me.size * kSvdWarps;
       for (int c = gw; c < C; c += nw) {
         double a = 0.0;
@@ -835,10 +837,10 @@ __global__ void __launch_bounds__(kSvdThreads) jacobi_coop_kernel(const SvdJob* 
       }
       if (!svd_group_sync(bar, me.size, phase, ctl)) return;
       for (int c = gw; c < C; c += nw) {
-        const double v = __ldcg(nrm + J.soff + c);
+        const double v = fmax(__ldcg(nrm + J.soff + c), -1.0);
         int rank = 0;
         for (int k = lane; k < C; k += 32) {
-          const double u = __ldcg(nrm + J.soff + k);
+          const double u = fmax(__ldcg(nrm + J.soff + k), -1.0);
           rank += (u > v || (u == v && k < c)) ? 1 : 0;
         }
         rank = __reduce_add_sync(0xffffffffu, rank);
