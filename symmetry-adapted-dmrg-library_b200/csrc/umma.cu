@@ -400,8 +400,10 @@ __global__ void __launch_bounds__(kGThreads, MINB)
       const uint32_t d = tmem + (uint32_t)(acc * BN);
       ok = __all_sync(0xffffffffu, mbar_wait(saddr(&tempty[acc]), (((uint32_t)il >> 1) & 1u) ^ 1u, &abort_sh, wlim));
       if (!ok) {
-        if (leader && !abort_sh) atomicExch(&g_umma_status, 5);
-        abort_sh = 1;
+        if (leader) {                 // (another lane's flag must not hide the status)
+          if (!abort_sh) atomicExch(&g_umma_status, 5);
+          abort_sh = 1;
+        }
         break;
       }
       fence_after();
@@ -413,8 +415,10 @@ __global__ void __launch_bounds__(kGThreads, MINB)
         const uint32_t n = (uint32_t)(g / ST);
         ok = __all_sync(0xffffffffu, mbar_wait(saddr(&full[st]), n & 1u, &abort_sh, wlim));
         if (!ok) {
-          if (leader && !abort_sh) atomicExch(&g_umma_status, 6);
-          abort_sh = 1;
+          if (leader) {
+            if (!abort_sh) atomicExch(&g_umma_status, 6);
+            abort_sh = 1;
+          }
           break;
         }
         fence_after();
