@@ -68,4 +68,26 @@ int nc_lincomb(int cplx, long long n, void* y, const void* V, int nv, const doub
   });
 }
 
+
+// SVD of column-major blocks m[j] x n[j] lying back to back in a; work, vmat and sv hold
+// max x min, min x min and min elements per block, back to back.  The sweeps, -1, or -2.
+int nc_jacobi(int cplx, const void* a, void* work, void* vmat, double* sv, int nj, const int* m, const int* n,
+              int precondition, int stream_rows, int block) {
+  int sweeps = -2;
+  call([&] {
+    std::vector<SvdJob> jobs(nj);
+    long long ao = 0, wo = 0, vo = 0, so = 0;
+    for (int j = 0; j < nj; ++j) {
+      const int R = m[j] < n[j] ? n[j] : m[j], C = m[j] < n[j] ? m[j] : n[j];
+      jobs[j] = {ao, wo, vo, so, m[j], n[j], m[j] < n[j] ? 1 : 0};
+      ao += (long long)m[j] * n[j];
+      wo += (long long)R * C;
+      vo += (long long)C * C;
+      so += C;
+    }
+    sweeps = run_jacobi_svd(cplx != 0, a, work, vmat, sv, jobs, 60, nullptr, nullptr, precondition, stream_rows, block);
+  });
+  return sweeps;
+}
+
 }  // extern "C"
