@@ -718,7 +718,7 @@ SvdStats block_svd(Ctx& c, const BTensor<S>& psi, BTensor<S>& tu, double p1, BTe
     int kept = 0;
     for (int k = 0; k < C; ++k)
       if (s[k] / smax > 1e-10) ++kept;
-    if (kept == 0) kept = 1;
+    if (kept == 0 && C > 0) kept = 1;   // (a sector without rows or columns keeps nothing)
     if (max_dcut > 0 && kept > max_dcut) kept = max_dcut;
     dc[i] = kept;
     for (int k = 0; k < kept; ++k) { wsort.push_back(s[k]); isort.push_back(i); }
