@@ -68,7 +68,7 @@ void HeffBatch<S>::finalize(Ctx& c) {
     auto base = [&](int buf) -> long long { return buf == 2 ? ooff[i] : buf == 3 ? xoff[i] : seg[i]; };
     for (size_t j = 0; j < q.jobs.size(); ++j) {
       const GemmJob& J = q.jobs[j];
-      const int nj = P.add_job(q.job_stage[j], J.cbuf, J.coff + base(J.cbuf), J.m, J.n, J.ldc, J.flags);
+      const int nj = P.add_job(q.job_stage[j], J.cbuf, J.coff + base(J.cbuf), J.m, J.n, J.ldc);
       P.jobs[nj].tag = i;   // a masked matvec skips the jobs of converged instances
       for (const GemmTerm& t : q.job_terms[j])
         P.add_term(nj, t.abuf, t.aoff + base(t.abuf), t.lda, t.bbuf, t.boff + base(t.bbuf), t.ldb, t.k, t.flags,

@@ -208,7 +208,7 @@ HeffPlan<S> build_heff(Ctx& c, const BTensor<S>& psi, const BTensor<S>* hhL, con
   }
   const std::vector<Blk> P = blocks_of(psi);
   std::vector<int> job_of(psi.nten(), -1);
-  for (auto& b : P) job_of[b.idx] = p.add_job(1, 1, b.off, b.d[0], b.d[1], b.d[0], 0);
+  for (auto& b : P) job_of[b.idx] = p.add_job(1, 1, b.off, b.d[0], b.d[1], b.d[0]);
   const Struct& ps = psi.st;
   int q[8], d[8];
   // diagonal terms: hh_L^T psi  (contract(hh[il], 0, vec1, 0))
@@ -275,7 +275,7 @@ HeffPlan<S> build_heff(Ctx& c, const BTensor<S>& psi, const BTensor<S>* hhL, con
           }
           if (x < 0) {
             xo = p.alloc_scratch((long long)a.d[2] * pk.d[1]);
-            x = p.add_job(0, 3, xo, a.d[2], pk.d[1], a.d[2], 0);
+            x = p.add_job(0, 3, xo, a.d[2], pk.d[1], a.d[2]);
             p.add_term(x, 2, base[t.op1] + a.off, a.d[0], 0, pk.off, pk.d[0], pk.d[0], TF_TA, 1.0, 0.0);
           }
           p.add_term(job_of[m], 3, xo, a.d[2], 2, o2off[l], o2d0[l], pk.d[1], 0, fac, 0.0);

@@ -13,7 +13,6 @@
 namespace sadmrg {
 
 enum TermFlags : int { TF_TA = 1, TF_CA = 2, TF_TB = 4, TF_CB = 8 };
-enum JobFlags : int { JF_ACCUM = 1 };   // C += sum(terms); otherwise C = sum(terms)
 enum Precision : int { PREC_FP64 = 0, PREC_TF32X3 = 1 };
 constexpr int kMaxBases = 8;
 
@@ -23,10 +22,10 @@ struct GemmTerm {             // alpha * op(A) * op(B), A: m x k, B: k x n after
   int lda, ldb, k, flags;
   double ar, ai;              // alpha (imaginary part ignored for real data)
 };
-struct GemmJob {              // C (m x n, column-major, ldc) receives its terms
+struct GemmJob {              // C (m x n, column-major, ldc) = the sum of its terms
   long long coff;
   int cbuf, m, n, ldc;
-  int t0, nt, flags;
+  int t0, nt;
   int tag;                    // instance of a merged batch plan (0 otherwise): a launch given a mask
                               // skips every item of a job whose mask[tag] is 0
 };
@@ -99,7 +98,7 @@ struct UJob {                 // output tile grid of one job
   long long pack;             // >= 0: the result becomes A panels (T = 128) at this byte offset of the
                               // per-apply buffer, scaled by alpha, with pack_nslab slabs per panel
   double alpha;
-  int cbuf, m, n, ldc, flags, pack_nslab;
+  int cbuf, m, n, ldc, pack_nslab;
   int dep;                    // counter bumped per finished tile (results read as panels later), or -1
   int tag;                    // as GemmJob::tag
   int cx;                     // complex plan: the tile is a real-form block (rows 2i, 2i+1 = Re, Im of

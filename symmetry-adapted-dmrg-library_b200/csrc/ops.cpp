@@ -70,9 +70,9 @@ BTensor<S> clone(Ctx& c, const BTensor<S>& t) {
 
 // ---------------------------------------------------------------------------
 // plan
-int GemmPlan::add_job(int stage, int cbuf, long long coff, int m, int n, int ldc, int flags) {
+int GemmPlan::add_job(int stage, int cbuf, long long coff, int m, int n, int ldc) {
   GemmJob j{};
-  j.coff = coff; j.cbuf = cbuf; j.m = m; j.n = n; j.ldc = ldc; j.flags = flags;
+  j.coff = coff; j.cbuf = cbuf; j.m = m; j.n = n; j.ldc = ldc;
   jobs.push_back(j);
   job_terms.emplace_back();
   job_stage.push_back(stage);
@@ -149,7 +149,6 @@ void GemmPlan::build_schedule(GemmSchedule& sc, bool cplx, double scale) {
       if (job_stage[j] != s) continue;
       const GemmJob& J = jobs[j];
       const long long kt = ktot[j];
-      SADMRG_REQUIRE(!(J.flags & JF_ACCUM), SADMRG_ERR_STATE, "plan: FP64 jobs overwrite their block");
       for (int r0 = 0; r0 < J.m; r0 += BM)
         for (int c0 = 0; c0 < J.n; c0 += BN) {
           WorkItem w{};
@@ -455,12 +454,11 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
     u.n = J.n;
     u.ldc = xm * J.ldc;
     u.cx = cplx ? 1 : 0;
-    u.flags = J.flags;
     u.tag = J.tag;
     u.dep = -1;
     if (J.cbuf == 3) {
       auto it = xreader.find(J.coff);
-      if (it == xreader.end() || job_stage[j] != 0 || (J.flags & JF_ACCUM)) return false;
+      if (it == xreader.end() || job_stage[j] != 0) return false;
       const Key& k = packs[it->second].k;
       if (k.rows != xm * J.m || k.K != xm * J.n || k.ld != J.ldc || k.trans != 0 || k.T != kUmmaTileM ||
           k.cm != (cplx ? 2 : 0))
@@ -509,7 +507,6 @@ bool GemmPlan::build_umma(Ctx& c, const Bases& cb, bool cplx) {
       if (job_stage[j] != s) continue;
       const GemmJob& J = jobs[j];
       const long long ns = slab0[j + 1] - slab0[j];
-      if (ns == 0 && (J.flags & JF_ACCUM)) continue;
       const int tm = (U->jobs[j].m + kUmmaTileM - 1) / kUmmaTileM, tn = (J.n + BN - 1) / BN;
       const long long nch = std::max<long long>(1, (ns + kc - 1) / kc);
       for (int a = 0; a < tm; ++a)
@@ -848,7 +845,7 @@ BTensor<S> overlap_initial(Ctx& c, const BTensor<S>& uu, const BTensor<S>& vv, i
     if (!pres[m]) continue;
     const Blk& u0 = U[contrib[m][0].first];
     const Blk& v0 = V[contrib[m][0].second];
-    const int job = p.add_job(1, 2, out.off[m], u0.d[2], v0.d[2], u0.d[2], 0);
+    const int job = p.add_job(1, 2, out.off[m], u0.d[2], v0.d[2], u0.d[2]);
     for (auto& jk : contrib[m]) {
       const Blk& u = U[jk.first];
       const Blk& v = V[jk.second];
@@ -895,7 +892,7 @@ BTensor<S> overlap_transformation(Ctx& c, const BTensor<S>& uu, const BTensor<S>
         const long m = st.index(lab);
         if (x < 0) {
           const long long xo = p.alloc_scratch((long long)u.d[2] * o.d[1]);
-          x = p.add_job(0, 3, xo, u.d[2], o.d[1], u.d[2], 0);
+          x = p.add_job(0, 3, xo, u.d[2], o.d[1], u.d[2]);
           p.add_term(x, 0, u.off, u.d[flag], 2, o.off, o.d[0], u.d[flag], TF_TA, 1.0, 0.0);
         }
         contrib[m].push_back(Item{x, v.off, v.d[flag]});
@@ -908,7 +905,7 @@ BTensor<S> overlap_transformation(Ctx& c, const BTensor<S>& uu, const BTensor<S>
     if (!pres[m]) continue;
     int lab[8], dd[8];
     st.block(m, lab, dd);
-    const int job = p.add_job(1, 4, out.off[m], dd[0], dd[1], dd[0], 0);
+    const int job = p.add_job(1, 4, out.off[m], dd[0], dd[1], dd[0]);
     for (auto& it : contrib[m]) {
       const GemmJob& x = p.jobs[it.x];
       p.add_term(job, 3, x.coff, x.m, 1, it.voff, it.vrows, x.n, TF_CB, 1.0, 0.0);
@@ -958,7 +955,7 @@ BTensor<S> operator_transformation(Ctx& c, const BTensor<S>& uu, const BTensor<S
         }
         if (x < 0) {
           const long long xo = p.alloc_scratch((long long)u.d[2] * o.d[2]);
-          x = p.add_job(0, 3, xo, u.d[2], o.d[2], u.d[2], 0);
+          x = p.add_job(0, 3, xo, u.d[2], o.d[2], u.d[2]);
           p.add_term(x, 0, u.off, u.d[flag], 2, o.off, o.d[0], u.d[flag], TF_TA, 1.0, 0.0);
         }
         contrib[m].push_back(Item{x, v.off, v.d[flag], fac});
@@ -971,7 +968,7 @@ BTensor<S> operator_transformation(Ctx& c, const BTensor<S>& uu, const BTensor<S
     if (!pres[m]) continue;
     int lab[8], dd[8];
     st.block(m, lab, dd);
-    const int job = p.add_job(1, 4, out.off[m], dd[0], dd[2], dd[0] * dd[1], 0);
+    const int job = p.add_job(1, 4, out.off[m], dd[0], dd[2], dd[0] * dd[1]);
     for (auto& it : contrib[m]) {
       const GemmJob& x = p.jobs[it.x];
       p.add_term(job, 3, x.coff, x.m, 1, it.voff, it.vrows, x.n, TF_CB, it.fac, 0.0);
@@ -1034,7 +1031,7 @@ BTensor<S> operator_pairup(Ctx& c, const BTensor<S>& uu, const BTensor<S>& vv, c
           }
           if (x < 0) {
             const long long xo = p.alloc_scratch((long long)u.d[2] * o.d[2]);
-            x = p.add_job(0, 3, xo, u.d[2], o.d[2], u.d[2], 0);
+            x = p.add_job(0, 3, xo, u.d[2], o.d[2], u.d[2]);
             p.add_term(x, 0, u.off, u.d[flag], 2, o.off, o.d[0], u.d[flag], TF_TA, 1.0, 0.0);
           }
           const S alpha = S(fac) * op2.host[s2.off];
@@ -1049,7 +1046,7 @@ BTensor<S> operator_pairup(Ctx& c, const BTensor<S>& uu, const BTensor<S>& vv, c
     if (!pres[m]) continue;
     int lab[8], dd[8];
     st.block(m, lab, dd);
-    const int job = p.add_job(1, 4, out.off[m], dd[0], dd[1], dd[0], 0);
+    const int job = p.add_job(1, 4, out.off[m], dd[0], dd[1], dd[0]);
     for (auto& it : contrib[m]) {
       const GemmJob& x = p.jobs[it.x];
       p.add_term(job, 3, x.coff, x.m, 1, it.voff, it.vrows, x.n, TF_CB, re_of(it.alpha), im_of(it.alpha));
@@ -1106,7 +1103,7 @@ BTensor<S> operator_initial(Ctx& c, const BTensor<S>& uu, const BTensor<S>& vv, 
     if (!pres[m]) continue;
     int lab[8], dd[8];
     st.block(m, lab, dd);
-    const int job = p.add_job(1, 2, out.off[m], dd[0], dd[2], dd[0] * dd[1], 0);
+    const int job = p.add_job(1, 2, out.off[m], dd[0], dd[2], dd[0] * dd[1]);
     for (auto& it : contrib[m])
       p.add_term(job, 0, it.uoff, it.k, 1, it.voff, it.k, it.k, TF_TA | TF_CB, re_of(it.alpha), im_of(it.alpha));
   }
@@ -1160,7 +1157,7 @@ BTensor<S> contract(Ctx& c, const BTensor<S>& t1, int i1, const BTensor<S>& t2, 
     long long rows = 1, cols = 1;
     for (int k = 0; k < n1 - 1; ++k) rows *= d[k];
     for (int k = 0; k < n2 - 1; ++k) cols *= d[n1 - 1 + k];
-    const int job = p.add_job(1, 2, out.off[m], (int)rows, (int)cols, (int)rows, 0);
+    const int job = p.add_job(1, 2, out.off[m], (int)rows, (int)cols, (int)rows);
     for (auto& it : contrib[m]) {
       // A' = t1 with the contracted bond last (rows x k): transposed view when it is first
       const int fa = (i1 == 0) ? TF_TA : 0;

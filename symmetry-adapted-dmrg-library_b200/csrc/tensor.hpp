@@ -165,7 +165,7 @@ struct GemmPlan {
   UmmaTune tune;                  // tcgen05 tile choice (build_umma reads it)
   Bases const_bases{};            // where the constant panels come from (kept for rebuilds)
 
-  int add_job(int stage, int cbuf, long long coff, int m, int n, int ldc, int flags);
+  int add_job(int stage, int cbuf, long long coff, int m, int n, int ldc);
   void add_term(int job, int abuf, long long aoff, int lda, int bbuf, long long boff, int ldb, int k, int flags,
                 double ar, double ai);
   long long alloc_scratch(long long elems) { long long o = scratch_elems; scratch_elems += elems; return o; }

@@ -17,7 +17,7 @@
 //                      tcgen05.commit frees the stage, and after the item's last slab
 //                      signals the accumulator full;
 //   warps 2-5          epilogue: tcgen05.ld of the 128 x BN accumulator (each
-//                      warp its 32 lanes), then FP64 store (optionally adding)
+//                      warp its 32 lanes), then FP64 store
 //                      or hi/lo panels of X; a split-K item writes an FP32
 //                      partial tile and the last item of its tile to finish
 //                      (atomic count per tile) sums all partials in slot order.
@@ -58,7 +58,7 @@ __device__ __forceinline__ uint32_t tf32_rna(float x) {
   asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(r) : "f"(x));
   return r;
 }
-// x ~ hi + lo, both TF32 (the split of the mma.sync 3xTF32 path)
+// x ~ hi + lo, both TF32
 __device__ __forceinline__ void split_hl(double v, uint32_t& hi, uint32_t& lo) {
   const float f = (float)v;
   hi = tf32_rna(f);
@@ -529,13 +529,12 @@ __global__ void __launch_bounds__(kGThreads, MINB)
           }
         } else if (row0 + r < J.m) {
           double* C = static_cast<double*>(bases.p[J.cbuf]) + J.coff;
-          const bool accum = J.flags & JF_ACCUM;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int col = col0 + cb + j;
             if (col < J.n) {
               const long long idx = (row0 + r) + (long long)col * J.ldc;
-              C[idx] = accum ? C[idx] + x[j] : x[j];
+              C[idx] = x[j];
             }
           }
         }
