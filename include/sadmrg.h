@@ -147,8 +147,8 @@ int sadmrg_set_svd_precondition(sadmrg_handle* h, int on);
  * The same results either way; for tests and profiling. */
 int sadmrg_set_svd_stream(sadmrg_handle* h, int on);
 /* Block SVD Jacobi column blocks (no counterpart in the reference): 8 or 16
- * columns per block, or 0 (the default) for 8 when the widest round of 16-column
- * pairs would keep fewer than half the SMs busy and 16 otherwise.  The same
+ * columns per block, or 0 (the default) for 8 when a round of all sectors'
+ * 16-column pairs would keep fewer than half the SMs busy and 16 otherwise.  The same
  * results either way; for tests and profiling. */
 int sadmrg_set_svd_block(sadmrg_handle* h, int b);
 /* A fixed tile choice for the H_eff plans made after this call, instead of the

@@ -355,9 +355,9 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, const WorkItem& it, 
 // per warp: on 8..512 log-uniform blocks whole 64 x 64 tiles are 1.55 times the useful
 // products.
 //
-// Measured (one H_eff*psi, graph replay): SU(2) D = 512 bond 145 -> 85 us, SU(2) ladder
-// centre 273 -> 216, SU(2) D = 1500 bond 1593 -> 1115 (24.7 TFLOP/s), U(1) D = 64 bond
-// 37 -> 14, complex U(1) D = 1024 bond 2343 -> 1213 (27.3 TFLOP/s).  Tried and slower: a
+// Measured (one H_eff*psi, graph replay): SU(2) D = 512 bond 145 -> 83 us, SU(2) ladder
+// centre 274 -> 217, SU(2) D = 1500 bond 1594 -> 1114 (24.6 TFLOP/s), U(1) D = 64 bond
+// 37 -> 13, complex U(1) D = 1024 bond 2351 -> 1219 (27.1 TFLOP/s).  Tried and slower: a
 // predicate on each mma instead of compiled strip counts (2x); one copying warp beside
 // four multiplying ones (it issues at one warp's rate: 90 us at D = 512); that with
 // persistent CTAs and both stages in one launch (130 us).

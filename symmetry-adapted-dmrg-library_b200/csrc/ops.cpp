@@ -93,9 +93,9 @@ void GemmPlan::add_term(int job, int abuf, long long aoff, int lda, int bbuf, lo
 // a stage's time, since three CTAs share an SM and the last ones run alone, and every
 // piece of a split reduction pays for a partial tile and the fix-up; so reductions are
 // cut where they exceed a sixth (complex: a sixteenth) of an SM's share of the stage,
-// but not below 128 of k.  Shares of 1/3, 1/6 and 1/16: 233, 216 and 241 us on the
-// SU(2) ladder centre (8..512 blocks), 1147, 1115 and 1142 us at D = 1500; complex U(1)
-// D = 1024: 1328, 1329 and 1213 us.  scale > 1 lengthens the pieces (fewer slots).
+// but not below 128 of k.  Shares of 1/3, 1/6 and 1/16: 232, 217 and 240 us on the
+// SU(2) ladder centre (8..512 blocks), 1174, 1113 and 1138 us at D = 1500; complex U(1)
+// D = 1024: 1343, 1348 and 1219 us.  scale > 1 lengthens the pieces (fewer slots).
 //
 // A stage-0 result (buffer 3) takes over the scale that all its readers apply, when
 // they agree (scaling an element before it is stored or after it is loaded rounds alike).

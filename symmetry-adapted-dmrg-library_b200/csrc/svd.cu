@@ -1525,7 +1525,7 @@ static int jacobi_run(const void* a, void* work, void* vmat, double* sv, const s
   return hctl.failed ? -1 : hctl.sweeps;
 }
 
-// Column blocks of the Jacobi for these jobs: 8 when the widest round of
+// Column blocks of the Jacobi for these jobs: 8 when a round of all sectors'
 // 16-column pairs would keep fewer than half the SMs busy, else 16.
 static bool narrow_blocks(const std::vector<SvdJob>& hjobs) {
   int dev = 0, nsm = 0;
@@ -1743,11 +1743,14 @@ int run_jacobi_svd(bool cplx, const void* a, void* work, void* vmat, double* sv,
       if (!fallback) return sw;
     }
   }
-  // column blocks of 16, or of 8 when the widest round of 16-column pairs would
+  // column blocks of 16, or of 8 when a round of all sectors' 16-column pairs would
   // keep fewer than half the SMs busy: narrower pairs double the CTAs per round
-  // and cut each visit's work to a quarter, which wins while SMs are idle (D=512:
-  // 1.87 -> 1.65 s of SVD per sweep) and loses once they are not (complex D=2048:
-  // 4.8 -> 5.5 s per iDMRG)
+  // and cut each visit's work to a quarter, which wins while SMs are idle and loses
+  // once they are not.  One truncation with 8 and 16 columns, ms: SU(2) D = 512 7.2 and
+  // 7.7, 768 14.7 and 16.3, 1,024 25.0 and 23.3, 2,048 107 and 80; complex U(1) D = 384
+  // 4.8 and 5.2, 1,024 24.5 and 27.5, 1,536 52.0 and 59.7, 2,048 145 and 106.  The rule
+  // takes 8 up to 1,024 in both, so it is 7% off the better width at SU(2) D = 1,024
+  // and 14% at complex D = 1,536.
   const bool narrow = block == 8 || (block == 0 && narrow_blocks(hjobs));
   if (cplx)
     return narrow ? jacobi_run<true, 8>(a, work, vmat, sv, hjobs, max_sweeps, s, kernel_ms, 1, stream)

@@ -31,8 +31,8 @@
 // launch: packing 13 us, the items' slabs, the last sums.  Panels are copied to the rows the
 // block has, the mma issued from uniform registers (550 cycles a slab, from a branch of one
 // lane 950), a slab's entry, dependencies and copies taken by a lane of their own (one lane
-// for all: four loads after one another per slab).  SU(2) ladder centre 97.8 -> 78.8 us,
-// complex U(1) D = 1024 337 -> 300, matvecs back to back.  Tried and no faster: the 128-byte
+// for all: four loads after one another per slab).  SU(2) ladder centre 96.4 -> 80.8 us,
+// complex U(1) D = 1024 331 -> 291 (graph replays, one plan without tuning).  Tried and no faster: the 128-byte
 // swizzle (panels are then written in scattered pieces), 8 epilogue warps (168 registers), the
 // longest item to the least loaded CTA, 4 groups at a time in the packing.
 //
